@@ -97,14 +97,19 @@ extern "C" __global__ void __launch_bounds__(CPV_BATCH_BLOCK, CPV_SETUP_MIN_BLOC
  * to its draw's parameters and its pipeline's stage functions. */
 struct CpvBatchSource {
     const CpvBatchParams& B;
-    uint64_t begin, end;
+    uint64_t begin, end;  /* of the current batch's first primitive, and of the tile */
     bool scan_rects;
     uint32_t tx, ty;
     float vw, vh;
     uint32_t fb_width, fb_height;
+    uint32_t taken;
 
-    __device__ __forceinline__ uint64_t count() const { return end > begin ? end - begin : 0; }
-    __device__ __forceinline__ void setup(uint64_t i, CpvTri& t) const {
+    __device__ __forceinline__ uint32_t next(uint32_t*) {
+        begin += taken;
+        taken = begin >= end ? 0u : static_cast<uint32_t>(end - begin < CPV_BATCH ? end - begin : CPV_BATCH);
+        return taken;
+    }
+    __device__ __forceinline__ void setup(uint32_t i, CpvTri& t) const {
         uint64_t g;
         if (scan_rects) {
             g = begin + i;
@@ -169,8 +174,10 @@ extern "C" __global__ void __launch_bounds__(CPV_RT_THREADS, CPV_RT_MIN_BLOCKS) 
             begin = B.tile_begin[tile];
             end = B.tile_end[tile];
         }
-        CpvBatchSource src{B, begin, end, overflow, tx, ty, B.vw, B.vh, B.fb_width, B.fb_height};
-        cpv_raster_tile(src, tx, ty, reinterpret_cast<CpvTri*>(cpv_dyn_smem), warp_sums);
+        CpvBatchSource src{B, begin, end, overflow, tx, ty, B.vw, B.vh, B.fb_width, B.fb_height, 0u};
+        const uint32_t first = src.next(warp_sums);
+        if (first == 0u) continue;
+        cpv_raster_tile(src, first, tx, ty, reinterpret_cast<CpvTri*>(cpv_dyn_smem), warp_sums);
     }
 }
 

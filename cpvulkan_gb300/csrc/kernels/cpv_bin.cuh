@@ -2,146 +2,195 @@
  * cpv_bin.cuh — order-preserving sort-middle binning and the other generic
  * device kernels (scan, fills).
  *
- * Binning builds, for every screen tile, the list of primitive ids that
- * touch it, in API order — the per-pixel order the reference's serial loop
- * (CPVulkan/CommandBuffer.Draw.cpp:1526-1593) produces. Primitives are split
- * into S contiguous spans, one warp per span, and the tiles are those of the
- * union of the draw's tile rectangles (reduced by cpv_setup_rects into
- * CpvDrawParams::tile_box), numbered row-major within it:
+ * The per-draw binning builds, for every bin (a square of screen tiles, at
+ * most CPV_MAX_BINS on the target), the list of primitive ids that touch it,
+ * in API order — the per-pixel order the reference's serial loop
+ * (CPVulkan/CommandBuffer.Draw.cpp:1526-1593) produces. The raster CTA of a
+ * tile filters its bin's list by the entries' tile rectangles, in order.
+ * Primitives are split into rows of row_prims consecutive ones:
  *
- *   1. cpv_span_count: each warp counts, per tile, the primitives of its span
- *      that touch the tile → counts[tile * S + span] (counts start zero).
- *   2. exclusive scan of counts in tile-major order (cpv_scan_dyn_reduce,
- *      cpv_scan_dyn_apply, which zeroes the counts again) → the write cursor
- *      of every (tile, span) pair; tile t's list is the contiguous range
- *      [cursor(t, 0), cursor(t + 1, 0)).
- *   3. cpv_span_write: each warp walks its span again in order and appends
- *      primitive ids at its cursors; within a warp, 32 (primitive, tile) pairs
- *      are placed per step with a match-any rank, so the order inside a span
- *      is the primitive order, and spans are laid out in span order.
+ *   1. cpv_setup_rects (the pipeline's module) writes every primitive's tile
+ *      rectangle and each row's count of primitives per bin;
+ *   2. cpv_bin_scan turns the counts, column by column, into the position of
+ *      each (row, bin)'s first entry and stores every bin's list range;
+ *   3. cpv_bin_write: one CTA per row writes the ids and the rectangles
+ *      within the bin at those positions, in primitive order.
  *
- * Grids are sized from host-known bounds (primitives, screen tiles, spans)
- * and the union's size is read on the device, so a draw needs no host round
- * trip and the whole sequence can be captured in a CUDA graph. The list has
- * a fixed capacity; a draw that would exceed it records the overflow and
- * the raster kernel falls back to scanning the per-primitive rectangles
+ * Every launch has a shape the host knows and no value is carried from one
+ * draw to the next, so the sequence needs no memset and can be captured in a
+ * CUDA graph. The list has a fixed capacity; a draw that would exceed it
+ * writes none and the raster filters the rectangles of all primitives
  * (slower, same result).
+ *
+ * Bins instead of tiles: a (tile x span) count matrix with one warp per span
+ * of 256 primitives is bound by its serial chain (a warp places 32
+ * (primitive, tile) pairs per dependent global step) for large primitives
+ * and by the matrix's size on large targets. Binning + raster on GB300, per
+ * tile then per bin: 300 triangles at 1280x720, 4800 + 526 us then 8 + 527
+ * (filtered); 12k quad triangles at 1280x720, 300 + 572 then 25 + 577; 400k at
+ * 1920x1080, 523 + 2385 then 68 + 2304; 500k small ones at 2048x2048, 173 + 315
+ * then 47 + 263. A bin's list is several times shorter than its tiles'
+ * lists together, and the filter reads 4 bytes per entry from L2.
  */
 #ifndef CPV_BIN_CUH
 #define CPV_BIN_CUH
 
 #include "cpv_device.cuh"
 
-__device__ __forceinline__ void cpv_rect_unpack(const uint16_t* rects, uint64_t g, uint32_t& x0, uint32_t& y0, uint32_t& x1, uint32_t& y1) {
-    const uint2 r = reinterpret_cast<const uint2*>(rects)[g];
-    x0 = r.x & 0xFFFFu;
-    y0 = r.x >> 16;
-    x1 = r.y & 0xFFFFu;
-    y1 = r.y >> 16;
-}
-
-__device__ __forceinline__ void cpv_span_range(uint64_t total, uint32_t spans, uint32_t span, uint64_t& begin, uint64_t& end) {
-    const uint64_t per = (total + spans - 1u) / spans;
-    begin = per * span;
-    end = begin + per;
-    if (begin > total) begin = total;
-    if (end > total) end = total;
-}
-
-/* Zeroes the (union tiles x spans) count matrix (grid-stride over a fixed
- * grid): for a matrix whose memory other buffers used since its last scan. */
-extern "C" __global__ void __launch_bounds__(256) cpv_bins_zero(uint32_t* __restrict__ counts, const uint32_t* __restrict__ box, uint32_t spans) {
-    const CpvTileBox b = cpv_tile_box(box);
-    const uint64_t n = static_cast<uint64_t>(b.w) * b.h * spans;
-    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) counts[i] = 0u;
-}
-
-/* counts[tile * spans + span] += primitives of the span touching the tile,
- * tile numbered row-major within the union. */
-extern "C" __global__ void __launch_bounds__(256) cpv_span_count(const uint16_t* __restrict__ rects, uint64_t total, uint32_t spans,
-                                                                 const uint32_t* __restrict__ box, uint32_t* __restrict__ counts) {
-    const uint32_t span = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t lane = threadIdx.x & 31u;
-    if (span >= spans) return;
-    const CpvTileBox b = cpv_tile_box(box);
-    uint64_t begin, end;
-    cpv_span_range(total, spans, span, begin, end);
-    for (uint64_t g = begin + lane; g < end; g += 32u) {
-        uint32_t x0, y0, x1, y1;
-        cpv_rect_unpack(rects, g, x0, y0, x1, y1);
-        for (uint32_t y = y0; y < y1; y++)
-            for (uint32_t x = x0; x < x1; x++) atomicAdd(&counts[(static_cast<uint64_t>(y - b.y0) * b.w + (x - b.x0)) * spans + span], 1u);
+/* 2. counts[row][bin] → the list position of the row's first entry in the
+ * bin; range[bin] = the bin's list. One CTA of 1024 threads per 8 bins: 128
+ * groups of rows are summed, scanned over the groups and walked again. A
+ * bin's list starts where an atomic on *total puts it (the lists' order in
+ * memory does not matter); *total (zeroed by cpv_setup_rects) ends as the
+ * draw's pair count. */
+#define CPV_BIN_SCAN_THREADS 1024
+#define CPV_BIN_SCAN_BINS 8
+extern "C" __global__ void __launch_bounds__(CPV_BIN_SCAN_THREADS) cpv_bin_scan(uint32_t* __restrict__ counts, uint32_t rows, uint32_t bins,
+                                                                               uint2* __restrict__ range, unsigned long long* __restrict__ total) {
+    __shared__ uint32_t warp_sums[CPV_BIN_SCAN_THREADS / 32][CPV_BIN_SCAN_BINS];
+    __shared__ uint32_t list_base[CPV_BIN_SCAN_BINS];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t b = threadIdx.x % CPV_BIN_SCAN_BINS, group = threadIdx.x / CPV_BIN_SCAN_BINS;
+    const uint32_t bin = blockIdx.x * CPV_BIN_SCAN_BINS + b;
+    const uint32_t groups = CPV_BIN_SCAN_THREADS / CPV_BIN_SCAN_BINS;
+    const uint32_t per = (rows + groups - 1u) / groups;
+    const uint32_t r0 = per * group < rows ? per * group : rows;
+    const uint32_t r1 = bin < bins ? (r0 + per < rows ? r0 + per : rows) : r0;
+    uint32_t* column = counts + bin;
+    uint32_t sum = 0u;
+#pragma unroll 8
+    for (uint32_t r = r0; r < r1; r++) sum += column[static_cast<uint64_t>(r) * bins];
+    uint32_t incl = sum;
+#pragma unroll
+    for (uint32_t o = CPV_BIN_SCAN_BINS; o < 32u; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane >= 32u - CPV_BIN_SCAN_BINS) warp_sums[warp][b] = incl;
+    __syncthreads();
+    if (warp < CPV_BIN_SCAN_BINS) {  /* warp k scans bin k over the 32 warps */
+        const uint32_t v = warp_sums[lane][warp];
+        uint32_t s = v;
+#pragma unroll
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, s, o);
+            if (lane >= o) s += t;
+        }
+        warp_sums[lane][warp] = s - v;
+        const uint32_t k = blockIdx.x * CPV_BIN_SCAN_BINS + warp;
+        if (lane == 31u && k < bins) {
+            const uint32_t base = s ? static_cast<uint32_t>(atomicAdd(total, static_cast<unsigned long long>(s))) : 0u;
+            list_base[warp] = base;
+            range[k] = make_uint2(base, base + s);
+        }
+    }
+    __syncthreads();
+    if (r1 <= r0) return;
+    uint32_t run = list_base[b] + warp_sums[warp][b] + incl - sum;
+#pragma unroll 8
+    for (uint32_t r = r0; r < r1; r++) {
+        const uint32_t c = column[static_cast<uint64_t>(r) * bins];
+        column[static_cast<uint64_t>(r) * bins] = run;
+        run += c;
     }
 }
 
-/* Appends primitive ids in order. cursor = scanned counts (modified in place:
- * afterwards cursor[t * spans + s] is the end of (t, s)). */
-extern "C" __global__ void __launch_bounds__(256) cpv_span_write(const uint16_t* __restrict__ rects, uint64_t total, uint32_t spans,
-                                                                 const uint32_t* __restrict__ box, uint32_t* __restrict__ cursor,
-                                                                 uint32_t* __restrict__ list, uint32_t capacity,
-                                                                 const uint32_t* __restrict__ pair_total) {
-    const uint32_t span = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t lane = threadIdx.x & 31u;
-    if (span >= spans) return;
-    const bool overflow = *pair_total > capacity;
-    const CpvTileBox b = cpv_tile_box(box);
-    uint64_t begin, end;
-    cpv_span_range(total, spans, span, begin, end);
+/* 3. One CTA per row, 256 primitives at a time: each warp counts its 32
+ * primitives per bin, the counts are scanned over the CTA's 8 warps onto the
+ * row's running positions, and each warp then places its (primitive, bin)
+ * pairs 32 at a time in primitive order (a match-any rank within the step,
+ * the warp's own position per bin between steps, all in shared memory).
+ * Dynamic shared memory: 9 words per bin. */
+extern "C" __global__ void __launch_bounds__(256) cpv_bin_write(const uint2* __restrict__ rects, uint64_t prims, uint32_t row_prims, uint32_t shift,
+                                                                uint32_t bins_x, uint32_t bins, const uint32_t* __restrict__ offsets,
+                                                                uint32_t* __restrict__ list, uint32_t* __restrict__ list_rects, uint32_t capacity,
+                                                                const unsigned long long* __restrict__ total) {
+    extern __shared__ uint32_t cpv_bin_smem[];
+    if (*total > capacity) return;
+    uint32_t* next = cpv_bin_smem;  /* [bin]: the row's next position */
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t* mine = cpv_bin_smem + (1u + warp) * bins;  /* [bin]: this warp's count, then its next position */
     const uint32_t lt_mask = (1u << lane) - 1u;
-    for (uint64_t base = begin; base < end; base += 32u) {
-        const uint64_t g = base + lane;
-        uint32_t x0 = 0, y0 = 0, x1 = 0, y1 = 0;
-        if (g < end) cpv_rect_unpack(rects, g, x0, y0, x1, y1);
-        const uint32_t w = x1 - x0;
-        const uint32_t n = w * (y1 - y0);
-        /* inclusive warp scan of pair counts → this lane's first pair */
+    const uint64_t begin = static_cast<uint64_t>(blockIdx.x) * row_prims;
+    const uint64_t end = begin + row_prims < prims ? begin + row_prims : prims;
+    for (uint32_t i = threadIdx.x; i < bins; i += 256u) next[i] = offsets[static_cast<uint64_t>(blockIdx.x) * bins + i];
+    for (uint64_t base = begin; base < end; base += 256u) {
+        for (uint32_t i = lane; i < bins; i += 32u) mine[i] = 0u;
+        __syncwarp();
+        const uint64_t g = base + threadIdx.x;
+        uint2 r = make_uint2(0u, 0u);
+        if (g < end) r = rects[g];
+        const uint32_t x0 = r.x & 0xFFFFu, y0 = r.x >> 16, x1 = r.y & 0xFFFFu, y1 = r.y >> 16;
+        const bool any = x1 > x0 && y1 > y0;
+        const uint32_t bx0 = x0 >> shift, by0 = y0 >> shift;
+        const uint32_t bw = any ? ((x1 - 1u) >> shift) + 1u - bx0 : 0u, bh = any ? ((y1 - 1u) >> shift) + 1u - by0 : 0u;
+        for (uint32_t y = 0; y < bh; y++)
+            for (uint32_t x = 0; x < bw; x++) atomicAdd(&mine[(by0 + y) * bins_x + bx0 + x], 1u);
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < bins; i += 256u) {
+            uint32_t run = next[i];
+#pragma unroll
+            for (uint32_t w = 0; w < 8u; w++) {
+                uint32_t* c = &cpv_bin_smem[(1u + w) * bins + i];
+                const uint32_t n = *c;
+                *c = run;
+                run += n;
+            }
+            next[i] = run;
+        }
+        __syncthreads();
+        /* inclusive warp scan of the pair counts */
+        const uint32_t n = bw * bh;
         uint32_t incl = n;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
             const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= static_cast<uint32_t>(o)) incl += v;
+            if (lane >= o) incl += v;
         }
-        const uint32_t total_pairs = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        const uint32_t pairs = __shfl_sync(0xFFFFFFFFu, incl, 31);
         const uint32_t excl = incl - n;
-        /* place the chunk's pairs 32 at a time, in (primitive, tile) order */
-        for (uint32_t p0 = 0; p0 < total_pairs; p0 += 32u) {
+        for (uint32_t p0 = 0; p0 < pairs; p0 += 32u) {
             const uint32_t p = p0 + lane;
-            const bool valid = p < total_pairs;
-            /* owner lane: last lane whose exclusive start <= p */
+            const bool valid = p < pairs;
+            /* owner lane: the last lane whose exclusive start is <= p (lanes
+             * without pairs share the next lane's start and are skipped) */
             uint32_t owner = 0;
 #pragma unroll
-            for (int step = 16; step >= 1; step >>= 1) {
-                const uint32_t cand = owner + static_cast<uint32_t>(step);
-                const uint32_t cand_excl = __shfl_sync(0xFFFFFFFFu, excl, cand);
-                if (cand_excl <= p) owner = cand;
+            for (uint32_t step = 16u; step >= 1u; step >>= 1) {
+                const uint32_t cand = owner + step;
+                if (__shfl_sync(0xFFFFFFFFu, excl, cand) <= p) owner = cand;
             }
-            /* excl is non-decreasing, so the last lane with excl <= p owns pair p
-             * (lanes with no pairs share the next lane's excl and are skipped) */
-            const uint32_t o_excl = __shfl_sync(0xFFFFFFFFu, excl, owner);
-            const uint32_t o_x0 = __shfl_sync(0xFFFFFFFFu, x0, owner);
-            const uint32_t o_y0 = __shfl_sync(0xFFFFFFFFu, y0, owner);
-            const uint32_t o_w = __shfl_sync(0xFFFFFFFFu, w, owner);
-            uint32_t tile = 0xFFFFFFFFu;
+            const uint32_t local = p - __shfl_sync(0xFFFFFFFFu, excl, owner);
+            const uint32_t o_x = __shfl_sync(0xFFFFFFFFu, r.x, owner), o_y = __shfl_sync(0xFFFFFFFFu, r.y, owner);
+            const uint32_t o_w = __shfl_sync(0xFFFFFFFFu, bw, owner);
+            uint32_t bin = 0xFFFFFFFFu, bx = 0u, by = 0u;
             if (valid) {
-                const uint32_t local = p - o_excl;
-                tile = (o_y0 - b.y0 + local / o_w) * b.w + (o_x0 - b.x0 + local % o_w);
+                const uint32_t row = local / o_w;
+                bx = ((o_x & 0xFFFFu) >> shift) + local - row * o_w;
+                by = (o_x >> (16u + shift)) + row;
+                bin = by * bins_x + bx;
             }
-            const uint32_t key = valid ? tile : (0x80000000u | lane);
-            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, valid ? bin : (0x80000000u | lane));
             const uint32_t rank = __popc(peers & lt_mask);
-            const uint32_t leader = __ffs(peers) - 1u;
-            uint32_t pos = 0;
-            volatile uint32_t* cur = nullptr;
-            if (valid) {
-                cur = &cursor[static_cast<uint64_t>(tile) * spans + span];
-                pos = *cur + rank;
-                if (!overflow && pos < capacity) list[pos] = static_cast<uint32_t>(base + owner);
-            }
+            uint32_t first = 0u;
+            if (valid) first = mine[bin];
             __syncwarp();
-            if (valid && lane == leader) *cur = *cur + __popc(peers);
+            if (valid) {
+                if (rank == 0u) mine[bin] = first + __popc(peers);
+                const uint32_t pos = first + rank;
+                if (pos < capacity) {  /* always, unless the pair total wrapped */
+                    /* the rectangle within the bin, in tiles */
+                    const uint32_t side = 1u << shift, tx = bx << shift, ty = by << shift;
+                    const uint32_t rx0 = o_x & 0xFFFFu, ry0 = o_x >> 16, rx1 = o_y & 0xFFFFu, ry1 = o_y >> 16;
+                    const uint32_t lx0 = rx0 > tx ? rx0 - tx : 0u, ly0 = ry0 > ty ? ry0 - ty : 0u;
+                    const uint32_t lx1 = rx1 - tx < side ? rx1 - tx : side, ly1 = ry1 - ty < side ? ry1 - ty : side;
+                    list[pos] = static_cast<uint32_t>(base + (threadIdx.x & ~31u) + owner);
+                    list_rects[pos] = lx0 | (ly0 << 8) | (lx1 << 16) | (ly1 << 24);
+                }
+            }
             __syncwarp();
         }
+        __syncthreads();
     }
 }
 
@@ -214,113 +263,6 @@ extern "C" __global__ void __launch_bounds__(CPV_SCAN_THREADS) cpv_scan_add(uint
 /* total = last exclusive prefix + last input. */
 extern "C" __global__ void cpv_scan_total(const uint32_t* __restrict__ in, const uint32_t* __restrict__ out, uint64_t n, uint32_t* __restrict__ total) {
     if (threadIdx.x == 0 && blockIdx.x == 0) *total = n ? out[n - 1] + in[n - 1] : 0u;
-}
-
-/* ---- exclusive scan of the (union tiles x spans) count matrix ----
- * Its size n = union tiles x spans is known on the device only. Two
- * launches over a fixed grid of G CTAs, CTA b owning the contiguous chunk
- * [b * C, (b + 1) * C), C = ceil(n / G): (1) each CTA sums its chunk and the
- * last CTA to finish scans the G sums (the counter at *done is reset for
- * the next draw; no CTA waits on another), (2) each CTA scans its chunk
- * from its scanned sum and zeroes the counts it read, so the matrix is
- * zero again for the next draw. */
-
-__device__ __forceinline__ void cpv_dyn_chunk(uint32_t n, uint32_t& begin, uint32_t& end) {
-    const uint32_t per = (n + gridDim.x - 1u) / gridDim.x;
-    begin = per * blockIdx.x;
-    end = begin + per;
-    if (begin > n) begin = n;
-    if (end > n) end = n;
-}
-
-__device__ __forceinline__ uint32_t cpv_box_bins(const uint32_t* box, uint32_t spans) {
-    const CpvTileBox b = cpv_tile_box(box);
-    return b.w * b.h * spans;
-}
-
-/* 1: sums[b] = the total of CTA b's chunk; the last CTA replaces sums[0 ..
- * G) by their exclusive scan and stores the pair total (G <= CPV_SCAN_BLOCK). */
-extern "C" __global__ void __launch_bounds__(CPV_SCAN_THREADS) cpv_scan_dyn_reduce(const uint32_t* __restrict__ in, const uint32_t* __restrict__ box,
-                                                                                  uint32_t spans, uint32_t* sums, uint32_t* done,
-                                                                                  uint32_t* __restrict__ total) {
-    uint32_t begin, end;
-    cpv_dyn_chunk(cpv_box_bins(box, spans), begin, end);
-    uint32_t s = 0;
-    /* CPV_SCAN_ITEMS independent loads in flight per thread and step */
-    for (uint32_t step = begin; step < end; step += CPV_SCAN_BLOCK) {
-#pragma unroll
-        for (int i = 0; i < CPV_SCAN_ITEMS; i++) {
-            const uint32_t k = step + static_cast<uint32_t>(i) * CPV_SCAN_THREADS + threadIdx.x;
-            s += k < end ? in[k] : 0u;
-        }
-    }
-    s = __reduce_add_sync(0xFFFFFFFFu, s);
-    __shared__ uint32_t warp_sums[CPV_SCAN_THREADS / 32];
-    __shared__ uint32_t last;
-    if ((threadIdx.x & 31u) == 0u) warp_sums[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0u) {
-        uint32_t t = 0;
-        for (int w = 0; w < CPV_SCAN_THREADS / 32; w++) t += warp_sums[w];
-        sums[blockIdx.x] = t;
-        __threadfence();
-        last = atomicAdd(done, 1u) == gridDim.x - 1u ? 1u : 0u;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const uint32_t count = gridDim.x;
-    const uint32_t base = threadIdx.x * CPV_SCAN_ITEMS;
-    uint32_t v[CPV_SCAN_ITEMS];
-    uint32_t sum = 0;
-#pragma unroll
-    for (int i = 0; i < CPV_SCAN_ITEMS; i++) {
-        v[i] = base + i < count ? __ldcg(&sums[base + i]) : 0u;
-        sum += v[i];
-    }
-    uint32_t all;
-    uint32_t run = cpv_block_exclusive_scan(sum, all);
-#pragma unroll
-    for (int i = 0; i < CPV_SCAN_ITEMS; i++) {
-        if (base + i < count) sums[base + i] = run;
-        run += v[i];
-    }
-    if (threadIdx.x == 0u) {
-        *total = all;
-        *done = 0u;
-    }
-}
-
-/* 2: cursor = exclusive scan of counts, CTA b's chunk offset by sums[b]
- * (CPV_SCAN_BLOCK elements per step, carried along the chunk); the counts
- * read are zeroed. */
-extern "C" __global__ void __launch_bounds__(CPV_SCAN_THREADS) cpv_scan_dyn_apply(uint32_t* __restrict__ counts, uint32_t* __restrict__ cursor,
-                                                                                 const uint32_t* __restrict__ box, uint32_t spans,
-                                                                                 const uint32_t* __restrict__ sums) {
-    uint32_t begin, end;
-    cpv_dyn_chunk(cpv_box_bins(box, spans), begin, end);
-    uint32_t carry = sums[blockIdx.x];
-    for (uint32_t step = begin; step < end; step += CPV_SCAN_BLOCK) {
-        const uint32_t base = step + threadIdx.x * CPV_SCAN_ITEMS;
-        uint32_t v[CPV_SCAN_ITEMS];
-        uint32_t sum = 0;
-#pragma unroll
-        for (int i = 0; i < CPV_SCAN_ITEMS; i++) {
-            v[i] = base + i < end ? counts[base + i] : 0u;
-            sum += v[i];
-        }
-        uint32_t all;
-        uint32_t run = carry + cpv_block_exclusive_scan(sum, all);
-#pragma unroll
-        for (int i = 0; i < CPV_SCAN_ITEMS; i++) {
-            if (base + i < end) {
-                cursor[base + i] = run;
-                counts[base + i] = 0u;
-            }
-            run += v[i];
-        }
-        carry += all;
-    }
 }
 
 /* ---- batched binning: pairs, stable radix sort by tile, tile ranges ----

@@ -53,6 +53,10 @@ struct CpvTexture {
     float lod_bias, min_lod, max_lod;
 };
 
+/* Bins of a draw: a square of tiles each, at most this many on the target
+ * (the per-draw binning kernels keep a counter per bin in shared memory). */
+#define CPV_MAX_BINS 1024u
+
 /* Everything one draw's kernels read. Passed by value as a kernel argument. */
 struct CpvDrawParams {
     /* geometry */
@@ -85,17 +89,19 @@ struct CpvDrawParams {
     uint32_t tile_shift;
     uint32_t tiles_x, tiles_y;
     uint32_t pad1;
-    /* binning scratch (null in direct mode) */
-    const uint32_t* tile_end;   /* tiles*spans cursor matrix after the write pass */
-    const uint32_t* bin_list;   /* primitive ids, tile-major, primitive order within a tile */
-    const uint32_t* pair_total; /* device word: pairs the draw needed */
-    const uint16_t* rects;      /* per primitive tile rectangle (x0,y0,x1,y1), exclusive ends */
-    /* the union of the draw's tile rectangles, 4 device words kept as maxima
-     * of (0xFFFF - x0, 0xFFFF - y0, x1, y1) (zeroed before the draw): the
-     * (tiles x spans) matrix covers only its tiles, row-major */
-    uint32_t* tile_box;
-    uint32_t spans;
+    /* binning: a bin is a square of 2^bin_shift x 2^bin_shift tiles. rects is
+     * null in direct mode (every tile walks every primitive), bin_counts is
+     * null when every tile filters the rectangles of all primitives */
+    uint2* rects;                 /* per primitive tile rectangle, packed x0 | y0 << 16, x1 | y1 << 16, ends exclusive */
+    uint32_t* bin_counts;         /* [row][bin]: the row's primitives touching the bin, then their first list position */
+    const uint2* bin_range;       /* per bin: its list's begin and end */
+    const uint32_t* bin_list;     /* primitive ids, bin after bin, primitive order within a bin */
+    const uint32_t* bin_rects;    /* per entry: its tile rectangle within the bin, x0 | y0 << 8 | x1 << 16 | y1 << 24 */
+    unsigned long long* pair_total; /* device word: (primitive, bin) pairs the draw needed */
+    uint32_t bin_shift, bins_x, bins;
+    uint32_t row_prims;           /* primitives per row (a multiple of 256) */
     uint32_t list_capacity;
+    uint32_t pad3;
     uint32_t* status;
     /* per primitive 4 x 256 bytes: the blend result of each channel for each
      * destination byte (pipelines blending a constant colour; null: compute) */

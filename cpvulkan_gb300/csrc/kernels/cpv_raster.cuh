@@ -458,15 +458,15 @@ __device__ __forceinline__ void cpv_list_small_warp(const CpvTri* tris, uint32_t
 #define CPV_RASTER_SMEM_BYTES \
     (CPV_BATCH * sizeof(CpvTri) + (CPV_DEFERRED ? CPV_NSLOT * (4u + 20u + 2u) : 0u) + (CPV_SPARSE ? CPV_SPARSE_BYTES : 0u))
 
-/* One screen tile (tx, ty): loads the tile's attachment texels into
- * registers, walks the tile's primitives from `src` in API order in batches
- * of CPV_BATCH (set-up into shared memory, then coverage, shading and the
+/* One screen tile (tx, ty) whose first batch holds `first` > 0 primitives:
+ * loads the tile's attachment texels into registers, walks the tile's
+ * primitives from `src` in API order in batches of CPV_BATCH (set-up into shared memory, then coverage, shading and the
  * per-fragment operations of each pixel in primitive order) and stores the
  * texels back once.
  *
  * Source supplies:
- *   uint64_t count()                         primitives of this tile
- *   void setup(uint64_t i, CpvTri& t)        set up the i-th (or mark it dead)
+ *   uint32_t next(uint32_t* warp_sums)       the size of the tile's next batch (up to CPV_BATCH; 0: done)
+ *   void setup(uint32_t i, CpvTri& t)        set up the batch's i-th primitive (or mark it dead)
  *   bool shade(const CpvTri&, const float w[3], int x, int y, float colour[CPV_COLOUR_FLOATS], float& mapped, const CpvPixel* early)
  *                                            (true: discarded, or failed the early depth
  *                                            test against *early when given)
@@ -499,9 +499,7 @@ __device__ __forceinline__ void cpv_list_small_warp(const CpvTri* tris, uint32_t
  * All apply each pixel's fragments in API primitive order, as the
  * reference's serial loop does. */
 template <class Source>
-__device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t tx, uint32_t ty, CpvTri* tris, uint32_t* warp_sums) {
-    const uint64_t end = src.count();
-    if (end == 0) return;
+__device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uint32_t tx, uint32_t ty, CpvTri* tris, uint32_t* warp_sums) {
     /* pixel-centre NDC of the tile's columns and rows (the values of
      * cpv_pixel_ndc); the barrier keeps the previous tile's readers of a
      * persistent CTA ahead of the rewrite */
@@ -562,8 +560,7 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t tx, uint32
 #endif
 #endif
 
-    for (uint64_t base = 0; base < end; base += CPV_BATCH) {
-        const uint32_t n = static_cast<uint32_t>((end - base) < CPV_BATCH ? (end - base) : CPV_BATCH);
+    for (uint32_t n = first; n != 0u; n = src.next(warp_sums)) {
         __syncthreads();
         /* a tile of 8 × 8 has fewer threads than CPV_BATCH: stride the set-up;
          * a primitive reaching beyond the tile that covers no pixel of it
@@ -571,7 +568,7 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t tx, uint32
          * is left to the pixel tests, which is cheaper for small primitives */
         for (uint32_t i = threadIdx.x; i < n; i += CPV_RT_THREADS) {
             CpvTri& t = tris[i];
-            src.setup(base + i, t);
+            src.setup(i, t);
             const int4 b = t.box;
             if (cpv_tri_live(t) && (b.x < tile_x0 || b.y < tile_y0 || b.z > tile_x0 + CPV_TILE || b.w > tile_y0 + CPV_TILE)) {
                 const int32_t rx0 = max(b.x, tile_x0), ry0 = max(b.y, tile_y0);

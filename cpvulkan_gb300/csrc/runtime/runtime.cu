@@ -283,8 +283,9 @@ Scratch::~Scratch() {
     if (!available()) return;
     cudaFree(rects_);
     cudaFree(counts_);
-    cudaFree(cursor_);
+    cudaFree(ranges_);
     cudaFree(list_);
+    cudaFree(list_rects_);
     for (auto* p : scan_) cudaFree(p);
     cudaFree(words_);
     cudaFree(tables_);
@@ -298,15 +299,19 @@ int Scratch::grow_tracked(T*& ptr, uint64_t& cap, uint64_t need) {
     return r;
 }
 
-int Scratch::reserve_rects(uint64_t prims) { return grow_tracked(rects_, rects_cap_, prims * 4); }
+int Scratch::reserve_rects(uint64_t prims) { return grow_tracked(rects_, rects_cap_, prims); }
 
-int Scratch::reserve_bins(uint64_t entries) {
+int Scratch::reserve_bins(uint64_t entries, uint64_t bins) {
     const int r = grow_tracked(counts_, counts_cap_, entries);
     if (r != kOk) return r;
-    return grow_tracked(cursor_, cursor_cap_, entries);
+    return grow_tracked(ranges_, ranges_cap_, bins);
 }
 
-int Scratch::reserve_list(uint64_t entries) { return grow_tracked(list_, list_cap_, entries); }
+int Scratch::reserve_list(uint64_t entries) {
+    const int r = grow_tracked(list_, list_cap_, entries);
+    if (r != kOk) return r;
+    return grow_tracked(list_rects_, list_rects_cap_, entries);
+}
 
 int Scratch::reserve_tables(uint64_t bytes) { return grow_tracked(tables_, tables_cap_, bytes); }
 
@@ -453,54 +458,87 @@ int blit(cudaStream_t stream, const CpvTexture& src, uint8_t* dst, uint32_t dst_
     return kOk;
 }
 
-static_assert(kWordsBytes >= 4ull * (kSumsWord + CPV_SCAN_BLOCK), "binning words hold a sum per scan element of a CTA");
-
 namespace {
 
-// CTAs of the per-draw binning kernels whose work is sized on the device,
-// for a count matrix of at most `bins` entries: one per CPV_SCAN_BLOCK
-// entries, at most one scanned CTA sum per scan element of a CTA (2048:
-// about 13 per SM, enough loads in flight for an image-sized matrix). Small
-// draws keep small grids, so draws of other queues run beside them.
-uint32_t bin_ctas(uint64_t bins) {
-    const uint64_t want = (bins + CPV_SCAN_BLOCK - 1) / CPV_SCAN_BLOCK;
-    return static_cast<uint32_t>(std::max<uint64_t>(1u, std::min<uint64_t>(CPV_SCAN_BLOCK, want)));
+// How a draw of the per-draw path finds a tile's primitives.
+struct BinShape {
+    enum Mode { kDirect, kFilter, kLists } mode = kDirect;
+    uint32_t shift = 0, bins_x = 0, bins = 0;  // bins of 2^shift x 2^shift tiles
+    uint32_t row_prims = 256, rows = 0;
+};
+
+// A draw of at most CPV_DIRECT_PRIMS primitives (and CPV_DIRECT_LIMIT
+// primitives x tiles) is walked whole by every tile: no launch but the
+// raster. One of at most CPV_FILTER_PRIMS is filtered by every tile from the
+// rectangles of all its primitives; a larger one is binned. Measured on
+// GB300: 1000 triangles on 256 tiles take 46 us of raster walked whole, 7 us
+// of set-up and 26 us of raster filtered, and 5 us more binned (two more
+// launches); 12000 triangles on 3600 tiles take 677 us filtered, 598 us
+// binned; the serving mix (1000 to 100000 triangles) 26.2 ms with the line
+// at 512 or 2048, 32.8 ms at 8192.
+BinShape bin_shape(uint64_t prims, uint32_t tiles_x, uint32_t tiles_y, uint64_t direct_limit) {
+    const uint32_t direct_prims = env_u32("CPV_DIRECT_PRIMS", 64u), filter_prims = env_u32("CPV_FILTER_PRIMS", 2048u);
+    BinShape b;
+    const uint64_t tiles = static_cast<uint64_t>(tiles_x) * tiles_y;
+    if (prims <= direct_prims && prims * tiles <= direct_limit) return b;
+    b.mode = BinShape::kFilter;
+    b.rows = static_cast<uint32_t>((prims + 255u) / 256u);
+    if (prims <= filter_prims) return b;
+    // bins of 4 x 4 tiles, or the smallest larger square that keeps them
+    // within CPV_MAX_BINS (a tile rectangle within a bin takes 8 bits a side)
+    for (b.shift = 2; b.shift <= 7; b.shift++) {
+        const uint32_t side = 1u << b.shift;
+        b.bins_x = (tiles_x + side - 1u) >> b.shift;
+        const uint64_t bins = static_cast<uint64_t>(b.bins_x) * ((tiles_y + side - 1u) >> b.shift);
+        if (bins > CPV_MAX_BINS) continue;
+        b.bins = static_cast<uint32_t>(bins);
+        b.mode = BinShape::kLists;
+        break;
+    }
+    // at most 16384 rows of a multiple of 256 primitives (CPV_BIN_ROW_PRIMS: at least so many)
+    while (b.mode == BinShape::kLists && b.row_prims < env_u32("CPV_BIN_ROW_PRIMS", 256u) && b.row_prims < (1u << 20)) b.row_prims *= 2u;
+    while (b.mode == BinShape::kLists && (prims + b.row_prims - 1u) / b.row_prims > 16384u) b.row_prims *= 2u;
+    if (b.mode == BinShape::kLists) b.rows = static_cast<uint32_t>((prims + b.row_prims - 1u) / b.row_prims);
+    return b;
 }
 
-// The per-draw binning after cpv_setup_rects has written the rectangles and
-// their union (tile_box): count into the (union tiles x spans) matrix, scan
-// it (reduce-then-scan over bin_ctas() CTAs; its size is read on the device;
-// the scan leaves the counts zero again), write the lists. zero_first: the
-// counts' memory is not known to be zero (the fixed scratch moves it with
-// the draw's size). words: [0] pair total, [9] the reduce's CTA counter,
-// [kSumsWord ..] the CTA sums.
-void bin_draw(cudaStream_t stream, const uint16_t* rects, uint64_t G, uint64_t spans, uint64_t bins, const uint32_t* tile_box, uint32_t* counts,
-              uint32_t* cursor, uint32_t* list, uint32_t capacity, uint32_t* words, bool zero_first) {
-    const uint32_t ctas = bin_ctas(bins);
-    uint32_t* sums = words + kSumsWord;
-    const uint32_t sp = static_cast<uint32_t>(spans);
-    if (zero_first) {
-        const unsigned zero_grid = static_cast<unsigned>(std::min<uint64_t>(ctas, (bins + 255) / 256));
-        profile_begin(stream, "cpv_bins_zero");
-        cpv_bins_zero<<<zero_grid, 256, 0, stream>>>(counts, tile_box, sp);
-        profile_end(stream);
-        count_launch();
-    }
-    const unsigned warp_blocks = static_cast<unsigned>((spans * 32 + 255) / 256);
-    profile_begin(stream, "cpv_span_count");
-    cpv_span_count<<<warp_blocks, 256, 0, stream>>>(rects, G, sp, tile_box, counts);
+// The per-draw kernels after P's buffers are set: set-up and binning.
+int bin_draw(cudaStream_t stream, const Module& m, const BinShape& b, CpvDrawParams& P) {
+    void* args[] = {&P};
+    profile_begin(stream, "cpv_setup_rects");
+    CPV_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(m.setup_rects), dim3(b.rows), dim3(256), args, 0, stream));
     profile_end(stream);
     count_launch();
-    profile_begin(stream, "cpv_scan");
-    cpv_scan_dyn_reduce<<<ctas, CPV_SCAN_THREADS, 0, stream>>>(counts, tile_box, sp, sums, words + 9, words);
-    cpv_scan_dyn_apply<<<ctas, CPV_SCAN_THREADS, 0, stream>>>(counts, cursor, tile_box, sp, sums);
+    if (b.mode != BinShape::kLists) return kOk;
+    profile_begin(stream, "cpv_bin_scan");
+    cpv_bin_scan<<<(b.bins + CPV_BIN_SCAN_BINS - 1u) / CPV_BIN_SCAN_BINS, CPV_BIN_SCAN_THREADS, 0, stream>>>(
+        P.bin_counts, b.rows, b.bins, const_cast<uint2*>(P.bin_range), P.pair_total);
     profile_end(stream);
     count_launch();
-    count_launch();
-    profile_begin(stream, "cpv_span_write");
-    cpv_span_write<<<warp_blocks, 256, 0, stream>>>(rects, G, sp, tile_box, cursor, list, capacity, words);
+    profile_begin(stream, "cpv_bin_write");
+    cpv_bin_write<<<b.rows, 256, 9u * b.bins * sizeof(uint32_t), stream>>>(P.rects, P.total_prims, b.row_prims, b.shift, b.bins_x, b.bins, P.bin_counts,
+                                                                          const_cast<uint32_t*>(P.bin_list), const_cast<uint32_t*>(P.bin_rects),
+                                                                          P.list_capacity, P.pair_total);
     profile_end(stream);
     count_launch();
+    CPV_CUDA(cudaGetLastError());
+    return kOk;
+}
+
+void set_bin_params(CpvDrawParams& P, const BinShape& b, uint2* rects, uint32_t* counts, uint2* ranges, uint32_t* list, uint32_t* list_rects,
+                    uint32_t capacity, uint32_t* words) {
+    P.rects = rects;
+    P.row_prims = b.row_prims;
+    if (b.mode != BinShape::kLists) return;
+    P.bin_counts = counts;
+    P.bin_range = ranges;
+    P.bin_list = list;
+    P.bin_rects = list_rects;
+    P.pair_total = reinterpret_cast<unsigned long long*>(words);
+    P.bin_shift = b.shift;
+    P.bins_x = b.bins_x;
+    P.bins = b.bins;
+    P.list_capacity = capacity;
 }
 
 }  // namespace
@@ -516,46 +554,18 @@ int draw_plain(cudaStream_t stream, const Module& m, CpvDrawParams P, Scratch& s
     const uint64_t G = P.total_prims;
     int r = sc.ensure_words();
     if (r != kOk) return r;
-    P.status = sc.words() + 1;
-    const uint32_t direct_limit = env_u32("CPV_DIRECT_LIMIT", 1u << 18);
-    uint32_t direct = (G * tiles <= direct_limit) ? 1u : 0u;
+    P.status = sc.words() + 2;
     if (G > 0xFFFFFFFFull) return kErrInvalid;
-    if (!direct) {
-        // Spans: one warp per ~CPV_SPAN_PRIMS primitives (default 256), at
-        // most 4096 spans; the (tiles x spans) count matrix grows with them.
-        static const uint32_t span_prims = std::max<uint32_t>(32u, env_u32("CPV_SPAN_PRIMS", 256u));
-        uint64_t spans = (G + span_prims - 1) / span_prims;
-        if (spans > 4096) spans = 4096;
-        if (spans < 1) spans = 1;
-        // the binning kernels index the (tiles x spans) matrix in 32 bits
-        while (spans > 1 && tiles * spans > 0x7FFFFFFFull) spans = (spans + 1) / 2;
-        if (tiles * spans > 0x7FFFFFFFull) return kErrInvalid;
-        const uint64_t bins = tiles * spans;
-        const uint32_t cap = env_u32("CPV_LIST_CAPACITY", 1u << 26);
+    const BinShape b = bin_shape(G, P.tiles_x, P.tiles_y, env_u32("CPV_DIRECT_LIMIT", 1u << 20));
+    if (b.mode != BinShape::kDirect) {
         if ((r = sc.reserve_rects(G)) != kOk) return r;
-        const uint32_t* counts_before = sc.counts();
-        if ((r = sc.reserve_bins(bins)) != kOk) return r;
-        // the count matrix is all zero between draws (each scan zeroes what
-        // it read); a new allocation starts it so
-        if (sc.counts() != counts_before) CPV_CUDA(cudaMemsetAsync(sc.counts(), 0, sc.counts_capacity() * sizeof(uint32_t), stream));
-        if ((r = sc.reserve_list(cap)) != kOk) return r;
-        P.rects = sc.rects();
-        P.spans = static_cast<uint32_t>(spans);
-        P.list_capacity = sc.list_capacity();
-        P.pair_total = sc.words();
-        P.tile_end = sc.cursor();
-        P.bin_list = sc.list();
-        P.tile_box = sc.words() + 4;
-        CPV_CUDA(cudaMemsetAsync(P.tile_box, 0, 4 * sizeof(uint32_t), stream));
-        {
-            void* args[] = {&P};
-            profile_begin(stream, "cpv_setup_rects");
-            CPV_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(m.setup_rects), dim3(static_cast<unsigned>((G + 255) / 256)), dim3(256), args, 0, stream));
-            profile_end(stream);
-            count_launch();
+        if (b.mode == BinShape::kLists) {
+            // the list holds what the draw can need at most, up to CPV_LIST_CAPACITY entries
+            const uint64_t cap = std::min<uint64_t>(env_u32("CPV_LIST_CAPACITY", 1u << 26), G * b.bins);
+            if ((r = sc.reserve_bins(static_cast<uint64_t>(b.rows) * b.bins, b.bins)) != kOk || (r = sc.reserve_list(cap)) != kOk) return r;
         }
-        bin_draw(stream, sc.rects(), G, spans, bins, P.tile_box, sc.counts(), sc.cursor(), sc.list(), sc.list_capacity(), sc.words(), false);
-        CPV_CUDA(cudaGetLastError());
+        set_bin_params(P, b, sc.rects(), sc.counts(), sc.ranges(), sc.list(), sc.list_rects(), sc.list_capacity(), sc.words());
+        if ((r = bin_draw(stream, m, b, P)) != kOk) return r;
     }
     // Blend tables: 1 KiB per primitive, built once per draw, when the
     // pipeline blends a per-primitive constant colour (up to 4 GiB of them;
@@ -571,7 +581,7 @@ int draw_plain(cudaStream_t stream, const Module& m, CpvDrawParams P, Scratch& s
         count_launch();
     }
     {
-        void* args[] = {&P, &direct};
+        void* args[] = {&P};
         profile_begin(stream, "cpv_raster");
         CPV_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(m.raster), dim3(static_cast<unsigned>(tiles)), dim3(m.raster_threads), args, m.raster_smem,
                                   stream));
@@ -1040,18 +1050,16 @@ int BatchPlan::launch(const Module& m, cudaStream_t stream) {
 //
 // One file-scope device array per device holds every per-draw scratch buffer
 // of the binning path. It is carved per draw, 256-byte aligned:
-//   words  (256 B)            [0] pair total (written by the scan before the
-//                             raster reads it), [1] status word
+//   words  (256 B)            the pair total (cleared by cpv_setup_rects), status
 //   rects  (8 B / primitive)  tile rectangles, written by cpv_setup_rects
-//   counts (4 B / tile·span)  bin counters: MUST start at zero; zeroed on
-//                             the stream at the start of every draw
-//   cursor (4 B / tile·span)  scanned counts, then write cursors
-//   scan   (per level)        block sums of the multi-level scan
-//   list   (the rest)         bin list; when the draw produces more
-//                             (primitive, tile) pairs than fit, the raster
-//                             walks the tile rectangles instead (same
-//                             image, slower)
-// Nothing else in the array needs an initial value.
+//   ranges (8 B / bin)        the bins' list ranges, written by the scan
+//   counts (4 B / row·bin)    row counts, then list positions
+//   lists  (the rest)         ids and rectangles, half each; when the draw
+//                             produces more (primitive, bin) pairs than fit,
+//                             or the counts leave too little room for lists,
+//                             each tile filters the rectangles of every
+//                             primitive instead (same image, slower)
+// Nothing in the array needs an initial value.
 // ---------------------------------------------------------------------------
 
 static __device__ __align__(256) uint8_t cpv_static_scratch[CPV_STATIC_SCRATCH_BYTES];
@@ -1064,47 +1072,19 @@ uint8_t* g_static_addr[kMaxStaticDevices] = {};
 
 uint64_t align256(uint64_t b) { return (b + 255u) & ~255ull; }
 
-struct StaticCarve {
-    uint64_t words = 0, rects = 0, counts = 0, cursor = 0, list = 0, end = 0;
-};
-
-// Offsets of the binning buffers for `prims` primitives over `bins` tile·span
-// bins; end = first byte of the bin list.
-StaticCarve static_carve(uint64_t prims, uint64_t bins) {
-    StaticCarve c;
-    uint64_t o = 0;
-    c.words = o;
-    o += kWordsBytes;
-    c.rects = o;
-    o += align256(prims * 8);
-    c.counts = o;
-    o += align256(bins * 4);
-    c.cursor = o;
-    o += align256(bins * 4);
-    c.list = o;
-    c.end = o;
-    return c;
-}
-
-// The binning decision of draw_plain: direct (no bins) or spans per tile.
+// Whether a draw of the fixed array is walked whole by every tile.
 // CPV_DIRECT_LIMIT is read once per process, so the pre-check and the draw
 // always take the same path.
-bool static_direct(uint64_t prims, uint64_t tiles) {
+uint64_t static_direct_limit() {
     static const uint32_t limit = env_u32("CPV_DIRECT_LIMIT", 1u << 18);
-    return prims * tiles <= limit;
+    return limit;
 }
 
-// Spans for a draw in the fixed array: draw_plain's choice, halved until the
-// buffers leave at least a quarter of the array for the bin list (or one
-// span remains).
-uint64_t static_spans(uint64_t prims, uint64_t tiles) {
-    uint64_t spans = (prims + 255) / 256;
-    if (spans > 4096) spans = 4096;
-    if (spans < 1) spans = 1;
-    while (spans > 1 && static_carve(prims, tiles * spans).end + CPV_STATIC_SCRATCH_BYTES / 4 > CPV_STATIC_SCRATCH_BYTES) spans = (spans + 1) / 2;
-    return spans;
-}
-
+// Bytes a draw may ask of the fixed array: 8 per primitive and 8 per tile
+// beside 8256 fixed ones. (The draw itself needs the rectangles only and
+// uses the rest as far as it goes; the limit is part of the entry point's
+// contract and stays with it.)
+uint64_t static_need(uint64_t prims, uint64_t tiles) { return 8256u + align256(prims * 8) + 2u * align256(tiles * 4); }
 
 }  // namespace
 
@@ -1137,8 +1117,8 @@ int static_scratch_check(uint64_t prims, uint32_t tile_shift, uint32_t width, ui
         error = "draw of " + std::to_string(prims) + " primitives exceeds 2^32 - 1";
         return kErrInvalid;
     }
-    if (static_direct(prims, tiles)) return kOk;
-    const uint64_t need = static_carve(prims, tiles * static_spans(prims, tiles)).end;
+    if (prims * tiles <= static_direct_limit()) return kOk;
+    const uint64_t need = static_need(prims, tiles);
     if (need > CPV_STATIC_SCRATCH_BYTES) {
         error = "draw of " + std::to_string(prims) + " primitives over " + std::to_string(tiles) + " tiles needs " + std::to_string(need) +
                 " bytes of binning scratch; the fixed scratch holds " + std::to_string(static_cast<uint64_t>(CPV_STATIC_SCRATCH_BYTES));
@@ -1170,35 +1150,35 @@ int draw_plain_static(cudaStream_t stream, const Module& m, CpvDrawParams P) {
         return r;
     }
     uint32_t* words = reinterpret_cast<uint32_t*>(base);
-    P.status = words + 1;
-    uint32_t direct = static_direct(G, tiles) ? 1u : 0u;
-    if (!direct) {
-        const uint64_t spans = static_spans(G, tiles);
-        const uint64_t bins = tiles * spans;
-        const StaticCarve c = static_carve(G, bins);
-        uint64_t cap = (CPV_STATIC_SCRATCH_BYTES - c.end) / 4;
-        if (cap > 0xFFFFFFFFull) cap = 0xFFFFFFFFull;
-        uint16_t* rects = reinterpret_cast<uint16_t*>(base + c.rects);
-        uint32_t* counts = reinterpret_cast<uint32_t*>(base + c.counts);
-        uint32_t* cursor = reinterpret_cast<uint32_t*>(base + c.cursor);
-        uint32_t* list = reinterpret_cast<uint32_t*>(base + c.list);
-        P.rects = rects;
-        P.spans = static_cast<uint32_t>(spans);
-        P.list_capacity = static_cast<uint32_t>(cap);
-        P.pair_total = words;
-        P.tile_end = cursor;
-        P.bin_list = list;
-        P.tile_box = words + 4;
-        CPV_CUDA(cudaMemsetAsync(P.tile_box, 0, 4 * sizeof(uint32_t), stream));
-        {
-            void* args[] = {&P};
-            CPV_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(m.setup_rects), dim3(static_cast<unsigned>((G + 255) / 256)), dim3(256), args, 0, stream));
-            count_launch();
+    P.status = words + 2;
+    BinShape b = bin_shape(G, P.tiles_x, P.tiles_y, static_direct_limit());
+    if (b.mode != BinShape::kDirect) {
+        // static_scratch_check has made sure that the rectangles fit
+        const uint64_t rects_at = align256(kWordsBytes), ranges_at = rects_at + align256(G * 8);
+        const uint64_t counts_at = ranges_at + align256(static_cast<uint64_t>(b.bins) * 8);
+        uint64_t lists_at = 0, entries = 0;
+        if (b.mode == BinShape::kLists) {
+            // fewer, longer rows until the counts leave half of what remains to the lists
+            auto counts_bytes = [&]() { return align256(static_cast<uint64_t>(b.rows) * b.bins * 4); };
+            while (b.rows > 1 && counts_at + 2 * counts_bytes() > CPV_STATIC_SCRATCH_BYTES) {
+                b.row_prims *= 2u;
+                b.rows = static_cast<uint32_t>((G + b.row_prims - 1u) / b.row_prims);
+            }
+            lists_at = counts_at + counts_bytes();
+            entries = lists_at < CPV_STATIC_SCRATCH_BYTES ? (CPV_STATIC_SCRATCH_BYTES - lists_at) / 8 : 0;
+            if (entries < G) {  // not a list entry per primitive: filter
+                b.mode = BinShape::kFilter;
+                b.row_prims = 256;
+                b.rows = static_cast<uint32_t>((G + 255u) / 256u);
+            }
         }
-        bin_draw(stream, rects, G, spans, bins, P.tile_box, counts, cursor, list, P.list_capacity, words, true);
+        uint32_t* list = reinterpret_cast<uint32_t*>(base + lists_at);
+        set_bin_params(P, b, reinterpret_cast<uint2*>(base + rects_at), reinterpret_cast<uint32_t*>(base + counts_at),
+                       reinterpret_cast<uint2*>(base + ranges_at), list, list + entries, static_cast<uint32_t>(entries), words);
+        if ((r = bin_draw(stream, m, b, P)) != kOk) return r;
     }
     {
-        void* args[] = {&P, &direct};
+        void* args[] = {&P};
         CPV_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(m.raster), dim3(static_cast<unsigned>(tiles)), dim3(m.raster_threads), args, m.raster_smem,
                                   stream));
         count_launch();

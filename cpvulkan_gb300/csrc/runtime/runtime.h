@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 #include <string>
@@ -58,11 +59,9 @@ int compile(const std::string& source, const std::string& name, std::vector<uint
 int load(const std::vector<uint8_t>& cubin, uint32_t tile_shift, bool batched, Module& out, std::string& error);
 void unload(Module& m);
 
-// Device words of a queue's per-draw binning: [0] pair total, [1] status,
-// [4..7] the union of the draw's tile rectangles, [9] the scan's CTA
-// counter, [kSumsWord ..] one scanned sum per binning CTA (at most 2048).
-constexpr uint32_t kSumsWord = 16;
-constexpr uint64_t kWordsBytes = 4ull * (kSumsWord + 2048u);
+// Device words of a queue's per-draw path: [0..1] the pair total (64 bits),
+// [2] status.
+constexpr uint64_t kWordsBytes = 256;
 
 // Grow-only device scratch owned by one queue. Draws on that queue's stream
 // reuse it in stream order.
@@ -70,18 +69,18 @@ class Scratch {
 public:
     ~Scratch();
     int reserve_rects(uint64_t prims);
-    int reserve_bins(uint64_t entries);  // tiles * spans
-    int reserve_list(uint64_t entries);
+    int reserve_bins(uint64_t entries, uint64_t bins);  // the count matrix, and a list range per bin
+    int reserve_list(uint64_t entries);                 // ids and rectangles
     int reserve_scan(uint64_t n);
     int reserve_tables(uint64_t bytes);
     uint8_t* tables() const { return tables_; }
-    uint16_t* rects() const { return rects_; }
+    uint2* rects() const { return rects_; }
     uint32_t* counts() const { return counts_; }
-    uint64_t counts_capacity() const { return counts_cap_; }
-    uint32_t* cursor() const { return cursor_; }
+    uint2* ranges() const { return ranges_; }
     uint32_t* list() const { return list_; }
-    uint32_t list_capacity() const { return static_cast<uint32_t>(list_cap_); }
-    uint32_t* words() const { return words_; }  // kWordsBytes: see kSumsWord
+    uint32_t* list_rects() const { return list_rects_; }
+    uint32_t list_capacity() const { return static_cast<uint32_t>(std::min(list_cap_, list_rects_cap_)); }
+    uint32_t* words() const { return words_; }  // kWordsBytes
     uint32_t* scan_level(int level) const { return scan_[level]; }
     int ensure_words();
     // Incremented whenever a buffer is (re)allocated: work captured in a CUDA
@@ -92,14 +91,16 @@ private:
     template <typename T>
     int grow_tracked(T*& ptr, uint64_t& cap, uint64_t need);
     uint64_t generation_ = 0;
-    uint16_t* rects_ = nullptr;
+    uint2* rects_ = nullptr;
     uint64_t rects_cap_ = 0;
     uint32_t* counts_ = nullptr;
     uint64_t counts_cap_ = 0;
-    uint32_t* cursor_ = nullptr;
-    uint64_t cursor_cap_ = 0;
+    uint2* ranges_ = nullptr;
+    uint64_t ranges_cap_ = 0;
     uint32_t* list_ = nullptr;
     uint64_t list_cap_ = 0;
+    uint32_t* list_rects_ = nullptr;
+    uint64_t list_rects_cap_ = 0;
     uint32_t* scan_[8] = {};
     uint64_t scan_cap_[8] = {};
     uint32_t* words_ = nullptr;
