@@ -193,11 +193,6 @@ std::string compose_module(const std::vector<std::string>& stages, const std::ve
     for (const std::string& st : stages)
         any_lines = any_lines || st.find("#define CPV_TOPOLOGY 1\n") != std::string::npos || st.find("#define CPV_TOPOLOGY 2\n") != std::string::npos;
     src << "#define CPV_ANY_LINES " << (any_lines ? 1 : 0) << "\n";
-    // Vertex-side kernels fill the UNORM8 decode table only when a vertex
-    // shader samples an image.
-    bool any_vs_samples = false;
-    for (const std::string& st : stages) any_vs_samples = any_vs_samples || st.find("#define CPV_VS_SAMPLES 1\n") != std::string::npos;
-    src << "#define CPV_ANY_VS_SAMPLES " << (any_vs_samples ? 1 : 0) << "\n";
     src << "#include \"cpv_device.cuh\"\n#include \"cpv_raster.cuh\"\n";
     for (size_t i = 0; i < stages.size(); i++) {
         src << "namespace cpv_p" << i << " {\n" << stages[i] << "#include \"cpv_stage.cuh\"\n";

@@ -36,10 +36,6 @@
  * set-up and raster kernels that follow (cpv_setup reads the slot instead of
  * shading the vertex again for each triangle and tile that uses it). */
 extern "C" __global__ void __launch_bounds__(CPV_BATCH_BLOCK) cpv_batch_vs(const __grid_constant__ CpvBatchParams B) {
-#if CPV_ANY_VS_SAMPLES
-    cpv_lut8_init();  /* the vertex shader samples images */
-    __syncthreads();
-#endif
     const uint32_t block = blockIdx.x;
     const uint32_t d = B.vs_block_draw[block];
     const CpvDrawParams& P = B.draws[d];
@@ -62,10 +58,6 @@ extern "C" __global__ void __launch_bounds__(CPV_BATCH_BLOCK) cpv_batch_vs(const
 #endif
 extern "C" __global__ void __launch_bounds__(CPV_BATCH_BLOCK, CPV_SETUP_MIN_BLOCKS) cpv_batch_setup(const __grid_constant__ CpvBatchParams B) {
     __shared__ uint32_t warp_pairs[CPV_BATCH_BLOCK / 32];
-#if CPV_ANY_VS_SAMPLES
-    cpv_lut8_init();  /* the vertex shader samples images */
-    __syncthreads();
-#endif
     const uint32_t block = blockIdx.x;
     const uint32_t d = B.block_draw[block];
     const CpvDrawParams& P = B.draws[d];
@@ -159,7 +151,6 @@ extern "C" __global__ void __launch_bounds__(CPV_RT_THREADS, CPV_RT_MIN_BLOCKS) 
     extern __shared__ float4 cpv_dyn_smem[];
     __shared__ uint32_t warp_sums[CPV_RT_THREADS / 32];
     __shared__ uint32_t next_tile;
-    cpv_lut8_init();
     const uint32_t tiles = B.tiles_x * B.tiles_y;
     const bool overflow = *B.pair_total > B.pair_capacity;
     for (;;) {

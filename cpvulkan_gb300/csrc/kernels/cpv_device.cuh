@@ -35,30 +35,32 @@ __device__ __forceinline__ float cpv_std_min(float a, float b) { return (b < a) 
 __device__ __forceinline__ float cpv_std_clamp(float v, float lo, float hi) { return (v < lo) ? lo : ((hi < v) ? hi : v); }
 
 /* UNORM encode (LLVMRuntime/ImageCompiler.cpp:27-32, 1081-1095):
- * minnum(maxnum(x,0),1) * (2^n-1), round half away from zero, to unsigned. */
+ * minnum(maxnum(x,0),1) * (2^n-1), round half away from zero, to unsigned,
+ * for 8 and 16 bits. Half away from zero of a value v >= 0 is floor(v + 0.5)
+ * of the exact sum: adding 0.5 plus a power of two rounded toward zero
+ * leaves the integer at a fixed place of the mantissa and drops only
+ * fraction bits, so no rounding function and no conversion is needed
+ * (compared for every binary32 v in [0, 1]). */
 __device__ __forceinline__ uint32_t cpv_encode_unorm(float x, float maxv) {
-    float v = fminf(fmaxf(x, 0.0f), 1.0f);
-    v = __fmul_rn(v, maxv);
-    v = roundf(v); /* half away from zero, as llvm.round */
-    return __float2uint_rz(v);
+    const float v = __fmul_rn(__saturatef(x), maxv); /* NaN → 0, as maxnum(NaN, 0) */
+    if (maxv == 255.0f) return (__float_as_uint(__fadd_rz(v, 32768.5f)) >> 8) & 0xFFu;
+    return (__float_as_uint(__fadd_rz(v, 131072.5f)) >> 6) & 0xFFFFu;
 }
 
-/* UNORM decode: uitofp then IEEE divide (LLVMRuntime/ImageCompiler.cpp:43-53). */
-__device__ __forceinline__ float cpv_decode_unorm8(uint32_t u) { return __fdiv_rn(__uint2float_rn(u), 255.0f); }
-__device__ __forceinline__ float cpv_decode_unorm16(uint32_t u) { return __fdiv_rn(__uint2float_rn(u), 65535.0f); }
-
-/* In pipeline modules the 256 UNORM8 decodes are a table in shared memory,
- * filled with exactly cpv_decode_unorm8(0..255) by each kernel before use:
- * one shared-memory read instead of an IEEE divide per channel. */
-#ifdef CPV_PIPELINE_MODULE
-__shared__ float cpv_lut8[256];
-#define CPV_DECODE8(u) cpv_lut8[(u)]
-__device__ __forceinline__ void cpv_lut8_init() {
-    for (uint32_t i = threadIdx.x; i < 256u; i += blockDim.x) cpv_lut8[i] = cpv_decode_unorm8(i);
+/* UNORM decode: uitofp then IEEE divide (LLVMRuntime/ImageCompiler.cpp:43-53).
+ * u / 255 and u / 65535 as u * hi + u * lo with hi + lo the reciprocal to
+ * twice the precision: equal to the rounded quotient for every code
+ * (compared for all 256 and all 65536). The code becomes a float through the
+ * mantissa of 2^23. */
+__device__ __forceinline__ float cpv_unorm_float(uint32_t u) { return __fsub_rn(__uint_as_float(0x4B000000u | u), 8388608.0f); }
+__device__ __forceinline__ float cpv_decode_unorm8(uint32_t u) {
+    const float f = cpv_unorm_float(u);
+    return __fmaf_rn(f, 0x1.010102p-8f, __fmul_rn(f, -0x1.fdfdfep-33f));
 }
-#else
-#define CPV_DECODE8(u) cpv_decode_unorm8(u)
-#endif
+__device__ __forceinline__ float cpv_decode_unorm16(uint32_t u) {
+    const float f = cpv_unorm_float(u);
+    return __fmaf_rn(f, 0x1.0001p-16f, __fmul_rn(f, 0x1.0001p-48f));
+}
 
 /* EdgeFunction (CPVulkan/CommandBuffer.Draw.cpp:410-418). */
 __device__ __forceinline__ float cpv_edge(float ax, float ay, float bx, float by, float cx, float cy) {
@@ -392,7 +394,7 @@ __device__ __forceinline__ void cpv_texel(const CpvTexture& t, uint32_t level, i
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int byte = (bgra && i < 3) ? 2 - i : i;
-        out[i] = CPV_DECODE8((px >> (8 * byte)) & 0xFFu);
+        out[i] = cpv_decode_unorm8((px >> (8 * byte)) & 0xFFu);
     }
 }
 

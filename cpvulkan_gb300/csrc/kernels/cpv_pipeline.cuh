@@ -32,9 +32,6 @@ extern "C" __global__ void __launch_bounds__(256) cpv_setup_rects(const __grid_c
         for (uint32_t i = threadIdx.x; i < P.bins; i += 256u) hist[i] = 0u;
         if (blockIdx.x == 0u && threadIdx.x == 0u) *P.pair_total = 0ull;
     }
-#if CPV_ANY_VS_SAMPLES
-    cpv_lut8_init();  /* the vertex shader samples images */
-#endif
     __syncthreads();
     const uint64_t begin = static_cast<uint64_t>(blockIdx.x) * P.row_prims;
     const uint64_t end = begin + P.row_prims < P.total_prims ? begin + P.row_prims : P.total_prims;
@@ -64,7 +61,6 @@ extern "C" __global__ void __launch_bounds__(256) cpv_setup_rects(const __grid_c
 extern "C" __global__ void __launch_bounds__(256) cpv_blend_tables(const __grid_constant__ CpvDrawParams P) {
     __shared__ float colours[256][4];
     __shared__ uint32_t live[256];
-    cpv_lut8_init();
     const uint64_t g = static_cast<uint64_t>(blockIdx.x) * 256u + threadIdx.x;
     uint32_t ok = 0u;
     if (cpv_p0::kBlendTable && g < P.total_prims) {
@@ -245,7 +241,6 @@ extern "C" __global__ void CPV_PLAIN_BOUNDS cpv_raster(const __grid_constant__ C
         first = src.next(warp_sums);
         if (first == 0u) return;
     }
-    cpv_lut8_init();
     cpv_raster_tile(src, first, tx, ty, reinterpret_cast<CpvTri*>(cpv_dyn_smem), warp_sums);
 }
 

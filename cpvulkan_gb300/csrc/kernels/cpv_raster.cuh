@@ -68,9 +68,6 @@
 #endif
 /* fragment shader outputs: 4 floats per colour attachment */
 #define CPV_COLOUR_FLOATS (4 * CPV_NUM_CA)
-#ifndef CPV_ANY_VS_SAMPLES
-#define CPV_ANY_VS_SAMPLES 1 /* some pipeline's vertex shader samples images */
-#endif
 #define CPV_NV_ALLOC (CPV_NV_MAX > 0 ? CPV_NV_MAX : 1)
 #define CPV_NV_ROOM0 (CPV_ANY_FS_CONSTANT && CPV_NV_ALLOC < 4 ? 4 : CPV_NV_ALLOC)
 #define CPV_NV_ROOM (CPV_ANY_LINES && CPV_NV_ROOM0 < 7 ? 7 : CPV_NV_ROOM0)

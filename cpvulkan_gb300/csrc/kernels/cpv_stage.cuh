@@ -415,7 +415,7 @@ __device__ __forceinline__ uint32_t cpv_channel_get(const uint32_t* t, int i) { 
  * as stored. */
 __device__ __forceinline__ float cpv_cf_decode(uint32_t raw) {
 #if CPV_CF_KIND == 0 && CPV_CF_BITS == 8
-    return CPV_DECODE8(raw);
+    return cpv_decode_unorm8(raw);
 #elif CPV_CF_KIND == 0
     return cpv_decode_unorm16(raw);
 #elif CPV_CF_KIND == 1
@@ -907,7 +907,7 @@ __device__ __forceinline__ void cpv_rop(const float blend_constants[4], bool fro
  * no DST_ALPHA-based colour factor, channel i's result depends only on
  * destination channel i). */
 __device__ __forceinline__ void cpv_blend_table_column(const float colour[4], const float blend_constants[4], uint32_t b, uint8_t out_bytes[4]) {
-    const float d = CPV_DECODE8(b);
+    const float d = cpv_decode_unorm8(b);
     const float dst[4] = {d, d, d, d};
     float out[4];
 #if CPV_BLEND
