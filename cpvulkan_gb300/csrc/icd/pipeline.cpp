@@ -63,7 +63,7 @@ const char* const kStageMacros[] = {
     "CPV_BLEND", "CPV_SRC_COLOR", "CPV_DST_COLOR", "CPV_COLOR_OP", "CPV_SRC_ALPHA", "CPV_DST_ALPHA", "CPV_ALPHA_OP", "CPV_WRITE_MASK", "CPV_LOGIC", "CPV_LOGIC_OP",
     "CPV_DEPTH_BOUNDS", "CPV_MIN_DEPTH_BOUNDS", "CPV_MAX_DEPTH_BOUNDS",
     "CPV_COLOR_FORMAT", "CPV_DEPTH_FORMAT", "CPV_ORIGIN_UPPER", "CPV_FS_CONSTANT", "CPV_BLEND_TABLE", "CPV_LINE_WIDTH", "CPV_PRIM_KIND",
-    "CPV_CF_BYTES", "CPV_CF_CHANNELS", "CPV_CF_BITS", "CPV_CF_KIND", "CPV_CF_BGRA", "CPV_FS_KILL", "CPV_EARLY_DEPTH", "CPV_VS_SAMPLES", "CPV_EXTRA_CA",
+    "CPV_CF_BYTES", "CPV_CF_CHANNELS", "CPV_CF_BITS", "CPV_CF_KIND", "CPV_CF_BGRA", "CPV_FS_KILL", "CPV_EARLY_DEPTH", "CPV_EXTRA_CA",
     "CPV_LOD_SITES",
 };
 
@@ -168,13 +168,12 @@ std::string compose_module(const std::vector<std::string>& stages, const std::ve
     if (const char* v = std::getenv("CPV_PLAIN_MIN_BLOCKS")) min_blocks = std::atoi(v);
     if (min_blocks >= 1 && min_blocks <= 32) src << "#define CPV_PLAIN_MIN_BLOCKS " << min_blocks << "\n";
     // Register budget of the persistent batched raster, in resident CTAs of
-    // 256 threads: 5 (48 registers a thread) for flat or lit shading, 4 (64)
-    // when a fragment shader samples images (C4: 39.4 ms at 5 against 40.2
-    // at 4; the textured heightfield: 0.41 ms at 4 against 0.43 at 5).
-    // CPV_BATCH_MIN_BLOCKS overrides.
+    // 256 threads: four (64 registers a thread; the 512-draw pass 3.00 ms,
+    // 3.01 at five, the 64-draw pass 176 and 204 us, the textured heightfield
+    // 217 and 238). CPV_BATCH_MIN_BLOCKS overrides.
     {
         const uint32_t threads = std::min(1u << (2 * mc.tile_shift), 32u * mc.warps);
-        int b = static_cast<int>((mc.samples ? 1024u : 1280u) / threads);
+        int b = static_cast<int>(1024u / threads);
         if (b < 1) b = 1;
         if (const char* v = std::getenv("CPV_BATCH_MIN_BLOCKS")) b = std::atoi(v);
         if (b >= 1 && b <= 32) src << "#define CPV_RT_MIN_BLOCKS " << b << "\n";
@@ -185,6 +184,17 @@ std::string compose_module(const std::vector<std::string>& stages, const std::ve
         const int k = std::atoi(v);
         if (k >= 1 && k <= 8) src << "#define CPV_SETUP_MIN_BLOCKS " << k << "\n";
     }
+    // Fragments divide by reciprocals prepared per triangle in per-draw
+    // modules that sample no images: their draws have the large triangles
+    // (raster of 300 blended half-float triangles at 1280x720 421 us, 519
+    // with divisions; of 12k interpolated ones 429 and 552). Where triangles
+    // are small the preparation and the wider record cost more than they
+    // save (the 512-draw pass's raster 3.14 ms, 3.00 with divisions; a
+    // 500k-triangle textured request's 199 us and 168). CPV_QUICK_DIV
+    // overrides.
+    int quick_div = !batched && !mc.samples ? 1 : 0;
+    if (const char* v = std::getenv("CPV_QUICK_DIV")) quick_div = std::atoi(v) ? 1 : 0;
+    src << "#define CPV_QUICK_DIV " << quick_div << "\n";
     src << "#define CPV_NV_MAX " << nv_max << "\n";
     bool any_constant = false;
     for (const std::string& st : stages) any_constant = any_constant || st.find("#define CPV_FS_CONSTANT 1\n") != std::string::npos;
@@ -559,7 +569,6 @@ VkResult create_graphics_pipeline(Device* dev, PipelineCache* cache, const VkGra
     for (int k : fr.interp) fs_constant = fs_constant && k == 2;
     src << "#define CPV_FS_CONSTANT " << (fs_constant ? 1 : 0) << "\n";
     src << "#define CPV_FS_KILL " << (fr.has_kill ? 1 : 0) << "\n";
-    src << "#define CPV_VS_SAMPLES " << (vr.samples > 0 ? 1 : 0) << "\n";
     src << "#define CPV_LOD_SITES " << fr.lod_sites << "\n";
     // Blending a per-primitive constant colour where each channel's result
     // depends only on that channel of the destination (no DST_ALPHA,

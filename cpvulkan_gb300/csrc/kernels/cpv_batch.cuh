@@ -65,8 +65,9 @@ extern "C" __global__ void __launch_bounds__(CPV_BATCH_BLOCK, CPV_SETUP_MIN_BLOC
     uint2 rect = make_uint2(0u, 0u);
     if (local < P.total_prims) {
         CpvTri t;
-        cpv_dispatch(B.draw_pipeline[d], [&](auto S) { decltype(S)::template setup<false>(P, local, t); });
-        rect = cpv_tile_rect(t, B.vw, B.vh, B.ndc_x, B.ndc_y);
+        int4 box;
+        cpv_dispatch(B.draw_pipeline[d], [&](auto S) { decltype(S)::template setup<false>(P, local, t, box); });
+        rect = cpv_tile_rect(t, box, B.vw, B.vh, B.ndc_x, B.ndc_y);
     }
     const uint64_t g = static_cast<uint64_t>(block) * CPV_BATCH_BLOCK + threadIdx.x;
     uint32_t pairs = ((rect.y & 0xFFFFu) - (rect.x & 0xFFFFu)) * ((rect.y >> 16) - (rect.x >> 16));
@@ -101,7 +102,7 @@ struct CpvBatchSource {
         taken = begin >= end ? 0u : static_cast<uint32_t>(end - begin < CPV_BATCH ? end - begin : CPV_BATCH);
         return taken;
     }
-    __device__ __forceinline__ void setup(uint32_t i, CpvTri& t) const {
+    __device__ __forceinline__ void setup(uint32_t i, CpvTri& t, int4& box) const {
         uint64_t g;
         if (scan_rects) {
             g = begin + i;
@@ -122,7 +123,7 @@ struct CpvBatchSource {
         const uint32_t d = B.block_draw[block];
         const uint64_t local = g - static_cast<uint64_t>(B.draw_block[d]) * CPV_BATCH_BLOCK;
         const uint32_t pid = B.draw_pipeline[d];
-        cpv_dispatch(pid, [&](auto S) { decltype(S)::template setup<true>(B.draws[d], local, t); });
+        cpv_dispatch(pid, [&](auto S) { decltype(S)::template setup<true>(B.draws[d], local, t, box); });
         cpv_tri_tag(t, pid, d);
     }
     __device__ __forceinline__ bool shade(const CpvTri& t, const float w[3], int32_t x, int32_t y, float* colour, float& mapped,

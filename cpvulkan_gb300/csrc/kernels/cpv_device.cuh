@@ -62,6 +62,19 @@ __device__ __forceinline__ float cpv_decode_unorm16(uint32_t u) {
     return __fmaf_rn(f, 0x1.0001p-16f, __fmul_rn(f, 0x1.0001p-48f));
 }
 
+/* a / b correctly rounded, for a divisor whose correctly rounded reciprocal
+ * y = 1 / b is at hand: one multiplication and two FMAs (N. Brisebarre, J.-M.
+ * Muller, S. K. Raina, "Accelerating correctly rounded floating-point
+ * division when the divisor is known in advance", IEEE Transactions on
+ * Computers 53(8), 2004; the correction step is Markstein's). It equals the
+ * IEEE quotient as long as nothing over- or underflows: callers keep |b| and
+ * |y| normal, |a| zero or at least 2^-91 and the quotient normal. A quotient
+ * of -0 may come out as +0. */
+__device__ __forceinline__ float cpv_div_by(float a, float b, float y) {
+    const float q = __fmul_rn(a, y);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
+
 /* EdgeFunction (CPVulkan/CommandBuffer.Draw.cpp:410-418). */
 __device__ __forceinline__ float cpv_edge(float ax, float ay, float bx, float by, float cx, float cy) {
     const float t0 = __fmul_rn(__fsub_rn(cx, ax), __fsub_rn(by, ay));

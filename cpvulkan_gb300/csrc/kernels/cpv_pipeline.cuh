@@ -37,8 +37,9 @@ extern "C" __global__ void __launch_bounds__(256) cpv_setup_rects(const __grid_c
     const uint64_t end = begin + P.row_prims < P.total_prims ? begin + P.row_prims : P.total_prims;
     for (uint64_t g = begin + threadIdx.x; g < end; g += 256u) {
         CpvTri t;
-        cpv_p0::Stage::setup<false>(P, g, t);
-        const uint2 r = cpv_tile_rect(t, P.viewport[2], P.viewport[3]);
+        int4 box;
+        cpv_p0::Stage::setup<false>(P, g, t, box);
+        const uint2 r = cpv_tile_rect(t, box, P.viewport[2], P.viewport[3]);
         P.rects[g] = r;
         const uint32_t x0 = r.x & 0xFFFFu, y0 = r.x >> 16, x1 = r.y & 0xFFFFu, y1 = r.y >> 16;
         if (lists && x1 > x0 && y1 > y0) {
@@ -71,7 +72,8 @@ extern "C" __global__ void __launch_bounds__(256) cpv_blend_tables(const __grid_
         }
         if (drawn) {
             CpvTri t;
-            cpv_p0::Stage::setup<true>(P, g, t);
+            int4 box;
+            cpv_p0::Stage::setup<true>(P, g, t, box);
             ok = cpv_tri_live(t) ? 1u : 0u;
 #pragma unroll
             for (int c = 0; c < 4; c++) colours[threadIdx.x][c] = t.var[0][c];
@@ -172,8 +174,8 @@ struct CpvPlainSource {
         return taken;
     }
     /* Sets up the i-th primitive of the current batch. */
-    __device__ __forceinline__ void setup(uint32_t i, CpvTri& t) const {
-        cpv_p0::Stage::setup<true>(P, L.ring[wrap(L.head + i)], t);
+    __device__ __forceinline__ void setup(uint32_t i, CpvTri& t, int4& box) const {
+        cpv_p0::Stage::setup<true>(P, L.ring[wrap(L.head + i)], t, box);
     }
     __device__ __forceinline__ bool shade(const CpvTri& t, const float w[3], int32_t x, int32_t y, float* colour, float& mapped,
                                           const CpvPixel* early = nullptr) const {

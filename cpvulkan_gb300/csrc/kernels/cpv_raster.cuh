@@ -42,14 +42,16 @@
 #ifndef CPV_ANY_FS_CONSTANT
 #define CPV_ANY_FS_CONSTANT 0 /* some pipeline of the module shades once per primitive */
 #endif
+#ifndef CPV_QUICK_DIV
+#define CPV_QUICK_DIV 0 /* fragments divide by reciprocals prepared at set-up */
+#endif
 #define CPV_TILE (1 << CPV_TILE_SHIFT)
 #define CPV_RT_THREADS ((CPV_TILE * CPV_TILE) < (32 * CPV_RT_WARPS) ? (CPV_TILE * CPV_TILE) : (32 * CPV_RT_WARPS))
 #define CPV_PPT ((CPV_TILE * CPV_TILE) / CPV_RT_THREADS)
-/* register budget of the persistent batched raster: 40 resident warps per
- * SM (48 registers a thread at 256 threads a CTA, the five CTAs shared
- * memory allows) */
+/* register budget of the persistent batched raster: 32 resident warps per
+ * SM (64 registers a thread) */
 #ifndef CPV_RT_MIN_BLOCKS
-#define CPV_RT_MIN_BLOCKS (1280 / CPV_RT_THREADS)
+#define CPV_RT_MIN_BLOCKS (1024 / CPV_RT_THREADS)
 #endif
 
 #define CPV_ROWS_PER_PASS (CPV_RT_THREADS / CPV_TILE)
@@ -80,7 +82,7 @@
  * groups so that the coverage loop reads them with 128-bit loads.
  *
  * Points and lines reuse the record (Draw.cpp:1315-1508):
- *   point — box is exactly the set of pixels the reference covers and the
+ *   point — its box is exactly the set of pixels the reference covers and the
  *           edges are zero (every pixel of the box passes); za.x = NDC z,
  *           wf.x = clip w, var[0] = the vertex's outputs;
  *   line  — e[0..2] and za are the four edges of the line's quad, wf.x/y
@@ -90,13 +92,41 @@
  *           first). */
 struct __align__(16) CpvTri {
     float4 e[3];     /* edge k: start vertex (x, y) and b - a (dx, dy), NDC */
-    int4 box;        /* pixel bounding box x0, y0, x1, y1 (end exclusive) */
     float4 za;       /* NDC z of p0..p2 (after the CW swap), |area| */
     float4 wf;       /* clip w of p0..p2, flags (see below) */
+#if CPV_QUICK_DIV
+    float4 rc;       /* triangles: 1 / wf.xyz and 1 / area, correctly rounded; w = 0: divide (cpv_tri_reciprocals) */
+#endif
     float var[3][CPV_NV_PAD]; /* varyings per vertex; for a pipeline whose fragment
                                  shader is constant per primitive, var[0][0..3]
                                  holds the shaded colour instead */
+#if (CPV_QUICK_DIV + 3 * CPV_NV_PAD / 4) % 2 == 1
+    /* an odd number of 16-byte units: 8 lanes that read a unit each of 8
+     * records then use all 32 banks once (the 500k-triangle request's raster
+     * 196 us at 12 units, 168 at 11; the 512-draw pass's 4.25 ms at 8 units,
+     * 3.0 at 9) */
+    float4 pad;
+#endif
 };
+
+/* A primitive's pixel bounding box within its tile, one byte each: x0, y0,
+ * x1 | 0x80, y1 | 0x80 (ends exclusive). The high bits make the subtraction of
+ * cpv_in_box borrow-free; a dead primitive has the empty box. */
+#define CPV_BOX_DEAD 0x80800000u
+__device__ __forceinline__ uint32_t cpv_box_pack(int32_t x0, int32_t y0, int32_t x1, int32_t y1) {
+    return static_cast<uint32_t>(x0) | (static_cast<uint32_t>(y0) << 8) | (static_cast<uint32_t>(x1) << 16) | (static_cast<uint32_t>(y1) << 24) | CPV_BOX_DEAD;
+}
+__device__ __forceinline__ int32_t cpv_box_x0(uint32_t b) { return static_cast<int32_t>(b & 0xFFu); }
+__device__ __forceinline__ int32_t cpv_box_y0(uint32_t b) { return static_cast<int32_t>((b >> 8) & 0xFFu); }
+__device__ __forceinline__ int32_t cpv_box_x1(uint32_t b) { return static_cast<int32_t>((b >> 16) & 0x7Fu); }
+__device__ __forceinline__ int32_t cpv_box_y1(uint32_t b) { return static_cast<int32_t>((b >> 24) & 0x7Fu); }
+/* A pixel of the tile as cpv_in_box takes it. */
+__device__ __forceinline__ uint32_t cpv_box_pixel(uint32_t lx, uint32_t ly) { return (lx | 0x80u) | ((ly | 0x80u) << 8) | ((lx + 1u) << 16) | ((ly + 1u) << 24); }
+/* x0 <= lx, y0 <= ly, lx + 1 <= x1 and ly + 1 <= y1, a byte each. */
+__device__ __forceinline__ bool cpv_in_box(uint32_t box, uint32_t pixel) {
+    const uint32_t hi = __byte_perm(pixel, box, 0x7610), lo = __byte_perm(box, pixel, 0x7610);
+    return ((hi - lo) & 0x80808080u) == 0x80808080u;
+}
 
 /* Flag word (wf.w bits): 1 live, 2 front facing, bits 2-5 pipeline index in
  * the module, bits 6-7 provoking-vertex slot (3: a line), bits 8-31 draw
@@ -141,15 +171,14 @@ __device__ __forceinline__ bool cpv_covers(const CpvTri& t, float xf, float yf, 
     return !(w[0] < 0.0f || w[1] < 0.0f || w[2] < 0.0f);
 }
 
-/* Tile rectangle of a set-up primitive (empty when culled, off screen, or
+/* Tile rectangle of a set-up primitive with pixel box b (empty when culled, off screen, or
  * when a bounding box of at most four pixels covers none of its pixel
  * centres — the raster would find no fragment there either). Packed as
  * x0 | y0 << 16, x1 | y1 << 16 in tile units, end exclusive. */
-__device__ __forceinline__ uint2 cpv_tile_rect(const CpvTri& t, float vw, float vh, const float* ndc_x = nullptr, const float* ndc_y = nullptr) {
+__device__ __forceinline__ uint2 cpv_tile_rect(const CpvTri& t, int4 b, float vw, float vh, const float* ndc_x = nullptr, const float* ndc_y = nullptr) {
     uint32_t r[4] = {0, 0, 0, 0};
     if (cpv_tri_live(t)) {
         bool any = true;
-        const int4 b = t.box;
         if ((b.z - b.x) * (b.w - b.y) <= 4) {
             /* pixel centres from the tables when given (the box lies inside
              * the attachment), else computed */
@@ -181,14 +210,14 @@ __device__ __forceinline__ uint2 cpv_tile_rect(const CpvTri& t, float vw, float 
  * picked by the signs of dy and dx; if that value is negative, every pixel
  * of the rectangle fails the edge and none is covered. Exact: it only
  * drops pixels the coverage test rejects. Edges with a non-finite
- * coefficient keep the primitive (NaN counts as covered). col/row hold the
- * tile's pixel-centre NDC values, indexed from (tile_x0, tile_y0). */
+ * coefficient keep the primitive (NaN counts as covered). The rectangle is
+ * relative to the tile; col/row hold the tile's pixel-centre NDC values. */
 __device__ __forceinline__ bool cpv_may_cover(const CpvTri& t, int32_t rx0, int32_t ry0, int32_t rx1, int32_t ry1, const float* col,
-                                              const float* row, int32_t tile_x0, int32_t tile_y0) {
+                                              const float* row) {
     /* the pixel-centre sequences are monotonic (in either direction for a
      * negative extent): their extremes over a range are its ends */
-    const float c0 = col[rx0 - tile_x0], c1 = col[rx1 - 1 - tile_x0];
-    const float r0 = row[ry0 - tile_y0], r1 = row[ry1 - 1 - tile_y0];
+    const float c0 = col[rx0], c1 = col[rx1 - 1];
+    const float r0 = row[ry0], r1 = row[ry1 - 1];
     const float xa = fminf(c0, c1), xb = fmaxf(c0, c1), ya = fminf(r0, r1), yb = fmaxf(r0, r1);
     if (!(fabsf(c0) <= 3.4e38f && fabsf(c1) <= 3.4e38f && fabsf(r0) <= 3.4e38f && fabsf(r1) <= 3.4e38f)) return true;
     bool may = true;
@@ -222,12 +251,12 @@ __device__ __forceinline__ bool cpv_may_cover(const CpvTri& t, int32_t rx0, int3
  * every pixel (a NaN corner value, a non-finite coefficient or a line's
  * fourth edge gives false, and the pixels are then tested one by one). */
 __device__ __forceinline__ bool cpv_must_cover(const CpvTri& t, int32_t rx0, int32_t ry0, int32_t rx1, int32_t ry1, const float* col,
-                                               const float* row, int32_t tile_x0, int32_t tile_y0) {
+                                               const float* row) {
 #if CPV_ANY_LINES
     if (((__float_as_uint(t.wf.w) >> 6) & 3u) == 3u) return false;
 #endif
-    const float c0 = col[rx0 - tile_x0], c1 = col[rx1 - 1 - tile_x0];
-    const float r0 = row[ry0 - tile_y0], r1 = row[ry1 - 1 - tile_y0];
+    const float c0 = col[rx0], c1 = col[rx1 - 1];
+    const float r0 = row[ry0], r1 = row[ry1 - 1];
     const float xa = fminf(c0, c1), xb = fmaxf(c0, c1), ya = fminf(r0, r1), yb = fmaxf(r0, r1);
     if (!(fabsf(c0) <= 3.4e38f && fabsf(c1) <= 3.4e38f && fabsf(r0) <= 3.4e38f && fabsf(r1) <= 3.4e38f)) return false;
     bool must = true;
@@ -373,16 +402,12 @@ __device__ __forceinline__ uint32_t cpv_block_scan(uint32_t v, uint32_t& total, 
     return base + incl - v;
 }
 
-/* Sparse schedule: class of a primitive in the tile — 0 dead or outside the
- * tile, 1 small (its bounding box covers at most CPV_SMALL_PX pixels of the
- * tile), 2 large. */
-__device__ __forceinline__ uint32_t cpv_tile_class(const CpvTri& t, int32_t tile_x0, int32_t tile_y0) {
-    if (!cpv_tri_live(t)) return 0u;
-    const int4 box = t.box;
-    const int32_t x0 = max(box.x, tile_x0), x1 = min(box.z, tile_x0 + CPV_TILE);
-    const int32_t y0 = max(box.y, tile_y0), y1 = min(box.w, tile_y0 + CPV_TILE);
-    if (x1 <= x0 || y1 <= y0) return 0u;
-    return (x1 - x0) * (y1 - y0) > CPV_SMALL_PX ? 2u : 1u;
+/* Sparse schedule: class of a primitive in the tile by its box — 0 dead or
+ * outside the tile, 1 small (at most CPV_SMALL_PX pixels of the tile), 2
+ * large. */
+__device__ __forceinline__ uint32_t cpv_tile_class(uint32_t box) {
+    const int32_t px = (cpv_box_x1(box) - cpv_box_x0(box)) * (cpv_box_y1(box) - cpv_box_y0(box));
+    return px == 0 ? 0u : (px > CPV_SMALL_PX ? 2u : 1u);
 }
 
 /* Sparse schedule: the small primitives j0 .. j0 + 31 of a batch (one per
@@ -394,18 +419,16 @@ __device__ __forceinline__ uint32_t cpv_tile_class(const CpvTri& t, int32_t tile
  * binary search over the lanes' sums) and is pixel i - (that lane's
  * exclusive sum) of its box, row-major. A pixel's list is applied in batch
  * order whatever the order of its appends. */
-__device__ __forceinline__ void cpv_list_small_warp(const CpvTri* tris, uint32_t j0, uint32_t n, int32_t tile_x0, int32_t tile_y0,
-                                                    const float* col_ndc, const float* row_ndc, uint32_t* list_count, uint8_t* list_j) {
+__device__ __forceinline__ void cpv_list_small_warp(const CpvTri* tris, const uint32_t* boxes, uint32_t j0, uint32_t n, const float* col_ndc,
+                                                     const float* row_ndc, uint32_t* list_count, uint8_t* list_j) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t j = j0 + lane;
     uint32_t size = 0u, geo = 0u, magic = 0u;
-    if (j < n && cpv_tile_class(tris[j], tile_x0, tile_y0) == 1u) {
-        const int4 box = tris[j].box;
-        const int32_t x0 = max(box.x, tile_x0), x1 = min(box.z, tile_x0 + CPV_TILE);
-        const int32_t y0 = max(box.y, tile_y0), y1 = min(box.w, tile_y0 + CPV_TILE);
-        const uint32_t bw = static_cast<uint32_t>(x1 - x0);
-        size = bw * static_cast<uint32_t>(y1 - y0);
-        geo = static_cast<uint32_t>(x0 - tile_x0) | (static_cast<uint32_t>(y0 - tile_y0) << 8) | (bw << 16);
+    const uint32_t box = j < n ? boxes[j] : CPV_BOX_DEAD;
+    if (cpv_tile_class(box) == 1u) {
+        const uint32_t bw = static_cast<uint32_t>(cpv_box_x1(box) - cpv_box_x0(box));
+        size = bw * static_cast<uint32_t>(cpv_box_y1(box) - cpv_box_y0(box));
+        geo = (box & 0xFFFFu) | (bw << 16);
         /* row = (k * magic) >> 16 = floor(k / bw) for every k < 1024 and bw
          * <= 32: magic = ceil(2^16 / bw) exceeds 2^16 / bw by less than 1,
          * so the product exceeds k * 2^16 / bw by less than k < 2^16 / 64,
@@ -447,13 +470,13 @@ __device__ __forceinline__ void cpv_list_small_warp(const CpvTri* tris, uint32_t
     }
 }
 
-/* Dynamic shared memory of the raster kernels: CPV_BATCH primitives, then
- * the schedule's buffers (deferred: fragment slots; sparse: per-pixel
+/* Dynamic shared memory of the raster kernels: CPV_BATCH primitives and
+ * their boxes in the tile, then the schedule's buffers (deferred: fragment slots; sparse: per-pixel
  * primitive lists, pixel-centre tables, the large-primitive list). */
 #define CPV_TILE_PX (CPV_TILE * CPV_TILE)
 #define CPV_SPARSE_BYTES (4u * CPV_TILE_PX + CPV_TILE_PX * CPV_SLOT_DEPTH + CPV_BATCH)
 #define CPV_RASTER_SMEM_BYTES \
-    (CPV_BATCH * sizeof(CpvTri) + (CPV_DEFERRED ? CPV_NSLOT * (4u + 20u + 2u) : 0u) + (CPV_SPARSE ? CPV_SPARSE_BYTES : 0u))
+    (CPV_BATCH * (sizeof(CpvTri) + 4u) + (CPV_DEFERRED ? CPV_NSLOT * (4u + 20u + 2u) : 0u) + (CPV_SPARSE ? CPV_SPARSE_BYTES : 0u))
 
 /* One screen tile (tx, ty) whose first batch holds `first` > 0 primitives:
  * loads the tile's attachment texels into registers, walks the tile's
@@ -463,7 +486,7 @@ __device__ __forceinline__ void cpv_list_small_warp(const CpvTri* tris, uint32_t
  *
  * Source supplies:
  *   uint32_t next(uint32_t* warp_sums)       the size of the tile's next batch (up to CPV_BATCH; 0: done)
- *   void setup(uint32_t i, CpvTri& t)        set up the batch's i-th primitive (or mark it dead)
+ *   void setup(uint32_t i, CpvTri& t, int4& box)  set up the batch's i-th primitive and its pixel box (or mark it dead)
  *   bool shade(const CpvTri&, const float w[3], int x, int y, float colour[CPV_COLOUR_FLOATS], float& mapped, const CpvPixel* early)
  *                                            (true: discarded, or failed the early depth
  *                                            test against *early when given)
@@ -507,7 +530,9 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
         col_ndc[i] = cpv_pixel_ndc(tile_x0 + static_cast<int32_t>(i), src.vw);
         row_ndc[i] = cpv_pixel_ndc(tile_y0 + static_cast<int32_t>(i), src.vh);
     }
+    uint32_t* boxes = reinterpret_cast<uint32_t*>(tris + CPV_BATCH);  /* per primitive: its box in the tile */
     int32_t px[CPV_PPT], py[CPV_PPT];
+    uint32_t bp[CPV_PPT];  /* the pixel as cpv_in_box takes it */
     float xf[CPV_PPT], yf[CPV_PPT];
     bool inside[CPV_PPT];
     CpvPixel st[CPV_PPT];
@@ -522,6 +547,7 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
         px[k] = static_cast<int32_t>(tx * CPV_TILE + (threadIdx.x % CPV_TILE));
         py[k] = static_cast<int32_t>(ty * CPV_TILE + (threadIdx.x / CPV_TILE) + k * CPV_ROWS_PER_PASS);
 #endif
+        bp[k] = cpv_box_pixel(static_cast<uint32_t>(px[k] - tile_x0), static_cast<uint32_t>(py[k] - tile_y0));
         inside[k] = px[k] < static_cast<int32_t>(src.fb_width) && py[k] < static_cast<int32_t>(src.fb_height);
         xf[k] = cpv_pixel_ndc(px[k], src.vw);
         yf[k] = cpv_pixel_ndc(py[k], src.vh);
@@ -529,14 +555,14 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
     }
 
 #if CPV_DEFERRED
-    uint8_t* slot_base = reinterpret_cast<uint8_t*>(tris + CPV_BATCH);
+    uint8_t* slot_base = reinterpret_cast<uint8_t*>(boxes + CPV_BATCH);
     uint32_t* slot_jk = reinterpret_cast<uint32_t*>(slot_base);          /* batch index | pixel k << 8 | discard << 31 */
     float* slot_f = reinterpret_cast<float*>(slot_jk + CPV_NSLOT);       /* 5 floats per slot: w0 w1 w2 → rgba + mapped */
     uint16_t* dense = reinterpret_cast<uint16_t*>(slot_f + 5 * CPV_NSLOT);
 #endif
 #if CPV_SPARSE
     static_assert(CPV_BATCH <= 256, "batch indices are stored in bytes");
-    uint32_t* list_count = reinterpret_cast<uint32_t*>(tris + CPV_BATCH);  /* per tile pixel: fragments listed this batch */
+    uint32_t* list_count = boxes + CPV_BATCH;  /* per tile pixel: fragments listed this batch */
     uint8_t* list_j = reinterpret_cast<uint8_t*>(list_count + CPV_TILE_PX);  /* per tile pixel: CPV_SLOT_DEPTH batch indices */
     uint8_t* large = list_j + CPV_TILE_PX * CPV_SLOT_DEPTH;                  /* batch indices of large primitives, in order */
     for (uint32_t i = threadIdx.x; i < CPV_TILE_PX; i += CPV_RT_THREADS) list_count[i] = 0u;
@@ -550,10 +576,10 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
      * (batch index; bit 15: the primitive covers the warp's whole block) */
     __shared__ uint16_t warp_list[(CPV_RT_THREADS / 32) * CPV_BATCH];
 #if CPV_WARP_BLOCKS
-    const int32_t warp_x0 = static_cast<int32_t>(tx * CPV_TILE + ((threadIdx.x >> 5) % (CPV_TILE / CPV_BLOCK_W)) * CPV_BLOCK_W);
-    const int32_t warp_y0 = static_cast<int32_t>(ty * CPV_TILE + ((threadIdx.x >> 5) / (CPV_TILE / CPV_BLOCK_W)) * CPV_BLOCK_H);
+    const int32_t warp_x0 = static_cast<int32_t>(((threadIdx.x >> 5) % (CPV_TILE / CPV_BLOCK_W)) * CPV_BLOCK_W);
+    const int32_t warp_y0 = static_cast<int32_t>(((threadIdx.x >> 5) / (CPV_TILE / CPV_BLOCK_W)) * CPV_BLOCK_H);
 #else
-    const int32_t warp_y0 = static_cast<int32_t>(ty * CPV_TILE + ((threadIdx.x & ~31u) / CPV_TILE));
+    const int32_t warp_y0 = static_cast<int32_t>((threadIdx.x & ~31u) / CPV_TILE);
 #endif
 #endif
 
@@ -565,16 +591,16 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
          * is left to the pixel tests, which is cheaper for small primitives */
         for (uint32_t i = threadIdx.x; i < n; i += CPV_RT_THREADS) {
             CpvTri& t = tris[i];
-            src.setup(i, t);
-            const int4 b = t.box;
-            if (cpv_tri_live(t) && (b.x < tile_x0 || b.y < tile_y0 || b.z > tile_x0 + CPV_TILE || b.w > tile_y0 + CPV_TILE)) {
-                const int32_t rx0 = max(b.x, tile_x0), ry0 = max(b.y, tile_y0);
-                const int32_t rx1 = min(b.z, tile_x0 + CPV_TILE), ry1 = min(b.w, tile_y0 + CPV_TILE);
-                /* worth a test when the primitive spans much of the tile */
-                if (rx1 <= rx0 || ry1 <= ry0 ||
-                    ((rx1 - rx0) * (ry1 - ry0) >= CPV_TILE_PX / 8 && !cpv_may_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc, tile_x0, tile_y0)))
-                    t.wf.w = __uint_as_float(__float_as_uint(t.wf.w) & ~1u);
-            }
+            int4 b = make_int4(0, 0, 0, 0);
+            src.setup(i, t, b);
+            const int32_t rx0 = max(b.x - tile_x0, 0), ry0 = max(b.y - tile_y0, 0);
+            const int32_t rx1 = min(b.z - tile_x0, CPV_TILE), ry1 = min(b.w - tile_y0, CPV_TILE);
+            bool live = cpv_tri_live(t) && rx1 > rx0 && ry1 > ry0;
+            /* worth a test when the primitive spans much of the tile */
+            if (live && (b.x < tile_x0 || b.y < tile_y0 || b.z > tile_x0 + CPV_TILE || b.w > tile_y0 + CPV_TILE) &&
+                (rx1 - rx0) * (ry1 - ry0) >= CPV_TILE_PX / 8)
+                live = cpv_may_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc);
+            boxes[i] = live ? cpv_box_pack(rx0, ry0, rx1, ry1) : CPV_BOX_DEAD;
         }
         __syncthreads();
 #if CPV_SPARSE
@@ -584,7 +610,7 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
         uint32_t nlarge = 0u;
         for (uint32_t round = 0; round < n; round += CPV_RT_THREADS) {
             const uint32_t j = round + threadIdx.x;
-            const uint32_t is_large = j < n && cpv_tile_class(tris[j], tile_x0, tile_y0) == 2u ? 1u : 0u;
+            const uint32_t is_large = j < n && cpv_tile_class(boxes[j]) == 2u ? 1u : 0u;
             uint32_t round_large;
             const uint32_t lpos = cpv_block_scan(is_large, round_large, warp_sums);
             if (is_large) large[nlarge + lpos] = static_cast<uint8_t>(j);
@@ -596,16 +622,15 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
         if (!immediate_batch) {
             /* 2. small primitives: each warp lists the pixels its 32 cover */
             for (uint32_t j0 = threadIdx.x & ~31u; j0 < n; j0 += CPV_RT_THREADS)
-                cpv_list_small_warp(tris, j0, n, tile_x0, tile_y0, col_ndc, row_ndc, list_count, list_j);
+                cpv_list_small_warp(tris, boxes, j0, n, col_ndc, row_ndc, list_count, list_j);
             /* 3. large primitives, in order: every pixel's thread tests its pixels */
             for (uint32_t m = 0; m < nlarge; m++) {
                 const uint32_t j = large[m];
                 const CpvTri& t = tris[j];
-                const int4 box = t.box;
+                const uint32_t box = boxes[j];
 #pragma unroll
                 for (int k = 0; k < CPV_PPT; k++) {
-                    if (!inside[k]) continue;
-                    if (px[k] < box.x || px[k] >= box.z || py[k] < box.y || py[k] >= box.w) continue;
+                    if (!cpv_in_box(box, bp[k])) continue;
                     float w[3];
                     if (!cpv_covers(t, xf[k], yf[k], w)) continue;
                     const uint32_t s = atomicAdd(&list_count[lp[k]], 1u);
@@ -638,10 +663,8 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
                 } else {
                     /* list overflow: walk the whole batch for this pixel */
                     for (uint32_t j = 0; j < n; j++) {
+                        if (!cpv_in_box(boxes[j], bp[k])) continue;
                         const CpvTri& t = tris[j];
-                        if (!cpv_tri_live(t)) continue;
-                        const int4 box = t.box;
-                        if (px[k] < box.x || px[k] >= box.z || py[k] < box.y || py[k] >= box.w) continue;
                         float w[3], colour[CPV_COLOUR_FLOATS], mapped;
                         if (!cpv_covers(t, xf[k], yf[k], w)) continue;
                         if (src.shade(t, w, px[k], py[k], colour, mapped, &st[k])) continue;
@@ -669,27 +692,27 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
                 const uint32_t j = b + lane;
                 bool hit = false;
                 uint32_t full = 0u;
-                if (j < n && cpv_tri_live(tris[j])) {
+                if (j < n) {
                     const CpvTri& t = tris[j];
-                    const int4 box = t.box;
+                    const uint32_t box = boxes[j];  /* a dead primitive's is empty */
 #if CPV_WARP_BLOCKS
                     /* the warp's block, within the box */
-                    const int32_t rx0 = max(box.x, warp_x0), rx1 = min(box.z, warp_x0 + CPV_BLOCK_W);
-                    const int32_t ry0 = max(box.y, warp_y0), ry1 = min(box.w, warp_y0 + CPV_BLOCK_H);
-                    hit = rx1 > rx0 && ry1 > ry0 && cpv_may_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc, tile_x0, tile_y0);
+                    const int32_t rx0 = max(cpv_box_x0(box), warp_x0), rx1 = min(cpv_box_x1(box), warp_x0 + CPV_BLOCK_W);
+                    const int32_t ry0 = max(cpv_box_y0(box), warp_y0), ry1 = min(cpv_box_y1(box), warp_y0 + CPV_BLOCK_H);
+                    hit = rx1 > rx0 && ry1 > ry0 && cpv_may_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc);
                     /* a block inside the box (so inside the attachment) and
                      * inside every edge: its pixels skip the box and edge tests */
                     if (hit && rx0 == warp_x0 && rx1 == warp_x0 + CPV_BLOCK_W && ry0 == warp_y0 && ry1 == warp_y0 + CPV_BLOCK_H &&
-                        cpv_must_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc, tile_x0, tile_y0))
+                        cpv_must_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc))
                         full = 0x8000u;
 #else
-                    const int32_t rx0 = max(box.x, tile_x0), rx1 = min(box.z, tile_x0 + CPV_TILE);
+                    const int32_t rx0 = cpv_box_x0(box), rx1 = cpv_box_x1(box);
 #pragma unroll
                     for (int k = 0; k < CPV_PPT; k++) {
                         /* the warp's rows of pass k, within the box */
-                        const int32_t ry0 = max(box.y, warp_y0 + k * CPV_ROWS_PER_PASS);
-                        const int32_t ry1 = min(box.w, warp_y0 + k * CPV_ROWS_PER_PASS + CPV_WARP_ROWS);
-                        hit = hit || (ry1 > ry0 && cpv_may_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc, tile_x0, tile_y0));
+                        const int32_t ry0 = max(cpv_box_y0(box), warp_y0 + k * CPV_ROWS_PER_PASS);
+                        const int32_t ry1 = min(cpv_box_y1(box), warp_y0 + k * CPV_ROWS_PER_PASS + CPV_WARP_ROWS);
+                        hit = hit || (ry1 > ry0 && cpv_may_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc));
                     }
 #endif
                 }
@@ -719,14 +742,12 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
 #endif
 #else
                 const uint32_t j = m;
-                if (!cpv_tri_live(tris[j])) continue;
 #endif
                 const CpvTri& t = tris[j];
-                const int4 box = t.box;
+                const uint32_t box = boxes[j];
 #pragma unroll
                 for (int k = 0; k < CPV_PPT; k++) {
-                    if (!inside[k]) continue;
-                    if (px[k] < box.x || px[k] >= box.z || py[k] < box.y || py[k] >= box.w) continue;
+                    if (!cpv_in_box(box, bp[k])) continue;
                     float w[3];
                     if (!cpv_covers(t, xf[k], yf[k], w)) continue;
                     if (src.table_fragment(t, st[k])) continue;
@@ -746,15 +767,12 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
                 const uint32_t j = cursor / CPV_PPT, k = cursor - j * CPV_PPT;
                 cursor++;
                 const CpvTri& t = tris[j];
-                if (!cpv_tri_live(t)) continue;
-                int32_t pxk = px[0], pyk = py[0];
+                uint32_t bpk = bp[0];
                 float xfk = xf[0], yfk = yf[0];
-                bool ink = inside[0];
 #pragma unroll
                 for (int kk = 1; kk < CPV_PPT; kk++)
-                    if (k == static_cast<uint32_t>(kk)) { pxk = px[kk]; pyk = py[kk]; xfk = xf[kk]; yfk = yf[kk]; ink = inside[kk]; }
-                const int4 box = t.box;
-                if (!ink || pxk < box.x || pxk >= box.z || pyk < box.y || pyk >= box.w) continue;
+                    if (k == static_cast<uint32_t>(kk)) { bpk = bp[kk]; xfk = xf[kk]; yfk = yf[kk]; }
+                if (!cpv_in_box(boxes[j], bpk)) continue;
                 float w[3];
                 if (!cpv_covers(t, xfk, yfk, w)) continue;
                 const uint32_t s = threadIdx.x * CPV_SLOTS + cnt;

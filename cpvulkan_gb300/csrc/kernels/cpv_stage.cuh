@@ -78,7 +78,7 @@ __device__ __forceinline__ void cpv_shade_constant(const CpvDrawParams& P, const
  * evaluating the reference's expression at the candidate range's ends; it
  * becomes the box, and the zero edges cover every pixel in it. */
 template <bool WITH_VARYINGS>
-__device__ __forceinline__ void cpv_setup(const CpvDrawParams& P, uint64_t g, CpvTri& t) {
+__device__ __forceinline__ void cpv_setup(const CpvDrawParams& P, uint64_t g, CpvTri& t, int4& box) {
     const uint32_t ppi = P.prims_per_instance;
     const uint32_t g32 = static_cast<uint32_t>(g);
     const uint32_t inst = P.instance_count > 1u ? g32 / ppi : 0u;
@@ -106,7 +106,7 @@ __device__ __forceinline__ void cpv_setup(const CpvDrawParams& P, uint64_t g, Cp
     while (yb < ye && !inside(yb - sy)) yb++;
     while (ye > yb && !inside(ye - 1 - sy)) ye--;
     bool live = xe > xb && ye > yb && size == size;
-    t.box = make_int4(static_cast<int32_t>(xb), static_cast<int32_t>(yb), static_cast<int32_t>(live ? xe : xb), static_cast<int32_t>(live ? ye : yb));
+    box = make_int4(static_cast<int32_t>(xb), static_cast<int32_t>(yb), static_cast<int32_t>(live ? xe : xb), static_cast<int32_t>(live ? ye : yb));
 #pragma unroll
     for (int k = 0; k < 3; k++) t.e[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     t.za = make_float4(nz, 0.0f, 0.0f, 1.0f);
@@ -125,7 +125,7 @@ __device__ __forceinline__ void cpv_setup(const CpvDrawParams& P, uint64_t g, Cp
  * (the edge tests decide coverage; the reference tests every viewport
  * pixel, and pixels that far outside the quad fail an edge). */
 template <bool WITH_VARYINGS>
-__device__ __forceinline__ void cpv_setup(const CpvDrawParams& P, uint64_t g, CpvTri& t) {
+__device__ __forceinline__ void cpv_setup(const CpvDrawParams& P, uint64_t g, CpvTri& t, int4& box) {
     static_assert(CPV_ANY_LINES && CPV_NV_PAD >= 7, "a module with line pipelines defines CPV_ANY_LINES");
     const uint32_t ppi = P.prims_per_instance;
     const uint32_t g32 = static_cast<uint32_t>(g);
@@ -195,7 +195,7 @@ __device__ __forceinline__ void cpv_setup(const CpvDrawParams& P, uint64_t g, Cp
         y1 = min(y1, hi(maxy, vh));
     }
     bool live = !nan && x1 > x0 && y1 > y0;
-    t.box = make_int4(static_cast<int32_t>(x0), static_cast<int32_t>(y0), static_cast<int32_t>(live ? x1 : x0), static_cast<int32_t>(live ? y1 : y0));
+    box = make_int4(static_cast<int32_t>(x0), static_cast<int32_t>(y0), static_cast<int32_t>(live ? x1 : x0), static_cast<int32_t>(live ? y1 : y0));
     const float dx = __fsub_rn(Pn[1][0], Pn[0][0]), dy = __fsub_rn(Pn[1][1], Pn[0][1]);
     const float len = __fsqrt_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)));
     if (WITH_VARYINGS) cpv_shade_constant<WITH_VARYINGS>(P, t.var[0], true, g32, t, live);
@@ -222,12 +222,51 @@ __device__ __forceinline__ void cpv_vertex_ndc(const CpvDrawParams& P, uint32_t 
     Pn[3] = w;
 }
 
+#if CPV_QUICK_DIV
+/* The divisors of a triangle's interpolation — area, and with perspective
+ * varyings the clip w of its vertices — as correctly rounded reciprocals, so
+ * that its fragments divide with cpv_div_by: an IEEE division costs a
+ * fragment about 15 instructions, and a perspective fragment has
+ * 6 + 4 per component of them. Ranges that rule out overflow and underflow
+ * for weights within [2^-40, 2^20], which cpv_tri_weights checks: |w| in
+ * [2^-20, 2^20], area in [2^-50, 2^40], varyings zero or in [2^-40, 2^20]; any
+ * other triangle gets rc.w = 0 and divides. t.za.w and t.var hold the
+ * triangle's values. */
+__device__ __forceinline__ void cpv_tri_reciprocals(const float Pn[3][4], CpvTri& t) {
+    bool perspective = false;
+    uint32_t least = 0xFFFFFFFFu;  /* smallest bit pattern x 2 - 1 of a varying: zero wraps to the largest */
+    float most = 0.0f;
+#pragma unroll
+    for (int c = 0; c < CPV_NV; c++) {
+        if (CPV_FS_CONSTANT || cpv_interp(c) != 0) continue;
+        perspective = true;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const float v = t.var[k][c];
+            least = min(least, __float_as_uint(v) * 2u - 1u);
+            most = fmaxf(most, v == v ? fabsf(v) : 3.0e38f);
+        }
+    }
+    const float area = t.za.w;
+    bool ok = area >= 0x1p-50f && area <= 0x1p40f && least >= 0x2B800000u * 2u - 1u && most <= 0x1p20f;
+    t.rc = make_float4(0.0f, 0.0f, 0.0f, __frcp_rn(area));
+    if (perspective) {
+        const float a = fabsf(Pn[0][3]), b = fabsf(Pn[1][3]), c = fabsf(Pn[2][3]);
+        ok = ok && a >= 0x1p-20f && a <= 0x1p20f && b >= 0x1p-20f && b <= 0x1p20f && c >= 0x1p-20f && c <= 0x1p20f;
+        t.rc.x = __frcp_rn(Pn[0][3]);
+        t.rc.y = __frcp_rn(Pn[1][3]);
+        t.rc.z = __frcp_rn(Pn[2][3]);
+    }
+    if (!ok) t.rc.w = 0.0f;
+}
+#endif
+
 /* The per-triangle part of the set-up from its three vertices (after the CW
  * swap): screen bounding box, area, facing and cull, and with varyings the
  * constant fragment colour. t.var must hold the vertices' outputs when
  * WITH_VARYINGS. */
 template <bool WITH_VARYINGS>
-__device__ __forceinline__ void cpv_setup_tri(const CpvDrawParams& P, const float Pn[3][4], uint32_t pslot, uint32_t g32, CpvTri& t) {
+__device__ __forceinline__ void cpv_setup_tri(const CpvDrawParams& P, const float Pn[3][4], uint32_t pslot, uint32_t g32, CpvTri& t, int4& box) {
     const float vw = P.viewport[2], vh = P.viewport[3];
     int32_t sx[3], sy[3];
 #pragma unroll
@@ -246,12 +285,10 @@ __device__ __forceinline__ void cpv_setup_tri(const CpvDrawParams& P, const floa
     y1 = y1 < ih ? y1 : ih;
     x1 = x1 < static_cast<int64_t>(P.fb_width) ? x1 : static_cast<int64_t>(P.fb_width);
     y1 = y1 < static_cast<int64_t>(P.fb_height) ? y1 : static_cast<int64_t>(P.fb_height);
-    int4 box;
     box.x = static_cast<int32_t>(x0);
     box.y = static_cast<int32_t>(y0);
     box.z = static_cast<int32_t>(x1 > x0 ? x1 : x0);
     box.w = static_cast<int32_t>(y1 > y0 ? y1 : y0);
-    t.box = box;
 
     float area = cpv_edge(Pn[0][0], Pn[0][1], Pn[1][0], Pn[1][1], Pn[2][0], Pn[2][1]);
     /* Edges (a → b): front (area >= 0) w0 = E(p1,p2), w1 = E(p2,p0), w2 = E(p0,p1);
@@ -275,7 +312,12 @@ __device__ __forceinline__ void cpv_setup_tri(const CpvDrawParams& P, const floa
     /* a fragment shader reading only flat inputs (the provoking vertex's)
      * gives every fragment of the primitive one colour; a discard discards
      * them all */
-    if (WITH_VARYINGS) cpv_shade_constant<WITH_VARYINGS>(P, t.var[pslot], front, g32, t, live);
+    if (WITH_VARYINGS) {
+#if CPV_QUICK_DIV
+        cpv_tri_reciprocals(Pn, t);
+#endif
+        cpv_shade_constant<WITH_VARYINGS>(P, t.var[pslot], front, g32, t, live);
+    }
     const uint32_t flags = (live ? 1u : 0u) | (front ? 2u : 0u) | (pslot << 6);
     t.wf = make_float4(Pn[0][3], Pn[1][3], Pn[2][3], __uint_as_float(flags));
 }
@@ -304,7 +346,7 @@ __device__ __forceinline__ void cpv_tri_vertices(const CpvDrawParams& P, uint32_
  * holds what cpv_vertex_ndc returns for the same vertex id and instance,
  * computed by the same function, so the bits are the same. */
 template <bool WITH_VARYINGS>
-__device__ __forceinline__ void cpv_setup(const CpvDrawParams& P, uint64_t g, CpvTri& t) {
+__device__ __forceinline__ void cpv_setup(const CpvDrawParams& P, uint64_t g, CpvTri& t, int4& box) {
     const uint32_t g32 = static_cast<uint32_t>(g);  /* draws hold < 2^32 primitives */
     uint32_t raw[3], instance, pslot, inst;
     cpv_tri_vertices(P, g32, raw, instance, pslot, inst);
@@ -350,13 +392,13 @@ __device__ __forceinline__ void cpv_setup(const CpvDrawParams& P, uint64_t g, Cp
         const float area = cpv_edge(Pn[0][0], Pn[0][1], Pn[1][0], Pn[1][1], Pn[2][0], Pn[2][1]);
         const bool front = !(area < 0.0f);
         if (((CPV_CULL_MODE & 2) && !front) || ((CPV_CULL_MODE & 1) && front)) {
-            t.box = make_int4(0, 0, 0, 0);
+            box = make_int4(0, 0, 0, 0);
             t.wf.w = __uint_as_float(0u);
             return;
         }
     }
 #endif
-    cpv_setup_tri<WITH_VARYINGS>(P, Pn, pslot, g32, t);
+    cpv_setup_tri<WITH_VARYINGS>(P, Pn, pslot, g32, t, box);
 }
 
 /* The vertex stage of the batched path: shades vertex id `vid` of
@@ -631,12 +673,50 @@ __device__ __forceinline__ float cpv_tri_depth(const CpvTri& t, const float w[3]
     return __fadd_rn(__fadd_rn(__fmul_rn(t.za.x, w[0]), __fmul_rn(t.za.y, w[1])), __fmul_rn(t.za.z, w[2]));
 }
 
+#if CPV_QUICK_DIV
+/* A triangle's barycentrics w_k / area from its edge functions, by the
+ * triangle's reciprocal of the area. False when that does not hold: a
+ * triangle without reciprocals, or weights outside the range
+ * cpv_tri_reciprocals counts on (a zero weight, whose sign matters,
+ * included). */
+__device__ __forceinline__ bool cpv_tri_weights(const CpvTri& t, const float wr[3], float w[3]) {
+    const float area = t.za.w, y = t.rc.w;
+#pragma unroll
+    for (int k = 0; k < 3; k++) w[k] = cpv_div_by(wr[k], area, y);
+    return y != 0.0f && fminf(fminf(w[0], w[1]), w[2]) >= 0x1p-40f && fmaxf(fmaxf(w[0], w[1]), w[2]) <= 0x1p20f;
+}
+#endif
+
 /* A triangle's varyings at barycentrics w: perspective Σ w·v/p ÷ Σ w/p,
  * linear Σ w·v, or flat from the provoking vertex
- * (CPVulkan/CommandBuffer.Draw.cpp:816-954). */
-__device__ __forceinline__ void cpv_tri_inputs(const CpvTri& t, const float w[3], float* in) {
+ * (CPVulkan/CommandBuffer.Draw.cpp:816-954). QUICK (cpv_tri_weights found
+ * the weights in range): the divisions by p use the triangle's reciprocals
+ * and the last one the reciprocal of the denominator; false when it or a
+ * numerator is out of range (|den| >= 2^-60, numerators zero or >= 2^-60). */
+template <bool QUICK>
+__device__ __forceinline__ bool cpv_tri_inputs(const CpvTri& t, const float w[3], float* in) {
     const float pw[3] = {t.wf.x, t.wf.y, t.wf.z};
     const uint32_t pslot = cpv_tri_pslot(t);
+#if CPV_QUICK_DIV
+    const float rp[3] = {t.rc.x, t.rc.y, t.rc.z};
+#else
+    const float rp[3] = {0.0f, 0.0f, 0.0f};
+#endif
+    float den = 0.0f, y = 0.0f;
+    uint32_t least = 0xFFFFFFFFu;
+    bool perspective = false;
+#pragma unroll
+    for (int c = 0; c < CPV_NV; c++) perspective = perspective || cpv_interp(c) == 0;
+    if (perspective) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            den = __fadd_rn(den, QUICK ? cpv_div_by(w[k], pw[k], rp[k]) : __fdiv_rn(w[k], pw[k]));
+        }
+        if (QUICK) {
+            y = __frcp_rn(den);
+            least = den == 0.0f ? 0u : __float_as_uint(den) * 2u - 1u;
+        }
+    }
 #pragma unroll
     for (int c = 0; c < CPV_NV; c++) {
         const int kind = cpv_interp(c);
@@ -648,15 +728,17 @@ __device__ __forceinline__ void cpv_tri_inputs(const CpvTri& t, const float w[3]
             for (int k = 0; k < 3; k++) r = __fadd_rn(r, __fmul_rn(w[k], t.var[k][c]));
             in[c] = r;
         } else {
-            float num = 0.0f, den = 0.0f;
+            float num = 0.0f;
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                num = __fadd_rn(num, __fdiv_rn(__fmul_rn(w[k], t.var[k][c]), pw[k]));
-                den = __fadd_rn(den, __fdiv_rn(w[k], pw[k]));
+                const float a = __fmul_rn(w[k], t.var[k][c]);
+                num = __fadd_rn(num, QUICK ? cpv_div_by(a, pw[k], rp[k]) : __fdiv_rn(a, pw[k]));
             }
-            in[c] = __fdiv_rn(num, den);
+            if (QUICK) least = min(least, __float_as_uint(num) * 2u - 1u);
+            in[c] = QUICK ? cpv_div_by(num, den, y) : __fdiv_rn(num, den);
         }
     }
+    return least >= 0x21800000u * 2u - 1u;
 }
 
 /* gl_FragCoord of pixel (x, y) at NDC depth `depth`. */
@@ -702,7 +784,7 @@ __device__ __forceinline__ void cpv_quad_helpers(const CpvDrawParams& P, const C
 #pragma unroll
         for (int k = 0; k < 3; k++) w[k] = __fdiv_rn(w[k], area);
         const float depth = cpv_tri_depth(t, w);
-        cpv_tri_inputs(t, w, in);
+        (void)cpv_tri_inputs<false>(t, w, in);  /* weights of any sign and size */
 #endif
         float fc[4], scratch[CPV_COLOUR_FLOATS];
         cpv_frag_coord(P, nx, ny, depth, fc);
@@ -713,13 +795,13 @@ __device__ __forceinline__ void cpv_quad_helpers(const CpvDrawParams& P, const C
 }
 #endif
 
-/* Shading of one covered pixel: barycentrics (w_k / area), screen-linear
- * depth, varyings (cpv_tri_inputs, cpv_line_inputs; a point's fragments
- * take its vertex's outputs as they are and its NDC z,
- * CPVulkan/CommandBuffer.Draw.cpp:1364-1374), viewport depth mapping
- * (:1300-1313) and the fragment shader. Returns true when the shader
- * discards, or when `early` (the pixel's current state) is given and the
- * fragment fails the early depth test. */
+/* Shading of one covered pixel: a triangle's barycentrics (w_k / area),
+ * screen-linear depth and varyings (cpv_tri_inputs), a line's
+ * (cpv_line_inputs); a point's fragments take its vertex's outputs as they
+ * are and its NDC z (CPVulkan/CommandBuffer.Draw.cpp:1364-1374); then the
+ * viewport depth mapping (:1300-1313) and the fragment shader. Returns true
+ * when the shader discards, or when `early` (the pixel's current state) is
+ * given and the fragment fails the early depth test. */
 __device__ __forceinline__ bool cpv_shade(const CpvDrawParams& P, const CpvTri& t, const float wr[3], int32_t x, int32_t y, float* colour,
                                           float& mapped, const CpvPixel* early = nullptr) {
     float in[CPV_NV_ALLOC];
@@ -732,11 +814,16 @@ __device__ __forceinline__ bool cpv_shade(const CpvDrawParams& P, const CpvTri& 
     (void)wr;
     const float depth = cpv_line_inputs(P, t, x, y, in);
 #else
-    const float area = t.za.w;
     float w[3];
-    w[0] = __fdiv_rn(wr[0], area);
-    w[1] = __fdiv_rn(wr[1], area);
-    w[2] = __fdiv_rn(wr[2], area);
+    bool quick = false;
+#if CPV_QUICK_DIV
+    quick = cpv_tri_weights(t, wr, w);
+#endif
+    if (!quick) {
+        const float area = t.za.w;
+#pragma unroll
+        for (int k = 0; k < 3; k++) w[k] = __fdiv_rn(wr[k], area);
+    }
     const float depth = cpv_tri_depth(t, w);
 #if CPV_EARLY_DEPTH
     if (early) {
@@ -746,7 +833,10 @@ __device__ __forceinline__ bool cpv_shade(const CpvDrawParams& P, const CpvTri& 
 #else
     (void)early;
 #endif
-    cpv_tri_inputs(t, w, in);
+#if CPV_QUICK_DIV
+    if (quick) quick = cpv_tri_inputs<true>(t, w, in);
+#endif
+    if (!quick) (void)cpv_tri_inputs<false>(t, w, in);
 #endif /* CPV_PRIM_KIND */
     const float min_d = P.viewport[4], max_d = P.viewport[5];
     mapped = __fadd_rn(__fmul_rn(__fsub_rn(max_d, min_d), depth), min_d);
@@ -943,7 +1033,7 @@ __device__ __forceinline__ void cpv_apply_table(const uint8_t* table, CpvPixel& 
  * dispatcher (cpv_dispatch) hands to generic code. */
 struct Stage {
     template <bool WITH_VARYINGS>
-    static __device__ __forceinline__ void setup(const CpvDrawParams& P, uint64_t g, CpvTri& t) { cpv_setup<WITH_VARYINGS>(P, g, t); }
+    static __device__ __forceinline__ void setup(const CpvDrawParams& P, uint64_t g, CpvTri& t, int4& box) { cpv_setup<WITH_VARYINGS>(P, g, t, box); }
     /* the vertex stage (triangle topologies only; the host gives other
      * draws no slots) */
     static __device__ __forceinline__ void vertex(const CpvDrawParams& P, uint32_t vid, uint32_t instance, uint64_t slot) {
