@@ -13,6 +13,16 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a GB300 (CUDA device)")
 
 
+def pytest_collection_modifyitems(items):
+    """The pinning tests compile the reference's own files: skipped where its
+    folder is there without them."""
+    if os.path.isfile("/root/reference/CPVulkan/CommandBuffer.Draw.cpp"):
+        return
+    for item in items:
+        if item.path.name == "test_oracle_pinned.py":
+            item.add_marker(pytest.mark.skip(reason="the reference sources are not on this machine"))
+
+
 @pytest.fixture(scope="session")
 def native():
     import cpvulkan_gb300 as c
