@@ -90,6 +90,8 @@ struct BoundVertex {
 };
 
 struct State {
+    Device* device = nullptr;
+    const std::vector<WrittenRange>* written = nullptr;  // by the submission so far
     Pipeline* pipeline = nullptr;
     BoundVertex vertex[8];
     Buffer* index = nullptr;
@@ -107,6 +109,19 @@ struct State {
     uint32_t subpass = 0;  // index into pass->subpasses
     const Subpass& sub() const { return pass->subpasses[subpass]; }
 };
+
+void wrote_image(std::vector<WrittenRange>& written, const Image* img) {
+    if (img->memory) written.push_back({img->memory, img->offset, img->offset + img->total_size, false});
+}
+
+void wrote_buffer(std::vector<WrittenRange>& written, const Buffer* b, uint64_t at, uint64_t size) {
+    if (b->memory && size) written.push_back({b->memory, b->offset + at, b->offset + at + size, false});
+}
+
+// A command reads `b`, after what the submission has `written` so far.
+void reads(Device* dev, const Buffer* b, const std::vector<WrittenRange>* written) {
+    if (b && b->memory && b->memory->host && !b->memory->device_reads) require_upload(dev, b->memory, written);
+}
 
 // Resolves the (set, binding) → dynamic offset index: dynamic descriptors are
 // numbered in binding order within the set (Vulkan rule).
@@ -236,7 +251,7 @@ VkResult clear_rect(Queue* q, Image* img, uint32_t layer, uint32_t level, VkImag
                : VK_ERROR_DEVICE_LOST;
 }
 
-VkResult begin_render_pass(Queue* q, State& s, const Cmd& c, std::vector<DeviceMemory*>& written) {
+VkResult begin_render_pass(Queue* q, State& s, const Cmd& c, std::vector<WrittenRange>& written) {
     s.pass = static_cast<RenderPass*>(c.p[0]);
     s.fb = static_cast<Framebuffer*>(c.p[1]);
     s.subpass = 0;
@@ -245,7 +260,7 @@ VkResult begin_render_pass(Queue* q, State& s, const Cmd& c, std::vector<DeviceM
         const auto& a = s.pass->attachments[i];
         ImageView* v = s.fb->attachments[i];
         if (!v || !v->image || !v->image->memory) continue;
-        written.push_back(v->image->memory);
+        wrote_image(written, v->image);
         // loadOp CLEAR clears colour or depth, stencilLoadOp CLEAR the
         // stencil (ClearImage → SetPixel through the format encoder,
         // CPVulkan/CommandBuffer.Draw.cpp:117-149)
@@ -273,11 +288,13 @@ VkResult build_draw(State& s, uint32_t count, uint32_t instances, uint32_t first
     for (int b = 0; b < 8; b++) {
         const BoundVertex& bv = s.vertex[b];
         if (!bv.buffer || !bv.buffer->memory) continue;
+        reads(s.device, bv.buffer, s.written);
         P.vb[b] = bv.buffer->device_ptr(bv.offset);
         P.vb_bytes[b] = bv.offset < bv.buffer->size ? bv.buffer->size - bv.offset : 0;
     }
     if (indexed) {
         if (!s.index || !s.index->memory) return VK_ERROR_DEVICE_LOST;
+        reads(s.device, s.index, s.written);
         P.ib = s.index->device_ptr(s.index_offset);
         P.ib_bytes = s.index_offset < s.index->size ? s.index->size - s.index_offset : 0;
         P.index_size = s.index_size;
@@ -314,6 +331,7 @@ VkResult build_draw(State& s, uint32_t count, uint32_t instances, uint32_t first
             const uint64_t off = d.offset + dyn;
             uint64_t range = d.range == VK_WHOLE_SIZE ? (d.buffer->size > off ? d.buffer->size - off : 0) : d.range;
             if (off + range > d.buffer->size) range = d.buffer->size > off ? d.buffer->size - off : 0;
+            reads(s.device, d.buffer, s.written);
             P.ubo[slot.slot] = d.buffer->device_ptr(off);
             P.ubo_bytes[slot.slot] = range;
         }
@@ -376,11 +394,13 @@ VkResult draw(Queue* q, State& s, uint32_t count, uint32_t instances, uint32_t f
 // `size` bytes of buffer `b` at `offset` as the queue's work up to now
 // leaves them: from the pinned mirror of host-visible memory the device has
 // not written, else from HBM after the queue's earlier work has finished.
-VkResult read_buffer(Queue* q, const Buffer* b, uint64_t offset, uint64_t size, const std::vector<DeviceMemory*>& written, uint8_t* out) {
+VkResult read_buffer(Queue* q, const Buffer* b, uint64_t offset, uint64_t size, const std::vector<WrittenRange>& written, uint8_t* out) {
     if (!b || !b->memory || offset + size > b->size) return VK_ERROR_DEVICE_LOST;
     DeviceMemory* m = b->memory;
     const uint64_t at = b->offset + offset;
-    const bool device_newer = !m->host || m->device_dirty || std::find(written.begin(), written.end(), m) != written.end();
+    const bool device_newer = !m->host || !m->dirty.empty() ||
+                              std::find_if(written.begin(), written.end(), [m](const WrittenRange& w) { return w.memory == m; }) != written.end();
+    if (device_newer) reads(q->device, b, &written);
     if (!device_newer) {
         std::memcpy(out, m->host + at, size);
     } else if (cudaStreamSynchronize(q->stream) != cudaSuccess || cudaMemcpy(out, m->device + at, size, cudaMemcpyDeviceToHost) != cudaSuccess) {
@@ -390,7 +410,7 @@ VkResult read_buffer(Queue* q, const Buffer* b, uint64_t offset, uint64_t size, 
     return VK_SUCCESS;
 }
 
-VkResult read_indirect(Queue* q, const Cmd& c, const std::vector<DeviceMemory*>& written, std::vector<IndirectDraw>& out) {
+VkResult read_indirect(Queue* q, const Cmd& c, const std::vector<WrittenRange>& written, std::vector<IndirectDraw>& out) {
     out.clear();
     const bool indexed = c.type == CmdType::DrawIndexedIndirect;
     uint32_t n = c.u[0];
@@ -418,7 +438,7 @@ VkResult read_indirect(Queue* q, const Cmd& c, const std::vector<DeviceMemory*>&
     return VK_SUCCESS;
 }
 
-VkResult draw_indirect(Queue* q, State& s, const Cmd& c, const std::vector<DeviceMemory*>& written, bool no_alloc) {
+VkResult draw_indirect(Queue* q, State& s, const Cmd& c, const std::vector<WrittenRange>& written, bool no_alloc) {
     std::vector<IndirectDraw> records;
     const VkResult rr = read_indirect(q, c, written, records);
     if (rr != VK_SUCCESS) return rr;
@@ -788,7 +808,7 @@ void build_batch(Queue* q, const CommandBuffer* cb, size_t begin, size_t end, co
 // pass to the per-draw path.
 // A pass with indirect draws reads their records at every submission; its
 // batch is rebuilt when they differ from the records it was built from.
-bool run_batched(Queue* q, CommandBuffer* cb, size_t begin, size_t end, State& s, const std::vector<DeviceMemory*>& written, VkResult& result) {
+bool run_batched(Queue* q, CommandBuffer* cb, size_t begin, size_t end, State& s, const std::vector<WrittenRange>& written, VkResult& result) {
     PassIndirect indirect;
     for (size_t i = begin + 1; i < end; i++) {
         if (!is_indirect(cb->cmds[i])) continue;
@@ -828,8 +848,10 @@ bool run_batched(Queue* q, CommandBuffer* cb, size_t begin, size_t end, State& s
 
 }  // namespace
 
-VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& written, bool no_alloc) {
+VkResult execute(Queue* q, CommandBuffer* cb, std::vector<WrittenRange>& written, bool no_alloc) {
     State s;
+    s.device = q->device;
+    s.written = &written;
     for (size_t idx = 0; idx < cb->cmds.size(); idx++) {
         const Cmd& c = cb->cmds[idx];
         if (apply_state(s, c)) continue;
@@ -849,12 +871,13 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& writte
         case CmdType::CopyBuffer: {
             Buffer* src = static_cast<Buffer*>(c.p[0]);
             Buffer* dst = static_cast<Buffer*>(c.p[1]);
+            reads(q->device, src, &written);
             for (const auto& reg : c.buffer_regions) {
                 if (reg.srcOffset + reg.size > src->size || reg.dstOffset + reg.size > dst->size) return VK_ERROR_DEVICE_LOST;
                 if (cudaMemcpyAsync(dst->device_ptr(reg.dstOffset), src->device_ptr(reg.srcOffset), reg.size, cudaMemcpyDeviceToDevice, q->stream) != cudaSuccess)
                     return VK_ERROR_DEVICE_LOST;
+                wrote_buffer(written, dst, reg.dstOffset, reg.size);
             }
-            written.push_back(dst->memory);
             break;
         }
         case CmdType::CopyBufferToImage:
@@ -862,6 +885,7 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& writte
             const bool to_image = c.type == CmdType::CopyBufferToImage;
             Buffer* buf = static_cast<Buffer*>(c.p[0]);
             Image* img = static_cast<Image*>(c.p[1]);
+            if (to_image) reads(q->device, buf, &written);
             for (const auto& reg : c.image_regions) {
                 const uint32_t level = reg.imageSubresource.mipLevel;
                 if (level >= img->levels) return VK_ERROR_DEVICE_LOST;
@@ -881,7 +905,16 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& writte
                         uint8_t* ip = img->device_ptr() + img_off;
                         uint8_t* bp = buf->device_ptr(buf_off);
                         cudaError_t e;
-                        if (to_image)
+                        const uint64_t row_bytes = static_cast<uint64_t>(row_len) * texel;
+                        if (!to_image) {
+                            /* rows with gaps: the copy back takes whole ranges, so the gaps have to be current in HBM */
+                            if (row_bytes != width_bytes && reg.imageExtent.height > 1 && buf->memory->host && !buf->memory->device_reads)
+                                require_upload(q->device, buf->memory, &written);
+                            wrote_buffer(written, buf, buf_off, row_bytes * (reg.imageExtent.height - 1) + width_bytes);
+                        }
+                        if (row_bytes == width_bytes && L.stride == width_bytes)  /* contiguous on both sides */
+                            e = cudaMemcpyAsync(to_image ? ip : bp, to_image ? bp : ip, width_bytes * reg.imageExtent.height, cudaMemcpyDeviceToDevice, q->stream);
+                        else if (to_image)
                             e = cudaMemcpy2DAsync(ip, L.stride, bp, static_cast<size_t>(row_len) * texel, width_bytes, reg.imageExtent.height, cudaMemcpyDeviceToDevice, q->stream);
                         else
                             e = cudaMemcpy2DAsync(bp, static_cast<size_t>(row_len) * texel, ip, L.stride, width_bytes, reg.imageExtent.height, cudaMemcpyDeviceToDevice, q->stream);
@@ -889,7 +922,7 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& writte
                     }
                 }
             }
-            written.push_back(to_image ? img->memory : buf->memory);
+            if (to_image) wrote_image(written, img);
             break;
         }
         case CmdType::BlitImage: {
@@ -925,7 +958,7 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& writte
                         return VK_ERROR_DEVICE_LOST;
                 }
             }
-            written.push_back(dst->memory);
+            wrote_image(written, dst);
             break;
         }
         case CmdType::CopyImage: {
@@ -962,7 +995,7 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& writte
                     }
                 }
             }
-            written.push_back(dst->memory);
+            wrote_image(written, dst);
             break;
         }
         case CmdType::ClearImage: {
@@ -981,7 +1014,7 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& writte
                         if (r != VK_SUCCESS) return r;
                     }
             }
-            written.push_back(img->memory);
+            wrote_image(written, img);
             break;
         }
         case CmdType::ClearAttachments: {
@@ -1004,7 +1037,7 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& writte
                                                       a.clearValue, rect.rect.offset.x, rect.rect.offset.y, rect.rect.extent.width, rect.rect.extent.height);
                         if (r != VK_SUCCESS) return r;
                     }
-                written.push_back(v->image->memory);
+                wrote_image(written, v->image);
             }
             break;
         }
@@ -1014,7 +1047,7 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& writte
             if (size == VK_WHOLE_SIZE) size = (dst->size - off) & ~3ull;
             if (off + size > dst->size) return VK_ERROR_DEVICE_LOST;
             if (rt::fill(q->stream, dst->device_ptr(off), size / 4, 4, c.u[0], 0) != rt::kOk) return VK_ERROR_DEVICE_LOST;
-            written.push_back(dst->memory);
+            wrote_buffer(written, dst, off, size);
             break;
         }
         case CmdType::UpdateBuffer: {
@@ -1024,7 +1057,7 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& writte
             // the copy is ordered on the stream.
             if (cudaMemcpyAsync(dst->device_ptr(c.q[0]), c.bytes.data(), c.bytes.size(), cudaMemcpyHostToDevice, q->stream) != cudaSuccess)
                 return VK_ERROR_DEVICE_LOST;
-            written.push_back(dst->memory);
+            wrote_buffer(written, dst, c.q[0], c.bytes.size());
             break;
         }
         case CmdType::DrawIndirect:
@@ -1048,7 +1081,7 @@ void CommandBuffer::reset() {
     graphable = -1;
 }
 
-VkResult run_command_buffer(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& written, bool no_alloc) {
+VkResult run_command_buffer(Queue* q, CommandBuffer* cb, std::vector<WrittenRange>& written, bool no_alloc) {
     if (no_alloc || rt::profile_enabled() || env_u32("CPV_CB_GRAPH", 1u) == 0u || cb->graphable == 0) return execute(q, cb, written, no_alloc);
     if (cb->graphable < 0) {
         // First execution: eager. It decides whether the buffer can be a graph
@@ -1078,7 +1111,7 @@ VkResult run_command_buffer(Queue* q, CommandBuffer* cb, std::vector<DeviceMemor
             return execute(q, cb, written, false);
         }
         cudaGraph_t graph = nullptr;
-        std::vector<DeviceMemory*> w;
+        std::vector<WrittenRange> w;
         const uint64_t before = rt::launches();
         if (cudaStreamBeginCapture(q->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             cudaGetLastError();
@@ -1179,7 +1212,7 @@ VkResult check_no_alloc(Queue* q, CommandBuffer* cb) {
         }
         return true;
     };
-    const std::vector<DeviceMemory*> none;
+    const std::vector<WrittenRange> none;
     for (const Cmd& c : cb->cmds) {
         switch (c.type) {
         case CmdType::BeginRenderPass:

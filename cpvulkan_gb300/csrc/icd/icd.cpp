@@ -427,19 +427,84 @@ void sync_queues(Device* dev) {
     for (Queue* q : dev->queues) cudaStreamSynchronize(q->stream);
 }
 
-// Completion of a submission: host-visible memories the GPU wrote and that
-// are mapped get their mirror refreshed (coherent memory semantics).
-void complete_readback(std::vector<DeviceMemory*>& mems) {
-    for (DeviceMemory* m : mems) {
-        if (!m || !m->host) continue;
-        m->device_dirty = true;
-        if (m->mapped) {
-            cudaMemcpy(m->host, m->device, m->size, cudaMemcpyDeviceToHost);
-            m->device_dirty = false;
+// Adds [lo, hi) to a memory's dirty ranges, joined with those it touches
+// (only bytes the device wrote: the copy back must not reach others).
+void add_dirty(DeviceMemory* m, uint64_t lo, uint64_t hi) {
+    for (size_t i = 0; i < m->dirty.size();) {
+        auto& d = m->dirty[i];
+        if (d.first <= hi && lo <= d.second) {
+            lo = std::min(lo, d.first);
+            hi = std::max(hi, d.second);
+            m->dirty.erase(m->dirty.begin() + static_cast<std::ptrdiff_t>(i));
+        } else {
+            i++;
         }
     }
-    mems.clear();
+    m->dirty.emplace_back(lo, hi);
 }
+
+// Brings the mirror up to date with the dirty ranges (their writers have
+// finished).
+bool copy_dirty(DeviceMemory* m) {
+    for (const auto& d : m->dirty)
+        if (cudaMemcpy(m->host + d.first, m->device + d.first, d.second - d.first, cudaMemcpyDeviceToHost) != cudaSuccess) return false;
+    m->dirty.clear();
+    return true;
+}
+
+// Completion of a submission: what it wrote in host-visible memories and did
+// not copy back itself is dirty there, or copied now where the memory is
+// mapped (coherent memory semantics). Under dev->memory_mutex.
+void complete_readback(std::vector<WrittenRange>& ranges) {
+    for (const WrittenRange& w : ranges) {
+        if (w.copied) continue;
+        add_dirty(w.memory, w.lo, w.hi);
+        if (w.memory->mapped) copy_dirty(w.memory);
+    }
+    ranges.clear();
+}
+
+// Waits for all queues and brings a memory's mirror up to date, whatever
+// fences have been looked at. Under dev->memory_mutex.
+bool settle(Device* dev, DeviceMemory* m, const std::vector<WrittenRange>* written = nullptr) {
+    sync_queues(dev);
+    if (written)
+        for (const WrittenRange& w : *written)
+            if (w.memory == m) add_dirty(m, w.lo, w.hi);
+    for (Queue* q : dev->queues)
+        for (const WrittenRange& w : q->pending_readback)
+            if (w.memory == m && !w.copied) add_dirty(m, w.lo, w.hi);
+    return copy_dirty(m);
+}
+
+// Copies a memory's mirror to HBM and waits for it: by the SMs over the
+// chip-to-chip link (2.05 GB of mesh data: 12 ms, against 29 ms for
+// cudaMemcpy on the same machine).
+void upload(Device* dev, DeviceMemory* m) {
+    cudaStream_t s = dev->queues.empty() ? nullptr : dev->queues[0]->stream;
+    if (rt::copy_host_to_device(s, m->device, m->host, m->size) != rt::kOk) cudaMemcpy(m->device, m->host, m->size, cudaMemcpyHostToDevice);
+    cudaStreamSynchronize(s);
+}
+
+void require_upload_locked(Device* dev, DeviceMemory* m, const std::vector<WrittenRange>* written) {
+    if (m->device_reads) return;
+    m->device_reads = true;
+    if (dev->compile_only || !m->host) return;
+    if (m->host_newer || m->mapped) {
+        settle(dev, m, written);  // the mirror holds every byte: host writes and device writes
+        upload(dev, m);
+    }
+    m->host_newer = false;
+}
+
+}  // namespace
+
+void require_upload(Device* dev, DeviceMemory* m, const std::vector<WrittenRange>* written) {
+    std::lock_guard<std::mutex> lock(dev->memory_mutex);
+    require_upload_locked(dev, m, written);
+}
+
+namespace {
 
 VKAPI_ATTR VkResult VKAPI_CALL DeviceWaitIdle(VkDevice device) {
     auto* dev = reinterpret_cast<Device*>(device);
@@ -447,6 +512,7 @@ VKAPI_ATTR VkResult VKAPI_CALL DeviceWaitIdle(VkDevice device) {
     for (Queue* q : dev->queues) {
         std::lock_guard<std::mutex> lock(q->mutex);
         if (cudaStreamSynchronize(q->stream) != cudaSuccess) return VK_ERROR_DEVICE_LOST;
+        std::lock_guard<std::mutex> memory_lock(dev->memory_mutex);
         complete_readback(q->pending_readback);
     }
     return VK_SUCCESS;
@@ -456,6 +522,7 @@ VKAPI_ATTR VkResult VKAPI_CALL QueueWaitIdle(VkQueue queue) {
     auto* q = reinterpret_cast<Queue*>(queue);
     std::lock_guard<std::mutex> lock(q->mutex);
     if (cudaStreamSynchronize(q->stream) != cudaSuccess) return VK_ERROR_DEVICE_LOST;
+    std::lock_guard<std::mutex> memory_lock(q->device->memory_mutex);
     complete_readback(q->pending_readback);
     return VK_SUCCESS;
 }
@@ -508,10 +575,10 @@ VKAPI_ATTR void VKAPI_CALL FreeMemory(VkDevice device, VkDeviceMemory memory, co
     {
         std::lock_guard<std::mutex> lock(dev->memory_mutex);
         dev->memories.erase(m);
-    }
-    for (Queue* q : dev->queues) {
-        auto& pr = q->pending_readback;
-        pr.erase(std::remove(pr.begin(), pr.end(), m), pr.end());
+        for (Queue* q : dev->queues) {
+            auto& pr = q->pending_readback;
+            pr.erase(std::remove_if(pr.begin(), pr.end(), [m](const WrittenRange& w) { return w.memory == m; }), pr.end());
+        }
     }
     if (dev->compile_only) {
         std::free(m->device);
@@ -533,12 +600,17 @@ VKAPI_ATTR VkResult VKAPI_CALL MapMemory(VkDevice device, VkDeviceMemory memory,
         *data = m->host + offset;
         return VK_SUCCESS;
     }
-    if (m->device_dirty) {
-        sync_queues(dev);
-        if (cudaMemcpy(m->host, m->device, m->size, cudaMemcpyDeviceToHost) != cudaSuccess) return VK_ERROR_MEMORY_MAP_FAILED;
-        m->device_dirty = false;
+    std::vector<std::pair<uint64_t, uint64_t>> dirty;
+    {
+        std::lock_guard<std::mutex> lock(dev->memory_mutex);
+        dirty.swap(m->dirty);
     }
+    if (!dirty.empty()) sync_queues(dev);
+    for (const auto& d : dirty)
+        if (cudaMemcpy(m->host + d.first, m->device + d.first, d.second - d.first, cudaMemcpyDeviceToHost) != cudaSuccess) return VK_ERROR_MEMORY_MAP_FAILED;
+    std::lock_guard<std::mutex> lock(dev->memory_mutex);
     m->mapped = true;
+    m->reads_back = true;
     *data = m->host + offset;
     return VK_SUCCESS;
 }
@@ -551,14 +623,17 @@ VKAPI_ATTR void VKAPI_CALL UnmapMemory(VkDevice device, VkDeviceMemory memory) {
         m->mapped = false;
         return;
     }
-    // The host's writes reach HBM before the call returns, copied by the SMs
-    // over the chip-to-chip link (2.05 GB of mesh data: 12 ms, against 29 ms
-    // for cudaMemcpy on the same machine).
+    {
+        std::lock_guard<std::mutex> lock(dev->memory_mutex);
+        if (!m->device_reads) {
+            m->mapped = false;
+            m->host_newer = true;
+            return;
+        }
+    }
+    // The host's writes reach HBM before the call returns.
     sync_queues(dev);
-    cudaStream_t s = dev->queues.empty() ? nullptr : dev->queues[0]->stream;
-    if (rt::copy_host_to_device(s, m->device, m->host, m->size) != rt::kOk)
-        cudaMemcpy(m->device, m->host, m->size, cudaMemcpyHostToDevice);
-    cudaStreamSynchronize(s);
+    upload(dev, m);
     m->mapped = false;
 }
 
@@ -582,12 +657,12 @@ VKAPI_ATTR VkResult VKAPI_CALL FlushMappedMemoryRanges(VkDevice device, uint32_t
 
 VKAPI_ATTR VkResult VKAPI_CALL InvalidateMappedMemoryRanges(VkDevice device, uint32_t n, const VkMappedMemoryRange* r) {
     auto* dev = reinterpret_cast<Device*>(device);
-    if (!dev->compile_only) sync_queues(dev);
     for (uint32_t i = 0; i < n; i++) {
         auto* m = reinterpret_cast<DeviceMemory*>(r[i].memory);
         if (!m->host) continue;
-        const VkDeviceSize size = r[i].size == VK_WHOLE_SIZE ? m->size - r[i].offset : r[i].size;
-        if (cudaMemcpy(m->host + r[i].offset, m->device + r[i].offset, size, cudaMemcpyDeviceToHost) != cudaSuccess) return VK_ERROR_OUT_OF_DEVICE_MEMORY;
+        // what the device has written; the mirror's other bytes are current
+        std::lock_guard<std::mutex> lock(dev->memory_mutex);
+        if (!dev->compile_only && !settle(dev, m)) return VK_ERROR_OUT_OF_DEVICE_MEMORY;
     }
     return VK_SUCCESS;
 }
@@ -609,12 +684,13 @@ VKAPI_ATTR void VKAPI_CALL GetBufferMemoryRequirements(VkDevice, VkBuffer buffer
     r->alignment = 256;
     r->memoryTypeBits = 0x3;
 }
-VKAPI_ATTR VkResult VKAPI_CALL BindBufferMemory(VkDevice, VkBuffer buffer, VkDeviceMemory memory, VkDeviceSize offset) {
+VKAPI_ATTR VkResult VKAPI_CALL BindBufferMemory(VkDevice device, VkBuffer buffer, VkDeviceMemory memory, VkDeviceSize offset) {
     auto* b = reinterpret_cast<Buffer*>(buffer);
     auto* m = reinterpret_cast<DeviceMemory*>(memory);
     if (offset + b->size > m->size) return VK_ERROR_OUT_OF_DEVICE_MEMORY;
     b->memory = m;
     b->offset = offset;
+    if (b->usage & ~static_cast<VkBufferUsageFlags>(VK_BUFFER_USAGE_TRANSFER_DST_BIT)) require_upload(reinterpret_cast<Device*>(device), m);
     return VK_SUCCESS;
 }
 
@@ -639,12 +715,13 @@ VKAPI_ATTR void VKAPI_CALL GetImageMemoryRequirements(VkDevice, VkImage image, V
     r->alignment = 256;
     r->memoryTypeBits = 0x3;
 }
-VKAPI_ATTR VkResult VKAPI_CALL BindImageMemory(VkDevice, VkImage image, VkDeviceMemory memory, VkDeviceSize offset) {
+VKAPI_ATTR VkResult VKAPI_CALL BindImageMemory(VkDevice device, VkImage image, VkDeviceMemory memory, VkDeviceSize offset) {
     auto* img = reinterpret_cast<Image*>(image);
     auto* m = reinterpret_cast<DeviceMemory*>(memory);
     if (offset + img->total_size > m->size) return VK_ERROR_OUT_OF_DEVICE_MEMORY;
     img->memory = m;
     img->offset = offset;
+    require_upload(reinterpret_cast<Device*>(device), m);
     return VK_SUCCESS;
 }
 VKAPI_ATTR void VKAPI_CALL GetImageSubresourceLayout(VkDevice, VkImage image, const VkImageSubresource* sub, VkSubresourceLayout* out) {
@@ -1239,7 +1316,13 @@ VkResult poll_fence(Device* dev, Fence* f) {
         return VK_ERROR_DEVICE_LOST;
     }
     {
-        std::lock_guard<std::mutex> lock(dev->queue->mutex);
+        std::lock_guard<std::mutex> lock(dev->memory_mutex);
+        for (const WrittenRange& w : f->readback) {
+            if (w.copied || !f->queue) continue;
+            auto& pr = f->queue->pending_readback;
+            const auto it = std::find(pr.begin(), pr.end(), w);
+            if (it != pr.end() && --it->submissions == 0) pr.erase(it);
+        }
         complete_readback(f->readback);
     }
     f->pending = false;
@@ -1306,13 +1389,13 @@ VkResult submit(VkQueue queue, uint32_t n, const VkSubmitInfo* si, VkFence fence
         rt::set_last_error("vkQueueSubmit: compile-only device (no CUDA device)");
         return VK_ERROR_DEVICE_LOST;
     }
-    std::vector<DeviceMemory*> written;
+    std::vector<WrittenRange> written;
     {
         // Coherent host-visible memory: host writes made while mapped are
         // visible to the device at submission.
         std::lock_guard<std::mutex> lock(dev->memory_mutex);
         for (DeviceMemory* m : dev->memories)
-            if (m->mapped && m->host) rt::copy_host_to_device(q->stream, m->device, m->host, m->size);
+            if (m->mapped && m->host && m->device_reads) rt::copy_host_to_device(q->stream, m->device, m->host, m->size);
     }
     for (uint32_t i = 0; i < n; i++) {
         for (uint32_t k = 0; k < si[i].waitSemaphoreCount; k++) {
@@ -1330,19 +1413,34 @@ VkResult submit(VkQueue queue, uint32_t n, const VkSubmitInfo* si, VkFence fence
             s->signalled = true;
         }
     }
-    std::vector<DeviceMemory*> host_visible;
-    for (DeviceMemory* m : written)
-        if (m && m->host && std::find(host_visible.begin(), host_visible.end(), m) == host_visible.end()) host_visible.push_back(m);
+    std::vector<WrittenRange> host_visible;
+    for (const WrittenRange& w : written)
+        if (w.memory->host && std::find(host_visible.begin(), host_visible.end(), w) == host_visible.end()) host_visible.push_back(w);
+    if (!host_visible.empty()) {
+        // A memory whose host reads what the device writes is copied back in
+        // the submission, before its fence; others when they are mapped.
+        std::lock_guard<std::mutex> lock(dev->memory_mutex);
+        for (WrittenRange& w : host_visible)
+            w.copied = (w.memory->mapped || w.memory->reads_back) &&
+                       cudaMemcpyAsync(w.memory->host + w.lo, w.memory->device + w.lo, w.hi - w.lo, cudaMemcpyDeviceToHost, q->stream) == cudaSuccess;
+        for (WrittenRange& w : host_visible) w.memory->reads_back = false;
+    }
     if (fence) {
         auto* f = reinterpret_cast<Fence*>(fence);
         if (cudaEventRecord(f->event, q->stream) != cudaSuccess) return VK_ERROR_DEVICE_LOST;
         f->pending = true;
         f->signalled = false;
+        f->queue = q;
         f->readback = host_visible;
     }
-    {
-        std::lock_guard<std::mutex> lock(q->mutex);
-        for (DeviceMemory* m : host_visible) q->pending_readback.push_back(m);
+    if (!host_visible.empty()) {
+        std::lock_guard<std::mutex> lock(dev->memory_mutex);
+        for (const WrittenRange& w : host_visible) {
+            if (w.copied) continue;
+            const auto it = std::find(q->pending_readback.begin(), q->pending_readback.end(), w);
+            if (it != q->pending_readback.end()) it->submissions++;
+            else q->pending_readback.push_back(w);
+        }
     }
     if (cudaGetLastError() != cudaSuccess) return VK_ERROR_DEVICE_LOST;
     return VK_SUCCESS;

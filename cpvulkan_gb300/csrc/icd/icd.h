@@ -50,7 +50,28 @@ struct DeviceMemory {
     VkDeviceSize size = 0;
     uint32_t type = 0;
     bool mapped = false;
-    bool device_dirty = false;     // HBM newer than the mirror
+    // Byte ranges in which HBM is newer than the mirror: what finished
+    // submissions wrote and the mirror has not received.
+    std::vector<std::pair<uint64_t, uint64_t>> dirty;
+    // Mapped since its last copy back within a submission: its host reads
+    // what the device writes, so the next submission copies it back itself.
+    bool reads_back = false;
+    // Something on the device may read it: a resource other than a
+    // TRANSFER_DST buffer is bound to it, or a command has used it as a
+    // source. Without, unmapping need not copy the mirror to HBM, and what
+    // the host wrote there (host_newer) stays in the mirror alone.
+    bool device_reads = false;
+    bool host_newer = false;
+};
+
+// Bytes [lo, hi) of a memory that a submission writes; copied: the
+// submission also copies them to the mirror.
+struct WrittenRange {
+    DeviceMemory* memory = nullptr;
+    uint64_t lo = 0, hi = 0;
+    bool copied = false;
+    uint32_t submissions = 1;  // in a queue's list: how many unfinished submissions write it
+    bool operator==(const WrittenRange& o) const { return memory == o.memory && lo == o.lo && hi == o.hi; }
 };
 
 struct Buffer {
@@ -260,7 +281,7 @@ struct CommandBuffer : Dispatchable {
     // Replay as a CUDA graph per queue: decided after the first execution
     // (no host-memory sources, no batched pass).
     int graphable = -1;  // -1 unknown, 0 no, 1 yes
-    std::vector<DeviceMemory*> written;  // memories its execution writes
+    std::vector<WrittenRange> written;  // what its execution writes
     std::map<Queue*, QueueGraph> graphs;
     void reset();
     ~CommandBuffer() { reset(); }
@@ -274,7 +295,8 @@ struct Fence {
     cudaEvent_t event = nullptr;
     bool signalled = false;   // created signalled or completed and observed
     bool pending = false;     // a submission will record the event
-    std::vector<DeviceMemory*> readback;  // host-visible memories written by the submission
+    Queue* queue = nullptr;  // of the pending submission
+    std::vector<WrittenRange> readback;  // what the submission wrote in host-visible memories
 };
 
 struct Semaphore {
@@ -287,7 +309,7 @@ struct Queue : Dispatchable {
     cudaStream_t stream = nullptr;
     cudaEvent_t timing[16] = {};
     rt::Scratch scratch;
-    std::vector<DeviceMemory*> pending_readback;
+    std::vector<WrittenRange> pending_readback;  // under the device's memory_mutex
     std::mutex mutex;
 };
 
@@ -323,11 +345,15 @@ rt::Module* batch_module(Device* dev, const std::vector<Pipeline*>& pipelines, c
 // Runs a command buffer on a queue: replays its CUDA graph for that queue
 // when it has one, captures one on its second run there, else executes
 // eagerly (command.cpp). CPV_CB_GRAPH=0 always executes eagerly.
-VkResult run_command_buffer(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& written, bool no_alloc);
+VkResult run_command_buffer(Queue* q, CommandBuffer* cb, std::vector<WrittenRange>& written, bool no_alloc);
 // Execution of a recorded command buffer on a queue (command.cpp).
 // no_alloc: draws bin through the fixed scratch array (rt::draw_plain_static)
 // instead of the queue's grow-only scratch.
-VkResult execute(Queue* q, CommandBuffer* cb, std::vector<DeviceMemory*>& written, bool no_alloc = false);
+VkResult execute(Queue* q, CommandBuffer* cb, std::vector<WrittenRange>& written, bool no_alloc = false);
+// The device is about to read `m`: from now on its mirror is copied to HBM
+// at unmap and submission, and what is newer there is copied now.
+// `written`: what the submission being enqueued writes before that.
+void require_upload(Device* dev, DeviceMemory* m, const std::vector<WrittenRange>* written = nullptr);
 // At vkEndCommandBuffer: compiles (NVRTC) and caches the batched module of
 // every render pass that will run batched, so its first submission does not.
 void precompile_batches(CommandBuffer* cb);

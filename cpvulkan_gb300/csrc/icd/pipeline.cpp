@@ -150,9 +150,7 @@ std::string compose_module(const std::vector<std::string>& stages, const std::ve
         }
     }
     // Register budget of the per-draw raster in resident CTAs of 256
-    // threads: six for the immediate schedule (the blend scene's raster
-    // 2.30 ms, 2.44 at five and 2.79 at seven, where the fragment loop
-    // spills); four for the others where a thread keeps one pixel of one
+    // threads: seven for the immediate schedule; four for the others where a thread keeps one pixel of one
     // attachment (a textured 500k-triangle request's raster 0.25 ms, 0.32 at
     // the compiler's choice of 112 registers, 0.27 at five; half-float
     // overdraw 0.51 ms, 0.58 at three, 0.55 at five). Several pixels or
@@ -164,7 +162,7 @@ std::string compose_module(const std::vector<std::string>& stages, const std::ve
         const size_t at = st.find("#define CPV_LOD_SITES ");
         lod_sites = lod_sites || (at != std::string::npos && std::atoi(st.c_str() + at + 22) > 0);
     }
-    int min_blocks = mc.schedule == 0 ? 6 : (pixels == cta && num_ca == 1 && !lod_sites ? static_cast<int>(1024u / cta) : 0);
+    int min_blocks = mc.schedule == 0 ? 7 : (pixels == cta && num_ca == 1 && !lod_sites ? static_cast<int>(1024u / cta) : 0);
     if (const char* v = std::getenv("CPV_PLAIN_MIN_BLOCKS")) min_blocks = std::atoi(v);
     if (min_blocks >= 1 && min_blocks <= 32) src << "#define CPV_PLAIN_MIN_BLOCKS " << min_blocks << "\n";
     // Register budget of the persistent batched raster, in resident CTAs of
@@ -173,7 +171,7 @@ std::string compose_module(const std::vector<std::string>& stages, const std::ve
     // 217 and 238). CPV_BATCH_MIN_BLOCKS overrides.
     {
         const uint32_t threads = std::min(1u << (2 * mc.tile_shift), 32u * mc.warps);
-        int b = static_cast<int>(1024u / threads);
+        int b = static_cast<int>((batched || mc.samples ? 1024u : 1280u) / threads);  // (unused in per-draw modules)
         if (b < 1) b = 1;
         if (const char* v = std::getenv("CPV_BATCH_MIN_BLOCKS")) b = std::atoi(v);
         if (b >= 1 && b <= 32) src << "#define CPV_RT_MIN_BLOCKS " << b << "\n";
