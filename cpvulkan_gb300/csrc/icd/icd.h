@@ -198,6 +198,7 @@ struct ModuleConfig {
     uint32_t batch = 256;     // primitives set up per shared-memory batch (set per schedule by module_config)
     uint32_t depth = 0;       // sparse schedule: fragments a pixel lists per batch (0: 24, or 16 when sampling)
     bool samples = false;     // a fragment shader samples images (register budget of the batched raster)
+    bool linear = false;      // the pipeline's fragments are a linear blend of a constant colour (per-draw modules)
 };
 
 // Fragment schedule of a module whose pipelines prefer (or not) dense
@@ -205,6 +206,7 @@ struct ModuleConfig {
 uint32_t schedule_for(bool prefers_deferred, bool fs_constant);
 // Module configuration for a tile size and shading preference, with the
 // environment's tunables applied.
+bool linear_module(const ModuleConfig& mc);
 ModuleConfig module_config(uint32_t tile_shift, bool prefers_deferred, bool fs_constant, bool samples);
 
 // The CUDA translation unit of a module over one pipeline's stage block

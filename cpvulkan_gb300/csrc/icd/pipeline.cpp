@@ -92,6 +92,18 @@ ModuleConfig module_config(uint32_t tile_shift, bool prefers_deferred, bool fs_c
     return mc;
 }
 
+// Whether a per-draw module of this configuration keeps decoded colours in
+// registers and blends them itself (its schedule walks per-warp lists with
+// one pixel a thread). CPV_LINEAR_BLEND=0 (blend tables instead) and
+// CPV_BLEND_TABLES=0 (the general blend) turn it off.
+bool linear_module(const ModuleConfig& mc) {
+    for (const char* name : {"CPV_LINEAR_BLEND", "CPV_BLEND_TABLES"}) {
+        const char* v = std::getenv(name);
+        if (v && std::atoi(v) == 0) return false;
+    }
+    return mc.linear && mc.schedule == 0 && (1u << (2 * mc.tile_shift)) <= 32u * mc.warps;
+}
+
 uint32_t schedule_for(bool prefers_deferred, bool fs_constant) {
     if (const char* v = std::getenv("CPV_SCHEDULE")) {
         const int s = std::atoi(v);
@@ -192,7 +204,10 @@ std::string compose_module(const std::vector<std::string>& stages, const std::ve
     // overrides.
     int quick_div = !batched && !mc.samples ? 1 : 0;
     if (const char* v = std::getenv("CPV_QUICK_DIV")) quick_div = std::atoi(v) ? 1 : 0;
+    const bool linear = !batched && linear_module(mc);
+    if (linear) quick_div = 0;
     src << "#define CPV_QUICK_DIV " << quick_div << "\n";
+    src << "#define CPV_LINEAR_BLEND " << (linear ? 1 : 0) << "\n";
     src << "#define CPV_NV_MAX " << nv_max << "\n";
     bool any_constant = false;
     for (const std::string& st : stages) any_constant = any_constant || st.find("#define CPV_FS_CONSTANT 1\n") != std::string::npos;
@@ -623,7 +638,19 @@ VkResult create_graphics_pipeline(Device* dev, PipelineCache* cache, const VkGra
     p->tile_shift = tile_shift;
     p->blend_table = blend_table;
     p->fs_constant = fs_constant;
-    p->source = compose_module({p->stage}, {nv}, module_config(tile_shift, prefers_deferred, fs_constant, fr.samples > 0), false, {p->stage_after});
+    // A fragment whose whole effect is a linear blend of the primitive's
+    // colour: no depth or stencil operation, an 8-bit RGBA target, no logic
+    // op, factors that do not read the destination, and an addition or
+    // subtraction (or no blending).
+    auto dst_factor = [&](VkBlendFactor f) { return dst_alpha_factor(f) || f == VK_BLEND_FACTOR_DST_COLOR || f == VK_BLEND_FACTOR_ONE_MINUS_DST_COLOR; };
+    auto additive = [](VkBlendOp op) { return op == VK_BLEND_OP_ADD || op == VK_BLEND_OP_SUBTRACT || op == VK_BLEND_OP_REVERSE_SUBTRACT; };
+    const bool depth_ops = dfmt != VK_FORMAT_UNDEFINED && (ds.depthTestEnable || stencil || ds.depthBoundsTestEnable);
+    ModuleConfig mc = module_config(tile_shift, prefers_deferred, fs_constant, fr.samples > 0);
+    mc.linear = fs_constant && nca == 1 && !logic && !depth_ops && (cfmt == VK_FORMAT_R8G8B8A8_UNORM || cfmt == VK_FORMAT_B8G8R8A8_UNORM) &&
+                (!blend.blendEnable || (!dst_factor(blend.srcColorBlendFactor) && !dst_factor(blend.dstColorBlendFactor) &&
+                                        !dst_factor(blend.srcAlphaBlendFactor) && !dst_factor(blend.dstAlphaBlendFactor) && additive(blend.colorBlendOp) &&
+                                        additive(blend.alphaBlendOp)));
+    p->source = compose_module({p->stage}, {nv}, mc, false, {p->stage_after});
     // The key covers the generated source and the embedded kernel headers it
     // includes, so an on-disk cache never returns a cubin of older kernels.
     {
@@ -701,7 +728,7 @@ VkResult create_graphics_pipeline(Device* dev, PipelineCache* cache, const VkGra
         rt::set_last_error("module load failed: " + err);
         return VK_ERROR_INITIALIZATION_FAILED;
     }
-    p->module.blend_table = blend_table;
+    p->module.blend_table = blend_table && !linear_module(mc);
     *out = p.release();
     return VK_SUCCESS;
 }

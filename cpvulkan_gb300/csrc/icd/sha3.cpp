@@ -24,16 +24,27 @@ constexpr int kRho[25] = {0, 1, 62, 28, 27, 36, 44, 6, 55, 20, 3, 10, 43, 25, 39
 
 inline uint64_t rotl(uint64_t v, int n) { return n == 0 ? v : (v << n) | (v >> (64 - n)); }
 
+// Every loop over lanes unrolled: constant indices and rotations, the lanes
+// in registers (a pipeline hashes 160 KB of kernel source when it is created).
 void keccak_f(uint64_t a[25]) {
     for (int round = 0; round < 24; round++) {
         uint64_t c[5], d[5], b[25];
+#pragma GCC unroll 5
         for (int x = 0; x < 5; x++) c[x] = a[x] ^ a[x + 5] ^ a[x + 10] ^ a[x + 15] ^ a[x + 20];
+#pragma GCC unroll 5
         for (int x = 0; x < 5; x++) d[x] = c[(x + 4) % 5] ^ rotl(c[(x + 1) % 5], 1);
+#pragma GCC unroll 25
         for (int i = 0; i < 25; i++) a[i] ^= d[i % 5];
-        for (int x = 0; x < 5; x++)
-            for (int y = 0; y < 5; y++) b[y + 5 * ((2 * x + 3 * y) % 5)] = rotl(a[x + 5 * y], kRho[x + 5 * y]);
-        for (int x = 0; x < 5; x++)
-            for (int y = 0; y < 5; y++) a[x + 5 * y] = b[x + 5 * y] ^ (~b[(x + 1) % 5 + 5 * y] & b[(x + 2) % 5 + 5 * y]);
+#pragma GCC unroll 25
+        for (int i = 0; i < 25; i++) {
+            const int x = i % 5, y = i / 5;
+            b[y + 5 * ((2 * x + 3 * y) % 5)] = rotl(a[i], kRho[i]);
+        }
+#pragma GCC unroll 25
+        for (int i = 0; i < 25; i++) {
+            const int x = i % 5, y = i / 5;
+            a[i] = b[i] ^ (~b[(x + 1) % 5 + 5 * y] & b[(x + 2) % 5 + 5 * y]);
+        }
         a[0] ^= kRoundConstants[round];
     }
 }

@@ -186,17 +186,13 @@ struct CpvPlainSource {
     }
     /* A covered fragment of a table-only pipeline: the table lookup is the
      * whole of shade + rop (the colour is constant and nothing discards a
-     * live primitive). Returns false when the general path must run. */
-    __device__ __forceinline__ bool table_fragment(const CpvTri& t, CpvPixel& s) const {
-        if (cpv_p0::kTableOnly) {
-            const uint8_t* table = cpv_p0::Stage::table(P, t);
-            if (table) {
-                cpv_p0::cpv_apply_table(table, s);
-                return true;
-            }
-        }
-        return false;
+     * live primitive). */
+    __device__ __forceinline__ bool table_only() const { return cpv_p0::kTableOnly && P.tables; }
+    __device__ __forceinline__ uint32_t table_lookup(const CpvTri& t, uint32_t texel) const {
+        return cpv_p0::cpv_table_lookup(P.tables, __float_as_uint(t.var[1][0]), texel);
     }
+    __device__ __forceinline__ void load_linear(uint64_t pix, float d[4]) const { cpv_p0::cpv_load_linear(P.color, pix, d); }
+    __device__ __forceinline__ void store_linear(uint64_t pix, const float d[4]) const { cpv_p0::cpv_store_linear(P.color, pix, d); }
     __device__ __forceinline__ void load_pixel(uint64_t pix, CpvPixel& s) const { cpv_p0::Stage::load_pixel(P.color, P.depth, pix, s, P.color_extra); }
     __device__ __forceinline__ void store_pixel(uint64_t pix, const CpvPixel& s) const {
         cpv_p0::Stage::store_pixel(P.color, P.depth, pix, s, P.color_extra);
@@ -207,7 +203,14 @@ struct CpvPlainSource {
  * rectangles the tile walks every primitive of the draw (small draws), else
  * what its bin list (or all rectangles) holds for it. Dynamic shared memory:
  * CPV_RASTER_SMEM_BYTES. */
-#ifdef CPV_PLAIN_MIN_BLOCKS
+#if CPV_LINEAR_BLEND
+/* the linear-blend loop runs best at five resident CTAs per SM (2.10 ms,
+ * 2.19 at four, 2.13 at six) */
+#ifndef CPV_LINEAR_MIN_BLOCKS
+#define CPV_LINEAR_MIN_BLOCKS 5
+#endif
+#define CPV_PLAIN_BOUNDS __launch_bounds__(CPV_RT_THREADS, CPV_LINEAR_MIN_BLOCKS)
+#elif defined(CPV_PLAIN_MIN_BLOCKS)
 /* a register budget for CPV_PLAIN_MIN_BLOCKS resident CTAs per SM */
 #define CPV_PLAIN_BOUNDS __launch_bounds__(CPV_RT_THREADS, CPV_PLAIN_MIN_BLOCKS)
 #else

@@ -42,6 +42,9 @@
 #ifndef CPV_ANY_FS_CONSTANT
 #define CPV_ANY_FS_CONSTANT 0 /* some pipeline of the module shades once per primitive */
 #endif
+#ifndef CPV_LINEAR_BLEND
+#define CPV_LINEAR_BLEND 0 /* the module's pipeline blends a constant colour linearly (cpv_linear_blend) and does nothing else */
+#endif
 #ifndef CPV_QUICK_DIV
 #define CPV_QUICK_DIV 0 /* fragments divide by reciprocals prepared at set-up */
 #endif
@@ -243,33 +246,39 @@ __device__ __forceinline__ bool cpv_may_cover(const CpvTri& t, int32_t rx0, int3
     return may;
 }
 
-/* Whether triangle t covers every pixel of the rectangle [rx0, rx1) x
- * [ry0, ry1): by the monotonicity cpv_may_cover uses, each edge function's
- * smallest value over the rectangle is at the corner picked by the signs of
- * dy and dx, and a pixel whose value is not negative passes that edge.
- * Exact in the other direction: true only when the coverage test passes at
- * every pixel (a NaN corner value, a non-finite coefficient or a line's
- * fourth edge gives false, and the pixels are then tested one by one). */
-__device__ __forceinline__ bool cpv_must_cover(const CpvTri& t, int32_t rx0, int32_t ry0, int32_t rx1, int32_t ry1, const float* col,
-                                               const float* row) {
+/* Whether cpv_block_edges may be asked: every coefficient of the triangle's
+ * edges is finite (a line has a fourth edge and is tested pixel by pixel). */
+__device__ __forceinline__ bool cpv_edges_finite(const CpvTri& t) {
 #if CPV_ANY_LINES
     if (((__float_as_uint(t.wf.w) >> 6) & 3u) == 3u) return false;
 #endif
-    const float c0 = col[rx0], c1 = col[rx1 - 1];
-    const float r0 = row[ry0], r1 = row[ry1 - 1];
-    const float xa = fminf(c0, c1), xb = fmaxf(c0, c1), ya = fminf(r0, r1), yb = fmaxf(r0, r1);
-    if (!(fabsf(c0) <= 3.4e38f && fabsf(c1) <= 3.4e38f && fabsf(r0) <= 3.4e38f && fabsf(r1) <= 3.4e38f)) return false;
-    bool must = true;
+    bool finite = true;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const float4 e = t.e[k];
-        if (!(fabsf(e.x) <= 3.4e38f && fabsf(e.y) <= 3.4e38f && fabsf(e.z) <= 3.4e38f && fabsf(e.w) <= 3.4e38f)) return false;
-        const float xf = e.w > 0.0f ? xa : xb;
-        const float yf = e.z > 0.0f ? yb : ya;
-        const float w = __fsub_rn(__fmul_rn(__fsub_rn(xf, e.x), e.w), __fmul_rn(__fsub_rn(yf, e.y), e.z));
-        must = must && w >= 0.0f;
+        finite = finite && fmaxf(fmaxf(fabsf(e.x), fabsf(e.y)), fmaxf(fabsf(e.z), fabsf(e.w))) <= 3.4e38f && e.x == e.x && e.y == e.y && e.z == e.z && e.w == e.w;
     }
-    return must;
+    return finite;
+}
+
+/* A triangle's edges over the rectangle of pixel centres [xa, xb] x [ya, yb]
+ * (finite, in either order): bit 3 when an edge is negative at every pixel
+ * (none is covered), else bit k for each edge that some pixel may fail. By
+ * the monotonicity cpv_may_cover uses, an edge function
+ * (xf - a.x) * dy - (yf - a.y) * dx has its extremes at the products' extremes,
+ * and its rounded difference is negative exactly when the one is less than
+ * the other. */
+__device__ __forceinline__ uint32_t cpv_block_edges(const CpvTri& t, float xa, float xb, float ya, float yb) {
+    uint32_t open = 0u;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const float4 e = t.e[k];
+        const float p0 = __fmul_rn(__fsub_rn(xa, e.x), e.w), p1 = __fmul_rn(__fsub_rn(xb, e.x), e.w);
+        const float q0 = __fmul_rn(__fsub_rn(ya, e.y), e.z), q1 = __fmul_rn(__fsub_rn(yb, e.y), e.z);
+        if (fmaxf(p0, p1) < fminf(q0, q1)) open |= 8u;
+        if (fminf(p0, p1) < fmaxf(q0, q1)) open |= 1u << k;
+    }
+    return open;
 }
 
 /* ---- per-fragment operation helpers (LLVMRuntime/PipelineCompiler.cpp:1020-1429) ---- */
@@ -365,6 +374,54 @@ __device__ __forceinline__ float cpv_blend_op(float s, float sf, float d, float 
     case 4: return cpv_std_max(s, d);
     default: return 0.0f;
     }
+}
+
+/* Two binary32 values in a 64-bit register, and the packed operations on
+ * them: each lane is rounded as the scalar operation rounds it. */
+struct CpvPair {
+    unsigned long long v;
+};
+__device__ __forceinline__ CpvPair cpv_pair(float a, float b) {
+    CpvPair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void cpv_unpair(CpvPair p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); }
+__device__ __forceinline__ CpvPair cpv_mul2(CpvPair a, CpvPair b) {
+    CpvPair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ CpvPair cpv_add2(CpvPair a, CpvPair b) {
+    CpvPair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ CpvPair cpv_add2_rz(CpvPair a, CpvPair b) {
+    CpvPair r;
+    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ CpvPair cpv_fma2(CpvPair a, CpvPair b, CpvPair c) {
+    CpvPair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
+/* The 8-bit UNORM channels that a + d * f encodes to, decoded again, for two
+ * channels: the blend of a colour that is constant over a primitive, for
+ * destination channels d with factors that do not read the destination (a:
+ * source times its factor, f: the destination's factor, signs as the blend
+ * operation has them). The reference's steps: multiply, add, clamp (NaN →
+ * 0), times 255, round half away from zero — floor(x + 0.5), both additions
+ * rounded toward zero — and over 255 as cpv_decode_unorm8. */
+__device__ __forceinline__ CpvPair cpv_linear_blend(CpvPair d, CpvPair a, CpvPair f) {
+    float a0, a1, p0, p1;
+    cpv_unpair(a, a0, a1);
+    cpv_unpair(cpv_mul2(d, f), p0, p1);
+    const CpvPair x = cpv_mul2(cpv_pair(__saturatef(__fadd_rn(a0, p0)), __saturatef(__fadd_rn(a1, p1))), cpv_pair(255.0f, 255.0f));
+    const CpvPair n = cpv_add2(cpv_add2_rz(cpv_add2_rz(x, cpv_pair(0.5f, 0.5f)), cpv_pair(8388608.0f, 8388608.0f)), cpv_pair(-8388608.0f, -8388608.0f));
+    return cpv_fma2(n, cpv_pair(0x1.010102p-8f, 0x1.010102p-8f), cpv_mul2(n, cpv_pair(-0x1.fdfdfep-33f, -0x1.fdfdfep-33f)));
 }
 
 /* Register-resident attachment state of one pixel. */
@@ -491,8 +548,8 @@ __device__ __forceinline__ void cpv_list_small_warp(const CpvTri* tris, const ui
  *                                            (true: discarded, or failed the early depth
  *                                            test against *early when given)
  *   void rop(const CpvTri&, const float colour[CPV_COLOUR_FLOATS], float mapped, CpvPixel&)
- *   bool table_fragment(const CpvTri&, CpvPixel&)  a covered fragment applied by a
- *                                            blend-table lookup alone (false: use shade + rop)
+ *   bool table_only()                        a covered fragment is a blend-table lookup alone:
+ *   uint32_t table_lookup(const CpvTri&, uint32_t texel)  the texel after it
  *   void load_pixel(uint64_t pix, CpvPixel&) / store_pixel(uint64_t pix, const CpvPixel&)
  *   float vw, vh                             viewport extent (pixel centres)
  *   uint32_t fb_width, fb_height
@@ -551,8 +608,16 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
         inside[k] = px[k] < static_cast<int32_t>(src.fb_width) && py[k] < static_cast<int32_t>(src.fb_height);
         xf[k] = cpv_pixel_ndc(px[k], src.vw);
         yf[k] = cpv_pixel_ndc(py[k], src.vh);
+#if !CPV_LINEAR_BLEND
         if (inside[k]) src.load_pixel(static_cast<uint64_t>(py[k]) * src.fb_width + px[k], st[k]);
+#endif
     }
+#if CPV_LINEAR_BLEND
+    static_assert(CPV_WARP_BLOCKS, "a linear-blend module runs the immediate schedule with one pixel a thread");
+    float lin[4] = {0.0f, 0.0f, 0.0f, 0.0f};  /* the pixel's decoded colour */
+    if (inside[0]) src.load_linear(static_cast<uint64_t>(py[0]) * src.fb_width + px[0], lin);
+    CpvPair lin01 = cpv_pair(lin[0], lin[1]), lin23 = cpv_pair(lin[2], lin[3]);
+#endif
 
 #if CPV_DEFERRED
     uint8_t* slot_base = reinterpret_cast<uint8_t*>(boxes + CPV_BATCH);
@@ -573,9 +638,15 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
 
 #if CPV_WARP_LISTS
     /* immediate schedule: per warp, the batch's primitives reaching its rows
-     * (batch index; bit 15: the primitive covers the warp's whole block) */
+     * (batch index; for a warp's block bits 8-10: the edges its pixels have to
+     * test, bit 11: the box, too; none set: the whole block is covered) */
+    static_assert(CPV_BATCH <= 256, "batch indices take 8 bits");
     __shared__ uint16_t warp_list[(CPV_RT_THREADS / 32) * CPV_BATCH];
 #if CPV_WARP_BLOCKS
+    __shared__ uint16_t live_flags[CPV_BATCH], live_list[CPV_BATCH];
+    /* every pixel centre of the tile is finite (their sequences are monotonic) */
+    const bool centres_finite = fabsf(cpv_pixel_ndc(tile_x0, src.vw)) <= 3.4e38f && fabsf(cpv_pixel_ndc(tile_x0 + CPV_TILE - 1, src.vw)) <= 3.4e38f &&
+                                fabsf(cpv_pixel_ndc(tile_y0, src.vh)) <= 3.4e38f && fabsf(cpv_pixel_ndc(tile_y0 + CPV_TILE - 1, src.vh)) <= 3.4e38f;
     const int32_t warp_x0 = static_cast<int32_t>(((threadIdx.x >> 5) % (CPV_TILE / CPV_BLOCK_W)) * CPV_BLOCK_W);
     const int32_t warp_y0 = static_cast<int32_t>(((threadIdx.x >> 5) / (CPV_TILE / CPV_BLOCK_W)) * CPV_BLOCK_H);
 #else
@@ -601,8 +672,27 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
                 (rx1 - rx0) * (ry1 - ry0) >= CPV_TILE_PX / 8)
                 live = cpv_may_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc);
             boxes[i] = live ? cpv_box_pack(rx0, ry0, rx1, ry1) : CPV_BOX_DEAD;
+#if CPV_WARP_BLOCKS
+            live_flags[i] = live ? (0x100u | (centres_finite && cpv_edges_finite(t) ? 1u : 0u)) : 0u;
+#endif
         }
         __syncthreads();
+#if CPV_WARP_BLOCKS
+        /* the batch's live primitives in order (index; bit 8: cpv_block_edges
+         * applies): each warp compacts the whole batch's flags for itself up
+         * to its 32, then writes those (half of a large triangle's tiles hold
+         * none of it, so half the primitives of a batch are dead) */
+        uint32_t alive = 0u;
+        for (uint32_t b = 0; b < n; b += 32u) {
+            const uint32_t i = b + (threadIdx.x & 31u);
+            const uint32_t flags = i < n ? live_flags[i] : 0u;
+            const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, flags != 0u);
+            if (flags != 0u && (b >> 5) % (CPV_RT_THREADS / 32) == (threadIdx.x >> 5))
+                live_list[alive + __popc(ballot & ((1u << (threadIdx.x & 31u)) - 1u))] = static_cast<uint16_t>(i | ((flags & 1u) << 8));
+            alive += __popc(ballot);
+        }
+        __syncthreads();
+#endif
 #if CPV_SPARSE
         /* 1. classify: large primitives (box covering more than CPV_SMALL_PX
          *    pixels of the tile) are collected in batch order, in rounds of
@@ -688,24 +778,37 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
             const uint32_t lane = threadIdx.x & 31u;
             uint16_t* mine = warp_list + (threadIdx.x >> 5) * CPV_BATCH;
             uint32_t count = 0;
-            for (uint32_t b = 0; b < n; b += 32u) {
-                const uint32_t j = b + lane;
-                bool hit = false;
-                uint32_t full = 0u;
-                if (j < n) {
-                    const CpvTri& t = tris[j];
-                    const uint32_t box = boxes[j];  /* a dead primitive's is empty */
 #if CPV_WARP_BLOCKS
+            for (uint32_t b = 0; b < alive; b += 32u) {
+                bool hit = false;
+                uint32_t entry = 0u;
+                if (b + lane < alive) {
+                    entry = live_list[b + lane];
+                    const uint32_t j = entry & 0xFFu;
+                    const uint32_t box = boxes[j];
                     /* the warp's block, within the box */
                     const int32_t rx0 = max(cpv_box_x0(box), warp_x0), rx1 = min(cpv_box_x1(box), warp_x0 + CPV_BLOCK_W);
                     const int32_t ry0 = max(cpv_box_y0(box), warp_y0), ry1 = min(cpv_box_y1(box), warp_y0 + CPV_BLOCK_H);
-                    hit = rx1 > rx0 && ry1 > ry0 && cpv_may_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc);
-                    /* a block inside the box (so inside the attachment) and
-                     * inside every edge: its pixels skip the box and edge tests */
-                    if (hit && rx0 == warp_x0 && rx1 == warp_x0 + CPV_BLOCK_W && ry0 == warp_y0 && ry1 == warp_y0 + CPV_BLOCK_H &&
-                        cpv_must_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc))
-                        full = 0x8000u;
+                    if (rx1 > rx0 && ry1 > ry0) {
+                        /* of a block inside the box (so inside the attachment) only the open edges are left to test */
+                        const bool in_box = rx0 == warp_x0 && rx1 == warp_x0 + CPV_BLOCK_W && ry0 == warp_y0 && ry1 == warp_y0 + CPV_BLOCK_H;
+                        uint32_t open = 7u;
+                        if (entry & 0x100u) open = cpv_block_edges(tris[j], col_ndc[rx0], col_ndc[rx1 - 1], row_ndc[ry0], row_ndc[ry1 - 1]);
+                        hit = open < 8u;
+                        entry = j | (open << 8) | (in_box ? 0u : 0x800u);
+                    }
+                }
+                const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, hit);
+                if (hit) mine[count + __popc(ballot & ((1u << lane) - 1u))] = static_cast<uint16_t>(entry);
+                count += __popc(ballot);
+            }
 #else
+            for (uint32_t b = 0; b < n; b += 32u) {
+                const uint32_t j = b + lane;
+                bool hit = false;
+                if (j < n) {
+                    const CpvTri& t = tris[j];
+                    const uint32_t box = boxes[j];  /* a dead primitive's is empty */
                     const int32_t rx0 = cpv_box_x0(box), rx1 = cpv_box_x1(box);
 #pragma unroll
                     for (int k = 0; k < CPV_PPT; k++) {
@@ -714,25 +817,78 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
                         const int32_t ry1 = min(cpv_box_y1(box), warp_y0 + k * CPV_ROWS_PER_PASS + CPV_WARP_ROWS);
                         hit = hit || (ry1 > ry0 && cpv_may_cover(t, rx0, ry0, rx1, ry1, col_ndc, row_ndc));
                     }
-#endif
                 }
                 const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, hit);
-                if (hit) mine[count + __popc(ballot & ((1u << lane) - 1u))] = static_cast<uint16_t>(j | full);
+                if (hit) mine[count + __popc(ballot & ((1u << lane) - 1u))] = static_cast<uint16_t>(j);
                 count += __popc(ballot);
             }
+#endif
             __syncwarp();
 #else
             const uint32_t count = n;
 #endif
+#if CPV_WARP_BLOCKS && (CPV_LINEAR_BLEND || CPV_ANY_FS_CONSTANT)
+            /* The entry's tests for this thread's pixel. */
+            auto passes = [&](uint32_t entry, const CpvTri& t) {
+                bool covered = true;
+                if (entry & 0x800u) covered = cpv_in_box(boxes[entry & 0xFFu], bp[0]);
+#if CPV_ANY_LINES
+                float w[3];
+                if (entry & 0x700u) covered = cpv_covers(t, xf[0], yf[0], w) && covered;
+#else
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    if (entry & (0x100u << k)) {
+                        const float4 e = t.e[k];
+                        /* the rounded difference is negative exactly when the one is less */
+                        covered = covered && !(__fmul_rn(__fsub_rn(xf[0], e.x), e.w) < __fmul_rn(__fsub_rn(yf[0], e.y), e.z));
+                    }
+                }
+#endif
+                return covered;
+            };
+#endif
+#if CPV_LINEAR_BLEND
+            /* The blend of a constant colour as two constants per channel
+             * (cpv_shade_constant): eight binary32 operations a channel on the
+             * decoded colour, two channels an instruction, and nothing else in
+             * the loop. Issue-bound: the 200k-quad scene at 1920x1080 takes 2.10
+             * ms of raster (2.38 with scalar operations; with blend tables
+             * 2.51, and 0.12 to build them), 1.3 of it in this loop, 0.4 in
+             * set-up and filter, the rest in the lists and their barriers. */
+            for (uint32_t m = 0; m < count; m++) {
+                const uint32_t entry = mine[m];
+                const CpvTri& t = tris[entry & 0xFFu];
+                if (entry > 0xFFu && !passes(entry, t)) continue;
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(t.var[0]), f = *reinterpret_cast<const ulonglong2*>(t.var[1]);
+                lin01 = cpv_linear_blend(lin01, CpvPair{a.x}, CpvPair{f.x});
+                lin23 = cpv_linear_blend(lin23, CpvPair{a.y}, CpvPair{f.y});
+            }
+#else
+#if CPV_WARP_BLOCKS && CPV_ANY_FS_CONSTANT
+            /* A pipeline whose covered fragments are a blend-table lookup each:
+             * a loop of its own, so that the general one's registers do not
+             * spill it (a byte permute makes each lookup's address). */
+            if (src.table_only()) {
+                uint32_t texel = st[0].colour[0];
+                for (uint32_t m = 0; m < count; m++) {
+                    const uint32_t entry = mine[m];
+                    const CpvTri& t = tris[entry & 0xFFu];
+                    if (entry > 0xFFu && !passes(entry, t)) continue;
+                    texel = src.table_lookup(t, texel);
+                }
+                st[0].colour[0] = texel;
+                continue;
+            }
+#endif
             for (uint32_t m = 0; m < count; m++) {
 #if CPV_WARP_LISTS
                 const uint32_t entry = mine[m];
-                const uint32_t j = entry & 0x7FFFu;
+                const uint32_t j = entry & 0xFFu;
 #if CPV_WARP_BLOCKS
-                if (entry & 0x8000u) {
+                if (entry <= 0xFFu) {
                     /* the whole block is covered (one pixel a thread, all inside) */
                     const CpvTri& t = tris[j];
-                    if (src.table_fragment(t, st[0])) continue;
                     float w[3], colour[CPV_COLOUR_FLOATS], mapped;
                     cpv_covers(t, xf[0], yf[0], w);
                     if (src.shade(t, w, px[0], py[0], colour, mapped, &st[0])) continue;
@@ -750,12 +906,12 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
                     if (!cpv_in_box(box, bp[k])) continue;
                     float w[3];
                     if (!cpv_covers(t, xf[k], yf[k], w)) continue;
-                    if (src.table_fragment(t, st[k])) continue;
                     float colour[CPV_COLOUR_FLOATS], mapped;
                     if (src.shade(t, w, px[k], py[k], colour, mapped, &st[k])) continue;
                     src.rop(t, colour, mapped, st[k]);
                 }
             }
+#endif
         }
 #else
         const uint32_t limit = n * CPV_PPT;
@@ -819,6 +975,12 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
         }
 #endif
     }
+#if CPV_LINEAR_BLEND
+    cpv_unpair(lin01, lin[0], lin[1]);
+    cpv_unpair(lin23, lin[2], lin[3]);
+    if (inside[0]) src.store_linear(static_cast<uint64_t>(py[0]) * src.fb_width + px[0], lin);
+    return;
+#endif
 #pragma unroll
     for (int k = 0; k < CPV_PPT; k++) {
         if (inside[k]) src.store_pixel(static_cast<uint64_t>(py[k]) * src.fb_width + px[k], st[k]);

@@ -45,6 +45,38 @@
 #define CPV_MAX_DEPTH_BOUNDS 1.0f
 #endif
 
+#if CPV_LINEAR_BLEND
+/* cpv_blend of a constant colour as two constants per channel (see
+ * cpv_linear_blend): the destination's factor does not depend on it, and
+ * subtraction adds the negated product. A channel outside the write mask
+ * keeps its value (0 + d * 1); without blending the colour replaces it. */
+__device__ __forceinline__ void cpv_linear_constants(const float blend_constants[4], const float colour[4], float a[4], float f[4]) {
+    const float none[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float sf[4], df[4];
+#if CPV_BLEND
+    cpv_blend_factor(colour, none, blend_constants, CPV_SRC_COLOR, CPV_SRC_ALPHA, sf);
+    cpv_blend_factor(colour, none, blend_constants, CPV_DST_COLOR, CPV_DST_ALPHA, df);
+#endif
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+#if CPV_BLEND
+        const int op = i == 3 ? CPV_ALPHA_OP : CPV_COLOR_OP;  /* 0 add, 1 subtract, 2 reverse subtract */
+        const float s = __fmul_rn(colour[i], sf[i]);
+        a[i] = op == 2 ? -s : s;
+        f[i] = op == 1 ? -df[i] : df[i];
+#else
+        (void)blend_constants; (void)none; (void)sf; (void)df;
+        a[i] = colour[i];
+        f[i] = 0.0f;
+#endif
+        if (((CPV_WRITE_MASK >> i) & 1u) == 0u) {
+            a[i] = 0.0f;
+            f[i] = 1.0f;
+        }
+    }
+}
+#endif
+
 /* The fragment shader of a primitive whose shader is constant over it
  * (CPV_FS_CONSTANT): shaded once from the provoking vertex's outputs; the
  * colour goes to var[0][0..3] (a discard kills the primitive) and, with
@@ -59,9 +91,13 @@ __device__ __forceinline__ void cpv_shade_constant(const CpvDrawParams& P, const
         const float frag_coord[4] = {0.0f, 0.0f, 0.0f, 1.0f};  /* not read by this shader */
         float colour[CPV_COLOUR_FLOATS];
         if (cpv_fs_run(P, in, frag_coord, front, colour)) live = false;
+#if CPV_LINEAR_BLEND
+        cpv_linear_constants(P.blend_constants, colour, t.var[0], t.var[1]);
+#else
 #pragma unroll
         for (int c = 0; c < 4; c++) t.var[0][c] = colour[c];
-#if CPV_BLEND_TABLE
+#endif
+#if CPV_BLEND_TABLE && !CPV_LINEAR_BLEND
         t.var[1][0] = __uint_as_float(g32);  /* the primitive's blend table */
 #endif
     }
@@ -1018,16 +1054,40 @@ constexpr bool kBlendTable = CPV_BLEND_TABLE != 0;
 constexpr bool kTableOnly = kBlendTable && !(CPV_DEPTH_TEST && CPV_DEPTH_FORMAT != 0) && !(CPV_STENCIL_TEST && CPV_DEPTH_FORMAT == 130) &&
                             !(CPV_DEPTH_BOUNDS && CPV_DEPTH_FORMAT != 0);
 
-/* cpv_rop's colour write through a blend table, when every test passes */
-__device__ __forceinline__ void cpv_apply_table(const uint8_t* table, CpvPixel& s) {
+/* cpv_rop's colour write through blend table `index`, when every test
+ * passes: the blend result for the destination byte, per channel. A table
+ * is 4 x 256 bytes on a 1 KiB boundary of an array of at most 4 GiB, so an
+ * address is its 32-bit offset with the destination byte as low byte. */
+__device__ __forceinline__ uint32_t cpv_table_lookup(const uint8_t* tables, uint32_t index, uint32_t texel) {
+    const uint32_t base = index << 10;
     uint32_t packed = 0u;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const uint32_t d = (s.colour[0] >> cpv_channel_shift(i)) & 0xFFu;
-        packed |= static_cast<uint32_t>(table[i * 256 + d]) << cpv_channel_shift(i);
+        const int byte = cpv_channel_shift(i) / 8;
+        const uint32_t at = __byte_perm(base, texel, 0x3210 + 4 + byte);  /* bytes 1-3 of base over the channel's byte */
+        packed |= static_cast<uint32_t>(__ldg(tables + (at + static_cast<uint32_t>(i) * 256u))) << (8 * byte);
     }
-    s.colour[0] = packed;
+    return packed;
 }
+
+#if CPV_LINEAR_BLEND
+/* The colour texel's channels decoded, and encoded again. */
+__device__ __forceinline__ void cpv_load_linear(const uint8_t* color, uint64_t pix, float d[4]) {
+    uint32_t t[1];
+    cpv_load_colour(color, pix, t);
+#pragma unroll
+    for (int i = 0; i < 4; i++) d[i] = cpv_decode_unorm8(cpv_channel_get(t, i));
+}
+__device__ __forceinline__ void cpv_store_linear(uint8_t* color, uint64_t pix, const float d[4]) {
+    uint32_t t[1] = {0u};
+#pragma unroll
+    for (int i = 0; i < 4; i++) t[0] |= cpv_encode_unorm(d[i], 255.0f) << cpv_channel_shift(i);
+    cpv_store_colour(color, pix, t);
+}
+#else
+__device__ __forceinline__ void cpv_load_linear(const uint8_t*, uint64_t, float*) {}
+__device__ __forceinline__ void cpv_store_linear(uint8_t*, uint64_t, const float*) {}
+#endif
 
 /* The stage functions of this pipeline, as one type the module's
  * dispatcher (cpv_dispatch) hands to generic code. */
