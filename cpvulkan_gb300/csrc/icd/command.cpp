@@ -89,7 +89,16 @@ struct BoundVertex {
     VkDeviceSize offset = 0;
 };
 
+// A load-op clear of a whole attachment that has not run: the pass's first
+// draw makes it (CpvClear), or it runs by itself before anything else.
+struct PendingClear {
+    const ImageView* view = nullptr;
+    VkImageAspectFlags aspects = 0;
+    VkClearValue value{};
+};
+
 struct State {
+    PendingClear clear_colour, clear_depth;
     Device* device = nullptr;
     const std::vector<WrittenRange>* written = nullptr;  // by the submission so far
     Pipeline* pipeline = nullptr;
@@ -255,6 +264,7 @@ VkResult begin_render_pass(Queue* q, State& s, const Cmd& c, std::vector<Written
     s.pass = static_cast<RenderPass*>(c.p[0]);
     s.fb = static_cast<Framebuffer*>(c.p[1]);
     s.subpass = 0;
+    s.clear_colour = s.clear_depth = PendingClear{};
     if (!s.pass || !s.fb || s.pass->subpasses.empty()) return VK_ERROR_DEVICE_LOST;
     for (size_t i = 0; i < s.pass->attachments.size() && i < s.fb->attachments.size(); i++) {
         const auto& a = s.pass->attachments[i];
@@ -269,11 +279,86 @@ VkResult begin_render_pass(Queue* q, State& s, const Cmd& c, std::vector<Written
         if (a.loadOp == VK_ATTACHMENT_LOAD_OP_CLEAR) aspects |= depth ? VK_IMAGE_ASPECT_DEPTH_BIT : VK_IMAGE_ASPECT_COLOR_BIT;
         if (depth && format_has_stencil(a.format) && a.stencilLoadOp == VK_ATTACHMENT_LOAD_OP_CLEAR) aspects |= VK_IMAGE_ASPECT_STENCIL_BIT;
         if (!aspects || i >= c.clears.size()) continue;
+        // the first colour and the depth attachment of a pass of one subpass
+        // wait for the first draw, when the clear covers their whole texels
+        if (s.pass->subpasses.size() == 1) {
+            const Subpass& sub = s.sub();
+            PendingClear* pending = nullptr;
+            uint32_t uses = sub.depth == i ? 1u : 0u;
+            for (uint32_t colour : sub.colour) uses += colour == i ? 1u : 0u;
+            if (uses == 1 && !depth && !sub.colour.empty() && sub.colour[0] == i) pending = &s.clear_colour;
+            if (uses == 1 && depth && sub.depth == i && (!format_has_stencil(a.format) || (aspects & VK_IMAGE_ASPECT_DEPTH_BIT && aspects & VK_IMAGE_ASPECT_STENCIL_BIT)))
+                pending = &s.clear_depth;
+            uint32_t words[4];
+            if (pending && a.format == v->image->format && clear_texel(v->image->format, c.clears[i], words)) {
+                *pending = {v, aspects, c.clears[i]};
+                continue;
+            }
+        }
         const ImageLevel& L = v->image->level[v->range.baseMipLevel];
         const VkResult r = clear_rect(q, v->image, v->range.baseArrayLayer, v->range.baseMipLevel, aspects, c.clears[i], 0, 0, L.width, L.height);
         if (r != VK_SUCCESS) return r;
     }
     return VK_SUCCESS;
+}
+
+VkResult run_clear(Queue* q, PendingClear& p) {
+    if (!p.view) return VK_SUCCESS;
+    const ImageView* v = p.view;
+    p.view = nullptr;
+    const ImageLevel& L = v->image->level[v->range.baseMipLevel];
+    return clear_rect(q, v->image, v->range.baseArrayLayer, v->range.baseMipLevel, p.aspects, p.value, 0, 0, L.width, L.height);
+}
+
+// Runs the clears that no draw has made.
+VkResult run_clears(Queue* q, State& s) {
+    const VkResult a = run_clear(q, s.clear_colour), b = run_clear(q, s.clear_depth);
+    return a != VK_SUCCESS ? a : b;
+}
+
+// Whether a draw's raster makes a pending clear. It runs by itself first for
+// a pipeline of another format, a linear blend's depth attachment (its raster
+// leaves that alone), and a draw that reads the image's memory.
+bool makes_clear(const PendingClear& c, uint32_t format, const CpvDrawParams& P) {
+    const Image* image = c.view->image;
+    if (format != static_cast<uint32_t>(image->format)) return false;
+    const uint8_t* begin = image->device_ptr();
+    const uint8_t* end = begin + image->total_size;
+    auto reads = [&](const void* p, uint64_t bytes) {
+        const uint8_t* b = static_cast<const uint8_t*>(p);
+        return b && b < end && begin < b + bytes;
+    };
+    for (const CpvTexture& t : P.tex)
+        if (reads(t.data, t.bytes)) return false;
+    for (int i = 0; i < CPV_MAX_UBO; i++)
+        if (reads(P.ubo[i], P.ubo_bytes[i])) return false;
+    for (int i = 0; i < 8; i++)
+        if (reads(P.vb[i], P.vb_bytes[i])) return false;
+    return !reads(P.ib, P.ib_bytes);
+}
+
+bool makes_clear_colour(const State& s, const CpvDrawParams& P) {
+    return !s.clear_colour.view || makes_clear(s.clear_colour, s.pipeline->colour_format, P);
+}
+
+bool makes_clear_depth(const State& s, const CpvDrawParams& P, bool linear) {
+    return !s.clear_depth.view || (!linear && makes_clear(s.clear_depth, s.pipeline->depth_format, P));
+}
+
+// The pending clears as a raster takes them.
+CpvClear clear_params(const State& s) {
+    CpvClear out{};
+    uint32_t words[4];
+    if (s.clear_colour.view && clear_texel(s.clear_colour.view->image->format, s.clear_colour.value, words)) {
+        out.mask |= 1u;
+        for (int i = 0; i < 4; i++) out.colour[i] = words[i];
+    }
+    if (s.clear_depth.view && clear_texel(s.clear_depth.view->image->format, s.clear_depth.value, words)) {
+        out.mask |= 2u;
+        out.depth[0] = words[0];
+        out.depth[1] = words[1];
+    }
+    return out;
 }
 
 // Parameters of one draw from the current state: the per-draw path launches
@@ -381,7 +466,13 @@ VkResult draw(Queue* q, State& s, uint32_t count, uint32_t instances, uint32_t f
     const VkResult vr = build_draw(s, count, instances, first, vertex_offset, first_instance, indexed, P, empty);
     if (vr != VK_SUCCESS || empty) return vr;
     Pipeline* p = s.pipeline;
+    VkResult cr = VK_SUCCESS;
+    if (!makes_clear_colour(s, P)) cr = run_clear(q, s.clear_colour);
+    if (cr == VK_SUCCESS && !makes_clear_depth(s, P, p->module.linear)) cr = run_clear(q, s.clear_depth);
+    if (cr != VK_SUCCESS) return cr;
+    P.clear = clear_params(s);
     const int r = no_alloc ? rt::draw_plain_static(q->stream, p->module, P) : rt::draw_plain(q->stream, p->module, P, q->scratch);
+    if (r == rt::kOk) s.clear_colour.view = s.clear_depth.view = nullptr;
     if (r == rt::kErrOutOfMemory) return VK_ERROR_OUT_OF_DEVICE_MEMORY;
     return r == rt::kOk ? VK_SUCCESS : VK_ERROR_DEVICE_LOST;
 }
@@ -711,6 +802,7 @@ void build_batch(Queue* q, const CommandBuffer* cb, size_t begin, size_t end, co
     rt::BatchDraws in;
     std::vector<Pipeline*> pipelines;
     float vw = 0.0f, vh = 0.0f;
+    bool own_clears = true;  // the raster makes the pass's clears
     // false when the draw cannot join the batch
     auto add = [&](uint32_t count, uint32_t instances, uint32_t first, int32_t vertex_offset, uint32_t first_instance, bool indexed) {
         CpvDrawParams P;
@@ -734,6 +826,7 @@ void build_batch(Queue* q, const CommandBuffer* cb, size_t begin, size_t end, co
         } else if (P.viewport[2] != vw || P.viewport[3] != vh) {
             return false;  // pixel centres depend on the viewport extent
         }
+        own_clears = own_clears && makes_clear_colour(s, P) && makes_clear_depth(s, P, false);
         in.draws.push_back(P);
         in.pipeline.push_back(static_cast<uint32_t>(it - pipelines.begin()));
         const VkPrimitiveTopology topo = s.pipeline->topology;
@@ -760,6 +853,7 @@ void build_batch(Queue* q, const CommandBuffer* cb, size_t begin, size_t end, co
     if (in.draws.empty()) return;
     in.vw = vw;
     in.vh = vh;
+    if (own_clears) in.clear = clear_params(entry);
     Device* dev = cb->device;
     ModuleConfig mc = batch_config(pipelines);
     if (tuning_enabled(in.draws.size())) {
@@ -840,9 +934,13 @@ bool run_batched(Queue* q, CommandBuffer* cb, size_t begin, size_t end, State& s
     }
     if (slot->plain) return false;
     for (size_t i = begin + 1; i < end; i++) apply_state(s, cb->cmds[i]);
+    // the plan makes the pass's clears, or was built to make none
+    const bool own_clears = slot->plan->clears() == clear_params(s).mask;
+    if (!own_clears && (result = run_clears(q, s)) != VK_SUCCESS) return true;
     rt::profile_begin(q->stream, "cpv_batch");
     result = slot->plan->launch(*slot->module, q->stream) == rt::kOk ? VK_SUCCESS : VK_ERROR_DEVICE_LOST;
     rt::profile_end(q->stream);
+    if (result == VK_SUCCESS) s.clear_colour.view = s.clear_depth.view = nullptr;
     return true;
 }
 
@@ -856,6 +954,8 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<WrittenRange>& written
         const Cmd& c = cb->cmds[idx];
         if (apply_state(s, c)) continue;
         VkResult r = VK_SUCCESS;
+        const bool is_draw = c.type == CmdType::Draw || c.type == CmdType::DrawIndexed || is_indirect(c);
+        if (!is_draw && c.type != CmdType::Barrier && (r = run_clears(q, s)) != VK_SUCCESS) return r;
         switch (c.type) {
         case CmdType::BeginRenderPass: {
             r = begin_render_pass(q, s, c, written);
@@ -1066,9 +1166,12 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<WrittenRange>& written
         default:
             break;
         }
-        if (r != VK_SUCCESS) return r;
+        if (r != VK_SUCCESS) {
+            run_clears(q, s);  // the commands before the failing one have run
+            return r;
+        }
     }
-    return VK_SUCCESS;
+    return run_clears(q, s);
 }
 
 void CommandBuffer::reset() {

@@ -728,7 +728,8 @@ VkResult create_graphics_pipeline(Device* dev, PipelineCache* cache, const VkGra
         rt::set_last_error("module load failed: " + err);
         return VK_ERROR_INITIALIZATION_FAILED;
     }
-    p->module.blend_table = blend_table && !linear_module(mc);
+    p->module.linear = linear_module(mc);
+    p->module.blend_table = blend_table && !p->module.linear;
     *out = p.release();
     return VK_SUCCESS;
 }

@@ -141,10 +141,11 @@ struct CpvBatchSource {
     /* batched passes build no blend tables */
     __device__ __forceinline__ bool table_only() const { return false; }
     __device__ __forceinline__ uint32_t table_lookup(const CpvTri&, uint32_t texel) const { return texel; }
-    __device__ __forceinline__ void load_pixel(uint64_t pix, CpvPixel& s) const { cpv_p0::Stage::load_pixel(B.color, B.depth, pix, s, B.color_extra); }
+    __device__ __forceinline__ void load_pixel(uint64_t pix, CpvPixel& s) const { cpv_p0::Stage::load_pixel(B.color, B.depth, pix, s, B.color_extra, B.clear); }
     __device__ __forceinline__ void store_pixel(uint64_t pix, const CpvPixel& s) const {
-        cpv_p0::Stage::store_pixel(B.color, B.depth, pix, s, B.color_extra);
+        cpv_p0::Stage::store_pixel(B.color, B.depth, pix, s, B.color_extra, B.clear);
     }
+    __device__ __forceinline__ void clear_pixel(uint64_t pix) const { cpv_p0::Stage::clear_pixel(B.color, B.depth, pix, B.clear); }
 };
 
 /* Persistent raster: CTAs take tiles from B.tile_counter (reset to zero
@@ -169,7 +170,10 @@ extern "C" __global__ void __launch_bounds__(CPV_RT_THREADS, CPV_RT_MIN_BLOCKS) 
         }
         CpvBatchSource src{B, begin, end, overflow, tx, ty, B.vw, B.vh, B.fb_width, B.fb_height, 0u};
         const uint32_t first = src.next(warp_sums);
-        if (first == 0u) continue;
+        if (first == 0u) {
+            if (B.clear.mask) cpv_clear_tile(src, tx, ty);
+            continue;
+        }
         cpv_raster_tile(src, first, tx, ty, reinterpret_cast<CpvTri*>(cpv_dyn_smem), warp_sums);
     }
 }

@@ -53,6 +53,15 @@ struct CpvTexture {
     float lod_bias, min_lod, max_lod;
 };
 
+/* A render pass's load-op clears of its first colour attachment (mask bit 0)
+ * and its depth attachment (bit 1), left to the first draw's raster: it
+ * starts every pixel from these texels instead of the attachments'. */
+struct CpvClear {
+    uint32_t mask;
+    uint32_t colour[4];
+    uint32_t depth[2];
+};
+
 /* Bins of a draw: a square of tiles each, at most this many on the target
  * (the per-draw binning kernels keep a counter per bin in shared memory). */
 #define CPV_MAX_BINS 1024u
@@ -85,6 +94,7 @@ struct CpvDrawParams {
     uint32_t fb_width, fb_height;
     float viewport[6];
     float blend_constants[4];
+    struct CpvClear clear;
     /* screen tiling */
     uint32_t tile_shift;
     uint32_t tiles_x, tiles_y;
@@ -139,6 +149,7 @@ struct CpvBatchParams {
     uint8_t* depth;
     uint8_t* color_extra[CPV_MAX_CA - 1];
     uint32_t fb_width, fb_height;
+    struct CpvClear clear;
     float vw, vh;
     uint32_t tiles_x, tiles_y;
     /* binning */

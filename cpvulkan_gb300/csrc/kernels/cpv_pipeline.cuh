@@ -191,12 +191,13 @@ struct CpvPlainSource {
     __device__ __forceinline__ uint32_t table_lookup(const CpvTri& t, uint32_t texel) const {
         return cpv_p0::cpv_table_lookup(P.tables, __float_as_uint(t.var[1][0]), texel);
     }
-    __device__ __forceinline__ void load_linear(uint64_t pix, float d[4]) const { cpv_p0::cpv_load_linear(P.color, pix, d); }
+    __device__ __forceinline__ void load_linear(uint64_t pix, float d[4]) const { cpv_p0::cpv_load_linear(P.color, pix, P.clear, d); }
     __device__ __forceinline__ void store_linear(uint64_t pix, const float d[4]) const { cpv_p0::cpv_store_linear(P.color, pix, d); }
-    __device__ __forceinline__ void load_pixel(uint64_t pix, CpvPixel& s) const { cpv_p0::Stage::load_pixel(P.color, P.depth, pix, s, P.color_extra); }
+    __device__ __forceinline__ void load_pixel(uint64_t pix, CpvPixel& s) const { cpv_p0::Stage::load_pixel(P.color, P.depth, pix, s, P.color_extra, P.clear); }
     __device__ __forceinline__ void store_pixel(uint64_t pix, const CpvPixel& s) const {
-        cpv_p0::Stage::store_pixel(P.color, P.depth, pix, s, P.color_extra);
+        cpv_p0::Stage::store_pixel(P.color, P.depth, pix, s, P.color_extra, P.clear);
     }
+    __device__ __forceinline__ void clear_pixel(uint64_t pix) const { cpv_p0::Stage::clear_pixel(P.color, P.depth, pix, P.clear); }
 };
 
 /* Raster kernel: one CTA per screen tile (blockIdx.x = tile id). Without
@@ -244,7 +245,10 @@ extern "C" __global__ void CPV_PLAIN_BOUNDS cpv_raster(const __grid_constant__ C
         }
         __syncthreads();
         first = src.next(warp_sums);
-        if (first == 0u) return;
+        if (first == 0u) {
+            if (P.clear.mask) cpv_clear_tile(src, tx, ty);
+            return;
+        }
     }
     cpv_raster_tile(src, first, tx, ty, reinterpret_cast<CpvTri*>(cpv_dyn_smem), warp_sums);
 }

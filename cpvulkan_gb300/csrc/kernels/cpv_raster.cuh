@@ -535,6 +535,15 @@ __device__ __forceinline__ void cpv_list_small_warp(const CpvTri* tris, const ui
 #define CPV_RASTER_SMEM_BYTES \
     (CPV_BATCH * (sizeof(CpvTri) + 4u) + (CPV_DEFERRED ? CPV_NSLOT * (4u + 20u + 2u) : 0u) + (CPV_SPARSE ? CPV_SPARSE_BYTES : 0u))
 
+/* A tile without primitives under a pending clear (CpvClear). */
+template <class Source>
+__device__ __forceinline__ void cpv_clear_tile(const Source& src, uint32_t tx, uint32_t ty) {
+    for (uint32_t i = threadIdx.x; i < CPV_TILE_PX; i += CPV_RT_THREADS) {
+        const uint32_t x = tx * CPV_TILE + i % CPV_TILE, y = ty * CPV_TILE + i / CPV_TILE;
+        if (x < src.fb_width && y < src.fb_height) src.clear_pixel(static_cast<uint64_t>(y) * src.fb_width + x);
+    }
+}
+
 /* One screen tile (tx, ty) whose first batch holds `first` > 0 primitives:
  * loads the tile's attachment texels into registers, walks the tile's
  * primitives from `src` in API order in batches of CPV_BATCH (set-up into shared memory, then coverage, shading and the
@@ -551,6 +560,8 @@ __device__ __forceinline__ void cpv_list_small_warp(const CpvTri* tris, const ui
  *   bool table_only()                        a covered fragment is a blend-table lookup alone:
  *   uint32_t table_lookup(const CpvTri&, uint32_t texel)  the texel after it
  *   void load_pixel(uint64_t pix, CpvPixel&) / store_pixel(uint64_t pix, const CpvPixel&)
+ *                                            (the load gives the pending clear's texel, if there is one)
+ *   void clear_pixel(uint64_t pix)           writes the pending clear
  *   float vw, vh                             viewport extent (pixel centres)
  *   uint32_t fb_width, fb_height
  *

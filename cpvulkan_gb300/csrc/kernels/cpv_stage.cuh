@@ -591,55 +591,79 @@ __device__ __forceinline__ void cpv_store_extra(uint8_t* const* color, uint64_t 
 __device__ __forceinline__ void cpv_write_extra(const float blend_constants[4], const float* colour, CpvPixel& s);
 #endif
 
-__device__ __forceinline__ void cpv_load_pixel(const uint8_t* color, const uint8_t* depth, uint64_t pix, CpvPixel& s,
-                                               const uint8_t* const* extra = nullptr) {
-    cpv_load_colour(color, pix, s.colour);
+__device__ __forceinline__ void cpv_load_pixel(const uint8_t* color, const uint8_t* depth, uint64_t pix, CpvPixel& s, const uint8_t* const* extra,
+                                               const CpvClear& clear) {
+    if (clear.mask & 1u) {
+#pragma unroll
+        for (int w = 0; w < CPV_CF_WORDS; w++) s.colour[w] = clear.colour[w];
+    } else {
+        cpv_load_colour(color, pix, s.colour);
+    }
 #if CPV_EXTRA_CA > 0
     cpv_load_extra(extra, pix, s);
 #else
     (void)extra;
 #endif
+    const bool cleared = (clear.mask & 2u) != 0u;
 #if CPV_DEPTH_FORMAT == 124
-    s.depth_raw = reinterpret_cast<const uint16_t*>(depth)[pix];
+    s.depth_raw = cleared ? clear.depth[0] : reinterpret_cast<const uint16_t*>(depth)[pix];
     s.depth = cpv_decode_unorm16(s.depth_raw);
     s.stencil = 0u;
 #elif CPV_DEPTH_FORMAT == 126
-    s.depth_raw = reinterpret_cast<const uint32_t*>(depth)[pix];
+    s.depth_raw = cleared ? clear.depth[0] : reinterpret_cast<const uint32_t*>(depth)[pix];
     s.depth = __uint_as_float(s.depth_raw);
     s.stencil = 0u;
 #elif CPV_DEPTH_FORMAT == 130
-    const uint2 v = reinterpret_cast<const uint2*>(depth)[pix];
+    const uint2 v = cleared ? make_uint2(clear.depth[0], clear.depth[1]) : reinterpret_cast<const uint2*>(depth)[pix];
     s.depth_raw = v.x;
     s.depth = __uint_as_float(v.x);
     s.stencil = v.y & 0xFFu;
 #else
-    (void)depth;
+    (void)depth; (void)cleared;
     s.depth_raw = 0u;
     s.depth = 0.0f;
     s.stencil = 0u;
 #endif
 }
 
-__device__ __forceinline__ void cpv_store_pixel(uint8_t* color, uint8_t* depth, uint64_t pix, const CpvPixel& s, uint8_t* const* extra = nullptr) {
+__device__ __forceinline__ void cpv_store_pixel(uint8_t* color, uint8_t* depth, uint64_t pix, const CpvPixel& s, uint8_t* const* extra,
+                                                const CpvClear& clear) {
     cpv_store_colour(color, pix, s.colour);
 #if CPV_EXTRA_CA > 0
     cpv_store_extra(extra, pix, s);
 #else
     (void)extra;
 #endif
+    (void)clear;
 #if CPV_DEPTH_FORMAT == 124
     reinterpret_cast<uint16_t*>(depth)[pix] = static_cast<uint16_t>(s.depth_raw);
 #elif CPV_DEPTH_FORMAT == 126
     reinterpret_cast<uint32_t*>(depth)[pix] = s.depth_raw;
 #elif CPV_DEPTH_FORMAT == 130
     uint2* p = reinterpret_cast<uint2*>(depth) + pix;
-    uint2 v = *p;
+    uint2 v = (clear.mask & 2u) ? make_uint2(clear.depth[0], clear.depth[1]) : *p;
     v.x = s.depth_raw;
     v.y = (v.y & ~0xFFu) | (s.stencil & 0xFFu);
     *p = v;
 #else
     (void)depth;
 #endif
+}
+
+/* The clear alone, for a pixel that nothing touches. */
+__device__ __forceinline__ void cpv_clear_pixel(uint8_t* color, uint8_t* depth, uint64_t pix, const CpvClear& clear) {
+    if (clear.mask & 1u) cpv_store_colour(color, pix, clear.colour);
+    if (clear.mask & 2u) {
+#if CPV_DEPTH_FORMAT == 124
+        reinterpret_cast<uint16_t*>(depth)[pix] = static_cast<uint16_t>(clear.depth[0]);
+#elif CPV_DEPTH_FORMAT == 126
+        reinterpret_cast<uint32_t*>(depth)[pix] = clear.depth[0];
+#elif CPV_DEPTH_FORMAT == 130
+        reinterpret_cast<uint2*>(depth)[pix] = make_uint2(clear.depth[0], clear.depth[1]);
+#else
+        (void)depth;
+#endif
+    }
 }
 
 __device__ __forceinline__ void cpv_write_depth(CpvPixel& s, float mapped) {
@@ -1072,9 +1096,9 @@ __device__ __forceinline__ uint32_t cpv_table_lookup(const uint8_t* tables, uint
 
 #if CPV_LINEAR_BLEND
 /* The colour texel's channels decoded, and encoded again. */
-__device__ __forceinline__ void cpv_load_linear(const uint8_t* color, uint64_t pix, float d[4]) {
-    uint32_t t[1];
-    cpv_load_colour(color, pix, t);
+__device__ __forceinline__ void cpv_load_linear(const uint8_t* color, uint64_t pix, const CpvClear& clear, float d[4]) {
+    uint32_t t[1] = {clear.colour[0]};
+    if (!(clear.mask & 1u)) cpv_load_colour(color, pix, t);
 #pragma unroll
     for (int i = 0; i < 4; i++) d[i] = cpv_decode_unorm8(cpv_channel_get(t, i));
 }
@@ -1085,7 +1109,7 @@ __device__ __forceinline__ void cpv_store_linear(uint8_t* color, uint64_t pix, c
     cpv_store_colour(color, pix, t);
 }
 #else
-__device__ __forceinline__ void cpv_load_linear(const uint8_t*, uint64_t, float*) {}
+__device__ __forceinline__ void cpv_load_linear(const uint8_t*, uint64_t, const CpvClear&, float*) {}
 __device__ __forceinline__ void cpv_store_linear(uint8_t*, uint64_t, const float*) {}
 #endif
 
@@ -1122,10 +1146,12 @@ struct Stage {
 #endif
     }
     /* `extra`: the colour attachments after the first (unused without them) */
-    static __device__ __forceinline__ void load_pixel(const uint8_t* c, const uint8_t* d, uint64_t pix, CpvPixel& s, const uint8_t* const* extra) {
-        cpv_load_pixel(c, d, pix, s, extra);
+    static __device__ __forceinline__ void load_pixel(const uint8_t* c, const uint8_t* d, uint64_t pix, CpvPixel& s, const uint8_t* const* extra,
+                                                      const CpvClear& clear) {
+        cpv_load_pixel(c, d, pix, s, extra, clear);
     }
-    static __device__ __forceinline__ void store_pixel(uint8_t* c, uint8_t* d, uint64_t pix, const CpvPixel& s, uint8_t* const* extra) {
-        cpv_store_pixel(c, d, pix, s, extra);
+    static __device__ __forceinline__ void store_pixel(uint8_t* c, uint8_t* d, uint64_t pix, const CpvPixel& s, uint8_t* const* extra, const CpvClear& clear) {
+        cpv_store_pixel(c, d, pix, s, extra, clear);
     }
+    static __device__ __forceinline__ void clear_pixel(uint8_t* c, uint8_t* d, uint64_t pix, const CpvClear& clear) { cpv_clear_pixel(c, d, pix, clear); }
 };

@@ -43,6 +43,7 @@ struct Module {
     cudaKernel_t vertex = nullptr;        // batched modules: the vertex stage
     uint32_t vs_stride = 0;               // batched modules: output floats per vertex slot
     bool blend_table = false;             // the pipeline blends a per-primitive constant colour
+    bool linear = false;                  // per-draw modules: the raster reads and writes the colour attachment alone
     bool batched = false;
     uint32_t tile_shift = 4;
     uint32_t raster_threads = 256;
@@ -141,6 +142,7 @@ struct BatchDraws {
     uint8_t* color_extra[CPV_MAX_CA - 1] = {};
     uint32_t fb_width = 0, fb_height = 0;
     float vw = 0.0f, vh = 0.0f;
+    CpvClear clear{};  // the pass's clears that the batch's raster makes
 };
 
 // Device state of one batched render pass of a recorded command buffer:
@@ -160,6 +162,8 @@ public:
     // buffers first when an earlier launch needed more than they hold.
     int launch(const Module& m, cudaStream_t stream);
     uint64_t primitives() const { return prims_; }
+    // The clears its raster makes (CpvClear::mask).
+    uint32_t clears() const { return P_.clear.mask; }
     uint32_t kernels_per_launch() const { return kernels_; }
     // Vertex slots of the vertex stage (0 when no draw has any).
     uint64_t vertex_slots() const { return vs_slots_; }
