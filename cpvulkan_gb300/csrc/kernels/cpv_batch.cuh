@@ -165,8 +165,9 @@ extern "C" __global__ void __launch_bounds__(CPV_RT_THREADS, CPV_RT_MIN_BLOCKS) 
         const uint32_t tx = tile % B.tiles_x, ty = tile / B.tiles_x;
         uint64_t begin = 0, end = static_cast<uint64_t>(B.total_blocks) * CPV_BATCH_BLOCK;
         if (!overflow) {
-            begin = B.tile_begin[tile];
-            end = B.tile_end[tile];
+            const uint2 range = B.tile_range[tile];
+            begin = range.x;
+            end = range.y;
         }
         CpvBatchSource src{B, begin, end, overflow, tx, ty, B.vw, B.vh, B.fb_width, B.fb_height, 0u};
         const uint32_t first = src.next(warp_sums);

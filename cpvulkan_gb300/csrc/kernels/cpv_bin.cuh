@@ -194,45 +194,73 @@ extern "C" __global__ void __launch_bounds__(256) cpv_bin_write(const uint2* __r
     }
 }
 
-/* ---- exclusive scan of u32 (three-level, 2048 elements per block) ---- */
+/* ---- batched binning: pairs, stable radix sort by tile, tile ranges ----
+ *
+ * The batched path bins every draw of a render pass at once. Set-up writes
+ * one tile rectangle per primitive and the pair count of each 256-primitive
+ * block; cpv_batch_scan makes the counts positions within chunks of
+ * CPV_SCAN_BLOCK blocks; cpv_batch_emit writes the (tile, primitive) pairs
+ * in primitive order; a stable radix sort by tile (one digit of at most
+ * CPV_RADIX_DIGITS, or two) groups them by tile while keeping primitive
+ * (API) order inside each tile. Each digit takes three launches:
+ * cpv_radix_hist, cpv_bin_scan over its counts, cpv_radix_scatter. The
+ * groups of one digit may lie in any order (cpv_bin_scan places them by an
+ * atomic): a tile's pairs stay together and in order all the same. With one
+ * digit the scan's ranges are the tiles'; with two, cpv_tile_ranges records
+ * where each tile's run starts and ends. Sizes that depend on the data (the
+ * pair count) are read on the device, so the sequence has fixed launch
+ * shapes, needs no memset and can be captured in a CUDA graph. Pairs beyond
+ * the capacity are not written; the raster then scans the rectangles instead
+ * (same image). */
 
 #define CPV_SCAN_THREADS 256
 #define CPV_SCAN_ITEMS 8
 #define CPV_SCAN_BLOCK (CPV_SCAN_THREADS * CPV_SCAN_ITEMS)
+#define CPV_RADIX_THREADS 256
+#define CPV_RADIX_DIGITS 1024
+#define CPV_RADIX_ITEMS 8
+#define CPV_RADIX_CHUNK (CPV_RADIX_THREADS * CPV_RADIX_ITEMS)
 
-__device__ __forceinline__ uint32_t cpv_block_exclusive_scan(uint32_t v, uint32_t& block_total) {
-    __shared__ uint32_t warp_sums[CPV_SCAN_THREADS / 32];
-    __shared__ uint32_t total_sh;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= static_cast<uint32_t>(o)) incl += t;
-    }
-    if (lane == 31u) warp_sums[warp] = incl;
-    __syncthreads();
-    if (warp == 0u) {
-        const uint32_t s = lane < CPV_SCAN_THREADS / 32 ? warp_sums[lane] : 0u;
-        uint32_t si = s;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, si, o);
-            if (lane >= static_cast<uint32_t>(o)) si += t;
-        }
-        if (lane < CPV_SCAN_THREADS / 32) warp_sums[lane] = si - s;
-        if (lane == CPV_SCAN_THREADS / 32 - 1) total_sh = si;
-    }
-    __syncthreads();
-    const uint32_t r = warp_sums[warp] + incl - v;
-    block_total = total_sh;
-    __syncthreads();
-    return r;
+__device__ __forceinline__ uint32_t cpv_pairs_in_bounds(const uint32_t* pair_total, uint32_t capacity) {
+    const uint32_t p = *pair_total;
+    return p <= capacity ? p : 0u;
 }
 
-/* Level scan: out[i] = exclusive prefix within the block; block_sums[b] = block total. */
-extern "C" __global__ void __launch_bounds__(CPV_SCAN_THREADS) cpv_scan_blocks(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                                                                              uint64_t n, uint32_t* __restrict__ block_sums) {
+/* Exclusive sum over the warp; `total` is the warp's sum. */
+__device__ __forceinline__ uint32_t cpv_warp_exclusive(uint32_t v, uint32_t& total) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t incl = v;
+#pragma unroll
+    for (uint32_t o = 1; o < 32u; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    return incl - v;
+}
+
+/* Block-wide exclusive sum over 256 threads; `total` is the block's sum. */
+__device__ __forceinline__ uint32_t cpv_block256_exclusive(uint32_t v, uint32_t* warp_sums /* [8] */, uint32_t& total) {
+    const uint32_t warp = threadIdx.x >> 5;
+    uint32_t mine;
+    const uint32_t excl = cpv_warp_exclusive(v, mine);
+    if ((threadIdx.x & 31u) == 0u) warp_sums[warp] = mine;
+    __syncthreads();
+    uint32_t base = 0;
+    total = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 8u; k++) {
+        const uint32_t s = warp_sums[k];
+        base += k < warp ? s : 0u;
+        total += s;
+    }
+    return base + excl;
+}
+
+/* out[i] = exclusive prefix of in within its chunk; chunk_sums[b] = chunk total. */
+extern "C" __global__ void __launch_bounds__(CPV_SCAN_THREADS) cpv_batch_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t n,
+                                                                              uint32_t* __restrict__ chunk_sums) {
+    __shared__ uint32_t warp_sums[8];
     const uint64_t base = static_cast<uint64_t>(blockIdx.x) * CPV_SCAN_BLOCK + static_cast<uint64_t>(threadIdx.x) * CPV_SCAN_ITEMS;
     uint32_t v[CPV_SCAN_ITEMS];
     uint32_t sum = 0;
@@ -241,90 +269,113 @@ extern "C" __global__ void __launch_bounds__(CPV_SCAN_THREADS) cpv_scan_blocks(c
         v[i] = (base + i < n) ? in[base + i] : 0u;
         sum += v[i];
     }
-    uint32_t total = 0;
-    uint32_t run = cpv_block_exclusive_scan(sum, total);
+    uint32_t total;
+    uint32_t run = cpv_block256_exclusive(sum, warp_sums, total);
 #pragma unroll
     for (int i = 0; i < CPV_SCAN_ITEMS; i++) {
         if (base + i < n) out[base + i] = run;
         run += v[i];
     }
-    if (threadIdx.x == 0 && block_sums) block_sums[blockIdx.x] = total;
+    if (threadIdx.x == 0) chunk_sums[blockIdx.x] = total;
 }
 
-/* out[i] += add[block(i)]; optionally writes the grand total. */
-extern "C" __global__ void __launch_bounds__(CPV_SCAN_THREADS) cpv_scan_add(uint32_t* __restrict__ out, uint64_t n, const uint32_t* __restrict__ add) {
-    const uint64_t base = static_cast<uint64_t>(blockIdx.x) * CPV_SCAN_BLOCK;
-    const uint32_t a = add[blockIdx.x];
-    for (uint32_t i = threadIdx.x; i < CPV_SCAN_BLOCK; i += CPV_SCAN_THREADS) {
-        if (base + i < n) out[base + i] += a;
-    }
-}
-
-/* total = last exclusive prefix + last input. */
-extern "C" __global__ void cpv_scan_total(const uint32_t* __restrict__ in, const uint32_t* __restrict__ out, uint64_t n, uint32_t* __restrict__ total) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *total = n ? out[n - 1] + in[n - 1] : 0u;
-}
-
-/* ---- batched binning: pairs, stable radix sort by tile, tile ranges ----
- *
- * The batched path bins every draw of a render pass at once. Set-up writes
- * one tile rectangle per primitive and the pair count of each 256-primitive
- * block; after an exclusive scan of the block counts, cpv_batch_emit writes
- * the (tile, primitive) pairs in primitive order; a stable LSD radix sort by
- * tile (8-bit digits, one or two passes) groups them by tile while keeping
- * primitive (API) order inside each tile; cpv_tile_ranges records where each
- * tile's run starts and ends. Sizes that depend on the data (the pair count)
- * are read on the device, so the sequence has fixed launch shapes and can be
- * captured in a CUDA graph. Pairs beyond the capacity are not written; the
- * raster then scans the rectangles instead (same image). */
-
-#define CPV_RADIX_THREADS 256
-#define CPV_RADIX_DIGITS 256
-
-__device__ __forceinline__ uint32_t cpv_pairs_in_bounds(const uint32_t* pair_total, uint32_t capacity) {
-    const uint32_t p = *pair_total;
-    return p <= capacity ? p : 0u;
-}
-
-/* Block-wide exclusive sum over 256 threads. */
-__device__ __forceinline__ uint32_t cpv_block256_exclusive(uint32_t v, uint32_t* warp_sums /* [8] */) {
+/* One warp per set-up block, eight blocks (of one chunk) a CTA: the block's
+ * pairs at the position of its chunk (summed here from the chunks' totals)
+ * + block_offsets[block] + the pairs of its earlier primitives. A block
+ * without pairs has no rectangles written this frame and emits nothing. A
+ * lane writes its primitive's pairs; those of one with many are written by
+ * the warp. Two dependent loads, then stores of 6 bytes a pair: latency-bound
+ * (99 M primitives, 30 M pairs: 260 us; a CTA per block, a block-wide scan
+ * and a division a pair took 500, every register of one fewer CTA an SM 272).
+ * CTA 0 stores the pair total and clears the words of the kernels
+ * that follow: words[2], the raster's tile counter, and words[4..7], the two
+ * digits' totals. */
+#define CPV_EMIT_LANE_PAIRS 16u
+extern "C" __global__ void __launch_bounds__(256, 6) cpv_batch_emit(const uint2* __restrict__ rects, const uint32_t* __restrict__ block_pairs,
+                                                                 const uint32_t* __restrict__ block_offsets, const uint32_t* __restrict__ chunk_sums,
+                                                                 uint32_t blocks, uint32_t tiles_x, uint16_t* __restrict__ keys,
+                                                                 uint32_t* __restrict__ vals, uint32_t capacity, uint32_t* __restrict__ words) {
+    __shared__ uint32_t sums[2][8];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= static_cast<uint32_t>(o)) incl += t;
+    const uint32_t block = blockIdx.x * 8u + warp;
+    const bool any = block < blocks;
+    const uint32_t block_n = any ? block_pairs[block] : 0u, block_pos = any ? block_offsets[block] : 0u;
+    const uint32_t chunk = blockIdx.x * 8u / CPV_SCAN_BLOCK, chunks = (blocks + CPV_SCAN_BLOCK - 1u) / CPV_SCAN_BLOCK;
+    uint32_t before = 0u, total = 0u;
+    for (uint32_t i = threadIdx.x; i < chunks; i += 256u) {
+        const uint32_t s = chunk_sums[i];
+        total += s;
+        before += i < chunk ? s : 0u;
     }
-    if (lane == 31u) warp_sums[warp] = incl;
+    before = __reduce_add_sync(0xFFFFFFFFu, before);
+    total = __reduce_add_sync(0xFFFFFFFFu, total);
+    if (lane == 0u) {
+        sums[0][warp] = before;
+        sums[1][warp] = total;
+    }
     __syncthreads();
-    uint32_t base = 0;
-    for (uint32_t k = 0; k < warp; k++) base += warp_sums[k];
-    return base + incl - v;
-}
-
-/* One block per 256-primitive set-up block: the block's pairs at
- * block_offsets[block] + (pairs of the block's earlier primitives). A block
- * without pairs has no rectangles written this frame and emits nothing. */
-extern "C" __global__ void __launch_bounds__(256) cpv_batch_emit(const uint2* __restrict__ rects, const uint32_t* __restrict__ block_pairs,
-                                                                 const uint32_t* __restrict__ block_offsets, uint32_t tiles_x,
-                                                                 uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t capacity,
-                                                                 const uint32_t* __restrict__ pair_total) {
-    __shared__ uint32_t warp_sums[8];
-    if (block_pairs[blockIdx.x] == 0u) return;
-    const uint64_t g = static_cast<uint64_t>(blockIdx.x) * 256u + threadIdx.x;
-    const uint2 r = rects[g];
-    const uint32_t x0 = r.x & 0xFFFFu, y0 = r.x >> 16, x1 = r.y & 0xFFFFu, y1 = r.y >> 16;
-    const uint32_t w = x1 - x0;
-    const uint32_t n = w * (y1 - y0);
-    const uint32_t excl = cpv_block256_exclusive(n, warp_sums);
-    if (*pair_total > capacity) return;
-    const uint32_t base = block_offsets[blockIdx.x] + excl;
-    for (uint32_t k = 0; k < n; k++) {
-        const uint64_t pos = static_cast<uint64_t>(base) + k;
-        if (pos >= capacity) break;  /* only reachable if the pair total wrapped 32 bits */
-        const uint32_t ty = y0 + k / w, tx = x0 + k % w;
-        keys[pos] = ty * tiles_x + tx;
-        vals[pos] = static_cast<uint32_t>(g);
+    before = total = 0u;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        before += sums[0][w];
+        total += sums[1][w];
+    }
+    if (blockIdx.x == 0u && threadIdx.x < 8u && (threadIdx.x == 0u || threadIdx.x == 2u || threadIdx.x >= 4u)) words[threadIdx.x] = threadIdx.x ? 0u : total;
+    if (total > capacity || block_n == 0u) return;
+    uint2 r[8];
+    const uint32_t g0 = block * 256u + lane;
+#pragma unroll
+    for (uint32_t j = 0; j < 8u; j++) r[j] = rects[g0 + 32u * j];
+    uint32_t pos = before + block_pos;
+#pragma unroll
+    for (uint32_t j = 0; j < 8u; j++) {
+        const uint32_t x0 = r[j].x & 0xFFFFu, y0 = r[j].x >> 16;
+        const uint32_t w = (r[j].y & 0xFFFFu) - x0;
+        const uint32_t n = w * ((r[j].y >> 16) - y0);
+        /* positions by ballots for up to three pairs each, else by a scan */
+        const uint32_t ones = __ballot_sync(0xFFFFFFFFu, (n & 1u) != 0u), more = __ballot_sync(0xFFFFFFFFu, n > 1u);
+        if ((ones | more) == 0u) continue;
+        const uint32_t earlier = (1u << lane) - 1u;
+        uint32_t p = pos + __popc(ones & earlier), step = __popc(ones), many = 0u;
+        if (more) {
+            if (__any_sync(0xFFFFFFFFu, n > 3u)) {
+                p = pos + cpv_warp_exclusive(n, step);
+                many = __ballot_sync(0xFFFFFFFFu, n > CPV_EMIT_LANE_PAIRS);
+            } else {
+                const uint32_t twos = __ballot_sync(0xFFFFFFFFu, (n & 2u) != 0u);
+                p += 2u * __popc(twos & earlier);
+                step += 2u * __popc(twos);
+            }
+        }
+        pos += step;
+        uint32_t key = y0 * tiles_x + x0;
+        while (many) {
+            const uint32_t src = __ffs(static_cast<int>(many)) - 1u;
+            many &= many - 1u;
+            const uint32_t s_key = __shfl_sync(0xFFFFFFFFu, key, src), s_w = __shfl_sync(0xFFFFFFFFu, w, src), s_n = __shfl_sync(0xFFFFFFFFu, n, src);
+            const uint32_t s_p = __shfl_sync(0xFFFFFFFFu, p, src), s_g = __shfl_sync(0xFFFFFFFFu, g0, src) + 32u * j;
+            for (uint32_t k = lane; k < s_n; k += 32u) {
+                const uint32_t row = k / s_w;
+                if (s_p + k < capacity) {  /* always, unless the pair total wrapped 32 bits */
+                    keys[s_p + k] = static_cast<uint16_t>(s_key + row * tiles_x + (k - row * s_w));
+                    vals[s_p + k] = s_g;
+                }
+            }
+        }
+        if (n <= CPV_EMIT_LANE_PAIRS) {
+            uint32_t x = 0u;
+            for (uint32_t k = 0; k < n; k++, p++) {
+                if (p < capacity) {
+                    keys[p] = static_cast<uint16_t>(key);
+                    vals[p] = g0 + 32u * j;
+                }
+                key++;
+                if (++x == w) {
+                    x = 0u;
+                    key += tiles_x - w;
+                }
+            }
+        }
     }
 }
 
@@ -370,80 +421,168 @@ extern "C" __global__ void __launch_bounds__(256) cpv_index_range(const CpvDrawP
     }
 }
 
-/* Contiguous item range of CTA c of `ctas` over n items. */
+/* Contiguous item range of CTA c of `ctas` over n items, starting at a
+ * multiple of 8 (16 bytes of keys). */
 __device__ __forceinline__ void cpv_cta_range(uint32_t n, uint32_t c, uint32_t ctas, uint32_t& begin, uint32_t& end) {
-    const uint32_t per = (n + ctas - 1u) / ctas;
-    const uint64_t b = static_cast<uint64_t>(per) * c, e = b + per;
+    const uint64_t per = ((n + ctas - 1u) / ctas + 7u) & ~7u;
+    const uint64_t b = per * c, e = b + per;
     begin = static_cast<uint32_t>(b < n ? b : n);
     end = static_cast<uint32_t>(e < n ? e : n);
 }
 
-/* hist[digit * gridDim.x + cta] = items of the CTA's range with that digit. */
-extern "C" __global__ void __launch_bounds__(CPV_RADIX_THREADS) cpv_radix_hist(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ pair_total,
-                                                                               uint32_t capacity, uint32_t shift, uint32_t* __restrict__ hist) {
-    __shared__ uint32_t counts[CPV_RADIX_DIGITS];
-    counts[threadIdx.x] = 0u;
+/* counts[cta * digits + digit] = items of the CTA's range with that digit.
+ * With tile_range (the first of two digits) it is also cleared here, for
+ * cpv_tile_ranges to fill. */
+extern "C" __global__ void __launch_bounds__(CPV_RADIX_THREADS) cpv_radix_hist(const uint16_t* __restrict__ keys, const uint32_t* __restrict__ pair_total,
+                                                                               uint32_t capacity, uint32_t shift, uint32_t digits,
+                                                                               uint32_t* __restrict__ counts, uint2* __restrict__ tile_range, uint32_t tiles) {
+    __shared__ uint32_t count[CPV_RADIX_DIGITS];
+    for (uint32_t d = threadIdx.x; d < digits; d += CPV_RADIX_THREADS) count[d] = 0u;
+    if (tile_range)
+        for (uint32_t i = blockIdx.x * CPV_RADIX_THREADS + threadIdx.x; i < tiles; i += gridDim.x * CPV_RADIX_THREADS) tile_range[i] = make_uint2(0u, 0u);
     __syncthreads();
     uint32_t begin, end;
     cpv_cta_range(cpv_pairs_in_bounds(pair_total, capacity), blockIdx.x, gridDim.x, begin, end);
-    for (uint32_t i = begin + threadIdx.x; i < end; i += CPV_RADIX_THREADS) atomicAdd(&counts[(keys[i] >> shift) & 0xFFu], 1u);
+    for (uint32_t i = begin + 8u * threadIdx.x; i < end; i += 8u * CPV_RADIX_THREADS) {
+        /* the buffer is a multiple of 8 keys long */
+        const uint4 v = *reinterpret_cast<const uint4*>(keys + i);
+        const uint32_t word[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (uint32_t k = 0; k < 8u; k++)
+            if (i + k < end) atomicAdd(&count[(((word[k >> 1] >> (16u * (k & 1u))) & 0xFFFFu) >> shift) & (digits - 1u)], 1u);
+    }
     __syncthreads();
-    hist[threadIdx.x * gridDim.x + blockIdx.x] = counts[threadIdx.x];
+    for (uint32_t d = threadIdx.x; d < digits; d += CPV_RADIX_THREADS) counts[blockIdx.x * digits + d] = count[d];
 }
 
-/* Stable scatter: offsets = exclusive scan of hist (digit-major). Each CTA
- * walks its range in order, 256 items at a time; an item's position is its
- * digit's running offset plus the number of earlier items of the sub-chunk
- * with the same digit (earlier warps, then earlier lanes). */
-extern "C" __global__ void __launch_bounds__(CPV_RADIX_THREADS) cpv_radix_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-                                                                                  uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
+/* Stable scatter to `offsets` (the counts made positions). Each CTA walks
+ * its range in order, CPV_RADIX_CHUNK items at a time: every warp ranks its
+ * 256 consecutive items by digit (a match-any rank within 32, the warp's own
+ * count per digit between them), the counts are scanned over the warps and
+ * the digits, and the chunk is put in digit order in shared memory first, so
+ * that the writes to a digit's run are consecutive. keys_out may be null (the
+ * last digit of a one-digit sort). Bound by the chunk's chain of shared
+ * memory steps at four CTAs an SM (30 M pairs, 14400 tiles, both passes: 267 us;
+ * 646 before, with 256 items a step written straight from the match and
+ * 32-bit keys; ballots per bit instead of the match 328). */
+extern "C" __global__ void __launch_bounds__(CPV_RADIX_THREADS) cpv_radix_scatter(const uint16_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+                                                                                  uint16_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
                                                                                   const uint32_t* __restrict__ pair_total, uint32_t capacity, uint32_t shift,
-                                                                                  const uint32_t* __restrict__ offsets) {
-    __shared__ uint32_t running[CPV_RADIX_DIGITS];
-    __shared__ uint32_t warp_count[CPV_RADIX_THREADS / 32][CPV_RADIX_DIGITS];
+                                                                                  uint32_t digits, const uint32_t* __restrict__ offsets) {
+    __shared__ uint32_t next[CPV_RADIX_DIGITS];   /* the digit's next position */
+    __shared__ uint32_t place[CPV_RADIX_DIGITS];  /* that, less the digit's first position in the chunk */
+    __shared__ uint16_t first[CPV_RADIX_DIGITS];  /* the digit's first position in the chunk */
+    __shared__ uint16_t warp_count[CPV_RADIX_THREADS / 32][CPV_RADIX_DIGITS];
+    __shared__ uint32_t chunk_val[CPV_RADIX_CHUNK];
+    __shared__ uint16_t chunk_key[CPV_RADIX_CHUNK];
+    __shared__ uint32_t warp_sums[8];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    running[threadIdx.x] = offsets[threadIdx.x * gridDim.x + blockIdx.x];
+    const uint32_t per_thread = (digits + CPV_RADIX_THREADS - 1u) / CPV_RADIX_THREADS, d0 = threadIdx.x * per_thread;
     uint32_t begin, end;
     cpv_cta_range(cpv_pairs_in_bounds(pair_total, capacity), blockIdx.x, gridDim.x, begin, end);
-    for (uint32_t base = begin; base < end; base += CPV_RADIX_THREADS) {
+    if (begin >= end) return;
+    for (uint32_t d = threadIdx.x; d < digits; d += CPV_RADIX_THREADS) {
+        next[d] = offsets[blockIdx.x * digits + d];
 #pragma unroll
-        for (uint32_t w = 0; w < CPV_RADIX_THREADS / 32; w++) warp_count[w][threadIdx.x] = 0u;
-        __syncthreads();
-        const uint32_t i = base + threadIdx.x;
-        const bool valid = i < end;
-        uint32_t key = 0, val = 0, digit = CPV_RADIX_DIGITS + lane;  /* invalid lanes never match a digit */
-        if (valid) {
-            key = keys_in[i];
-            val = vals_in[i];
-            digit = (key >> shift) & 0xFFu;
-        }
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, digit);
-        const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-        if (valid && rank == 0u) warp_count[warp][digit] = __popc(peers);
-        __syncthreads();
-        if (valid) {
-            uint32_t pos = running[digit] + rank;
-            for (uint32_t w = 0; w < warp; w++) pos += warp_count[w][digit];
-            keys_out[pos] = key;
-            vals_out[pos] = val;
-        }
-        __syncthreads();
-        uint32_t add = 0;
+        for (uint32_t w = 0; w < CPV_RADIX_THREADS / 32u; w++) warp_count[w][d] = 0u;
+    }
+    __syncthreads();
+    for (uint32_t base = begin; base < end; base += CPV_RADIX_CHUNK) {
+        const uint32_t items = end - base < CPV_RADIX_CHUNK ? end - base : CPV_RADIX_CHUNK;
+        uint32_t key[CPV_RADIX_ITEMS], val[CPV_RADIX_ITEMS], rank[CPV_RADIX_ITEMS];  /* rank: first the lanes of the same digit */
+        const uint32_t i0 = warp * 32u * CPV_RADIX_ITEMS + lane;
 #pragma unroll
-        for (uint32_t w = 0; w < CPV_RADIX_THREADS / 32; w++) add += warp_count[w][threadIdx.x];
-        running[threadIdx.x] += add;
+        for (uint32_t j = 0; j < CPV_RADIX_ITEMS; j++) {
+            const bool valid = i0 + 32u * j < items;
+            key[j] = valid ? keys_in[base + i0 + 32u * j] : 0u;
+            val[j] = valid ? vals_in[base + i0 + 32u * j] : 0u;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < CPV_RADIX_ITEMS; j++)
+            rank[j] = __match_any_sync(0xFFFFFFFFu, i0 + 32u * j < items ? (key[j] >> shift) & (digits - 1u) : CPV_RADIX_DIGITS + lane);
+#pragma unroll
+        for (uint32_t j = 0; j < CPV_RADIX_ITEMS; j++) {
+            const bool valid = i0 + 32u * j < items;
+            const uint32_t digit = (key[j] >> shift) & (digits - 1u);
+            const uint32_t peers = rank[j];
+            const uint32_t earlier = __popc(peers & ((1u << lane) - 1u));
+            const uint32_t seen = warp_count[warp][digit];
+            rank[j] = seen + earlier;
+            __syncwarp();
+            if (valid && earlier == 0u) warp_count[warp][digit] = static_cast<uint16_t>(seen + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        uint32_t count[CPV_RADIX_DIGITS / CPV_RADIX_THREADS], sum = 0u;
+#pragma unroll
+        for (uint32_t m = 0; m < CPV_RADIX_DIGITS / CPV_RADIX_THREADS; m++) {
+            uint32_t run = 0u;
+            if (m < per_thread && d0 + m < digits) {
+#pragma unroll
+                for (uint32_t w = 0; w < CPV_RADIX_THREADS / 32u; w++) {
+                    const uint32_t c = warp_count[w][d0 + m];
+                    warp_count[w][d0 + m] = static_cast<uint16_t>(run);
+                    run += c;
+                }
+            }
+            count[m] = run;
+            sum += run;
+        }
+        uint32_t total;
+        uint32_t run = cpv_block256_exclusive(sum, warp_sums, total);
+#pragma unroll
+        for (uint32_t m = 0; m < CPV_RADIX_DIGITS / CPV_RADIX_THREADS; m++) {
+            if (m < per_thread && d0 + m < digits) {
+                const uint32_t at = next[d0 + m];
+                first[d0 + m] = static_cast<uint16_t>(run);
+                place[d0 + m] = at - run;
+                next[d0 + m] = at + count[m];
+                run += count[m];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < CPV_RADIX_ITEMS; j++) {
+            if (i0 + 32u * j < items) {
+                const uint32_t digit = (key[j] >> shift) & (digits - 1u);
+                const uint32_t p = first[digit] + warp_count[warp][digit] + rank[j];
+                chunk_key[p] = static_cast<uint16_t>(key[j]);
+                chunk_val[p] = val[j];
+            }
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < items; i += CPV_RADIX_THREADS) {
+            const uint32_t k = chunk_key[i];
+            const uint32_t p = place[(k >> shift) & (digits - 1u)] + i;
+            if (keys_out) keys_out[p] = static_cast<uint16_t>(k);
+            vals_out[p] = chunk_val[i];
+        }
+        for (uint32_t d = lane; d < digits; d += 32u) warp_count[warp][d] = 0u;
         __syncthreads();
     }
 }
 
-/* tile_begin / tile_end (zeroed beforehand) from the sorted keys. */
-extern "C" __global__ void __launch_bounds__(256) cpv_tile_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ pair_total,
-                                                                  uint32_t capacity, uint32_t* __restrict__ tile_begin, uint32_t* __restrict__ tile_end) {
+/* tile_range (zeroed beforehand) from the sorted keys, eight a thread. */
+extern "C" __global__ void __launch_bounds__(256) cpv_tile_ranges(const uint16_t* __restrict__ keys, const uint32_t* __restrict__ pair_total,
+                                                                  uint32_t capacity, uint2* __restrict__ tile_range) {
     const uint32_t n = cpv_pairs_in_bounds(pair_total, capacity);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t k = keys[i];
-        if (i == 0u || keys[i - 1u] != k) tile_begin[k] = i;
-        if (i + 1u == n || keys[i + 1u] != k) tile_end[k] = i + 1u;
+    for (uint64_t at = 8ull * (blockIdx.x * 256u + threadIdx.x); at < n; at += 8ull * 256u * gridDim.x) {
+        const uint32_t i = static_cast<uint32_t>(at);
+        const uint4 v = *reinterpret_cast<const uint4*>(keys + i);
+        const uint32_t word[4] = {v.x, v.y, v.z, v.w};
+        uint32_t before = i ? keys[i - 1u] : 0x10000u;
+#pragma unroll
+        for (uint32_t k = 0; k < 8u; k++) {
+            const uint32_t key = (word[k >> 1] >> (16u * (k & 1u))) & 0xFFFFu;
+            if (i + k < n) {
+                if (key != before) {
+                    tile_range[key].x = i + k;
+                    if (before < 0x10000u) tile_range[before].y = i + k;
+                }
+                if (i + k + 1u == n) tile_range[key].y = n;
+            }
+            before = key;
+        }
     }
 }
 

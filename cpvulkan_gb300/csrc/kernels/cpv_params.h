@@ -155,13 +155,11 @@ struct CpvBatchParams {
     /* binning */
     uint2* rects;                 /* per primitive tile rectangle, packed */
     uint32_t* block_pairs;        /* per set-up block: (primitive, tile) pairs */
-    const uint32_t* block_offsets;/* exclusive scan of block_pairs */
     const uint32_t* pair_total;   /* device word: pairs of the batch */
     uint32_t pair_capacity;
     uint32_t pad0;
     const uint32_t* sorted_prims; /* pair primitives sorted by tile, API order within a tile */
-    const uint32_t* tile_begin;   /* per tile: range in sorted_prims */
-    const uint32_t* tile_end;
+    const uint2* tile_range;      /* per tile: range in sorted_prims */
     uint32_t* tile_counter;       /* persistent raster work queue */
     uint32_t* status;
     /* pixel-centre NDC of every column (fb_width) and row (fb_height):

@@ -286,7 +286,6 @@ Scratch::~Scratch() {
     cudaFree(ranges_);
     cudaFree(list_);
     cudaFree(list_rects_);
-    for (auto* p : scan_) cudaFree(p);
     cudaFree(words_);
     cudaFree(tables_);
 }
@@ -315,18 +314,6 @@ int Scratch::reserve_list(uint64_t entries) {
 
 int Scratch::reserve_tables(uint64_t bytes) { return grow_tracked(tables_, tables_cap_, bytes); }
 
-int Scratch::reserve_scan(uint64_t n) {
-    int level = 0;
-    while (n > CPV_SCAN_BLOCK && level < 8) {
-        n = (n + CPV_SCAN_BLOCK - 1) / CPV_SCAN_BLOCK;
-        // two arrays per level (sums and scanned sums) share one allocation
-        const int r = grow_tracked(scan_[level], scan_cap_[level], 2 * n);
-        if (r != kOk) return r;
-        level++;
-    }
-    return kOk;
-}
-
 int Scratch::ensure_words() {
     if (words_) return kOk;
     if (cudaMalloc(reinterpret_cast<void**>(&words_), kWordsBytes) != cudaSuccess) {
@@ -335,41 +322,6 @@ int Scratch::ensure_words() {
     }
     cudaMemset(words_, 0, kWordsBytes);
     generation_++;
-    return kOk;
-}
-
-namespace {
-
-int scan_level(cudaStream_t stream, const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* total, Scratch& sc, int level) {
-    const uint64_t blocks = (n + CPV_SCAN_BLOCK - 1) / CPV_SCAN_BLOCK;
-    if (blocks <= 1) {
-        cpv_scan_blocks<<<1, CPV_SCAN_THREADS, 0, stream>>>(in, out, n, nullptr);
-        count_launch();
-    } else {
-        uint32_t* sums = sc.scan_level(level);
-        uint32_t* sums_scanned = sums + blocks;
-        cpv_scan_blocks<<<static_cast<unsigned>(blocks), CPV_SCAN_THREADS, 0, stream>>>(in, out, n, sums);
-        count_launch();
-        const int r = scan_level(stream, sums, sums_scanned, blocks, nullptr, sc, level + 1);
-        if (r != kOk) return r;
-        cpv_scan_add<<<static_cast<unsigned>(blocks), CPV_SCAN_THREADS, 0, stream>>>(out, n, sums_scanned);
-        count_launch();
-    }
-    if (total) {
-        cpv_scan_total<<<1, 32, 0, stream>>>(in, out, n, total);
-        count_launch();
-    }
-    return kOk;
-}
-
-}  // namespace
-
-int scan_u32(cudaStream_t stream, const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* total, Scratch& sc) {
-    int r = sc.reserve_scan(n);
-    if (r != kOk) return r;
-    r = scan_level(stream, in, out, n, total, sc, 0);
-    if (r != kOk) return r;
-    CPV_CUDA(cudaGetLastError());
     return kOk;
 }
 
@@ -629,11 +581,11 @@ BatchPlan::~BatchPlan() {
     dev_free(rects_);
     dev_free(block_pairs_);
     dev_free(block_offsets_);
+    dev_free(chunk_sums_);
     free_pairs();
     dev_free(hist_);
-    dev_free(hist_offsets_);
-    dev_free(tile_begin_);
-    dev_free(tile_end_);
+    dev_free(digit_range_);
+    dev_free(tile_range_);
     dev_free(words_);
     dev_free(ndc_);
     dev_free(vs_pos_);
@@ -651,11 +603,19 @@ void BatchPlan::free_pairs() {
     cap_ = 0;
 }
 
-int BatchPlan::alloc_pairs(uint32_t capacity) {
+int BatchPlan::alloc_pairs(uint64_t pairs, uint64_t entries) {
     free_pairs();
+    // the sort's 32-bit positions may step past the last pair
+    const uint32_t capacity = static_cast<uint32_t>(entries < 0xFFFF0000ull ? entries : 0xFFFF0000ull);
+    // Whole chunks for at most four sorting CTAs an SM. One digit's scatter on
+    // GB300, 608 CTAs then this: 14.6 us then 8.5 for 316k pairs and 1024
+    // digits (155 CTAs; 12.2 at 78 of two chunks), 15.9 then 12.4 for 1.7 M
+    // pairs and 128 digits (413 CTAs, two chunks each instead of 1.4).
+    const uint64_t per = ((pairs + radix_max_ctas_ - 1) / radix_max_ctas_ + CPV_RADIX_CHUNK - 1) / CPV_RADIX_CHUNK * CPV_RADIX_CHUNK;
+    radix_ctas_ = per ? static_cast<uint32_t>((pairs + per - 1) / per) : 1u;
     for (int i = 0; i < 2; i++) {
         int r;
-        if ((r = dev_alloc(keys_[i], capacity)) != kOk || (r = dev_alloc(vals_[i], capacity)) != kOk) {
+        if ((r = dev_alloc(keys_[i], capacity + 8ull)) != kOk || (r = dev_alloc(vals_[i], capacity)) != kOk) {
             free_pairs();
             return r;
         }
@@ -695,18 +655,26 @@ int BatchPlan::build(const Module& m, const BatchDraws& in, cudaStream_t stream)
         set_last_error("batch plan: attachment needs more than 65536 tiles");
         return kErrInvalid;
     }
-    passes_ = tiles_ > 256u ? 2u : 1u;
+    // One digit sorts up to CPV_RADIX_DIGITS tiles (316k pairs on 920 tiles:
+    // 17 us, 35 as two digits), two halves of the tile index more.
+    uint32_t tile_bits = 1;
+    while ((1u << tile_bits) < tiles_) tile_bits++;
+    passes_ = (1u << tile_bits) > CPV_RADIX_DIGITS ? 2u : 1u;
+    digit_bits_ = (tile_bits + passes_ - 1u) / passes_;
+    const uint64_t chunks = (blocks + CPV_SCAN_BLOCK - 1) / CPV_SCAN_BLOCK;
     int r;
     if ((r = dev_alloc(draws_, n)) != kOk || (r = dev_alloc(pipeline_, n)) != kOk || (r = dev_alloc(draw_block_, n + 1)) != kOk ||
         (r = dev_alloc(block_draw_, block_draw.size())) != kOk || (r = dev_alloc(rects_, blocks * CPV_BATCH_BLOCK)) != kOk ||
         (r = dev_alloc(block_pairs_, blocks)) != kOk || (r = dev_alloc(block_offsets_, blocks)) != kOk ||
-        (r = dev_alloc(tile_begin_, tiles_)) != kOk || (r = dev_alloc(tile_end_, tiles_)) != kOk || (r = dev_alloc(words_, 64)) != kOk)
+        (r = dev_alloc(chunk_sums_, chunks)) != kOk || (r = dev_alloc(digit_range_, 1ull << digit_bits_)) != kOk ||
+        (r = dev_alloc(tile_range_, passes_ > 1u ? 65536u : 1u)) != kOk || (r = dev_alloc(words_, 64)) != kOk)
         return r;
     if (cudaMallocHost(reinterpret_cast<void**>(&pinned_pairs_), 64) != cudaSuccess) {
         cudaGetLastError();
         set_last_error("batch plan: pinned word allocation failed");
         return kErrOutOfMemory;
     }
+    *pinned_pairs_ = 0;
     CPV_CUDA(cudaEventCreateWithFlags(&done_, cudaEventDisableTiming));
     CPV_CUDA(cudaMemcpy(draws_, in.draws.data(), n * sizeof(CpvDrawParams), cudaMemcpyHostToDevice));
     CPV_CUDA(cudaMemcpy(pipeline_, in.pipeline.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice));
@@ -737,12 +705,8 @@ int BatchPlan::build(const Module& m, const BatchDraws& in, cudaStream_t stream)
     if (per_sm < 1) per_sm = 1;
     raster_ctas_ = static_cast<uint32_t>(sms * per_sm);
     if (raster_ctas_ > tiles_) raster_ctas_ = tiles_;
-    radix_ctas_ = static_cast<uint32_t>(sms * 4);
-    if ((r = dev_alloc(hist_, static_cast<uint64_t>(CPV_RADIX_DIGITS) * radix_ctas_)) != kOk ||
-        (r = dev_alloc(hist_offsets_, static_cast<uint64_t>(CPV_RADIX_DIGITS) * radix_ctas_)) != kOk)
-        return r;
-    // Scan levels for both scans, reserved now so that no launch allocates.
-    if ((r = scan_.reserve_scan(blocks)) != kOk || (r = scan_.reserve_scan(static_cast<uint64_t>(CPV_RADIX_DIGITS) * radix_ctas_)) != kOk) return r;
+    radix_max_ctas_ = static_cast<uint32_t>(sms * 4);
+    if ((r = dev_alloc(hist_, static_cast<uint64_t>(radix_max_ctas_) << digit_bits_)) != kOk) return r;
 
     P_ = CpvBatchParams{};
     P_.draws = draws_;
@@ -763,10 +727,8 @@ int BatchPlan::build(const Module& m, const BatchDraws& in, cudaStream_t stream)
     P_.tiles_y = tiles_y;
     P_.rects = rects_;
     P_.block_pairs = block_pairs_;
-    P_.block_offsets = block_offsets_;
     P_.pair_total = words_;
-    P_.tile_begin = tile_begin_;
-    P_.tile_end = tile_end_;
+    P_.tile_range = passes_ > 1u ? tile_range_ : digit_range_;
     P_.tile_counter = words_ + 2;
     P_.status = words_ + 1;
     P_.ndc_x = ndc_;
@@ -783,16 +745,25 @@ int BatchPlan::build(const Module& m, const BatchDraws& in, cudaStream_t stream)
         }
         CPV_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(m.setup_rects), dim3(static_cast<unsigned>(blocks)), dim3(CPV_BATCH_BLOCK), args, 0, stream));
         count_launch();
-        if ((r = scan_u32(stream, block_pairs_, block_offsets_, blocks, words_, scan_)) != kOk) return r;
+        if ((r = scan_blocks(stream)) != kOk) return r;
+        std::vector<uint32_t> sums(chunks);
+        CPV_CUDA(cudaMemcpyAsync(sums.data(), chunk_sums_, chunks * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+        CPV_CUDA(cudaStreamSynchronize(stream));
+        for (uint32_t v : sums) *pinned_pairs_ += v;
     }
-    CPV_CUDA(cudaMemcpyAsync(pinned_pairs_, words_, 4, cudaMemcpyDeviceToHost, stream));
-    CPV_CUDA(cudaStreamSynchronize(stream));
     const uint64_t pairs = *pinned_pairs_;
-    uint64_t cap = pairs + pairs / 4 + (1u << 20);
-    if (cap > 0xFFFFFFFFull) cap = 0xFFFFFFFFull;
     // CPV_BATCH_PAIR_CAPACITY forces a capacity (tests of the overflow path).
-    if (const uint32_t forced = env_u32("CPV_BATCH_PAIR_CAPACITY", 0u)) cap = forced;
-    return alloc_pairs(static_cast<uint32_t>(cap));
+    if (const uint32_t forced = env_u32("CPV_BATCH_PAIR_CAPACITY", 0u)) return alloc_pairs(pairs, forced);
+    return alloc_pairs(pairs, pairs + pairs / 4 + (1u << 20));
+}
+
+// Positions of the set-up blocks' pairs within chunks, and the chunks' totals.
+int BatchPlan::scan_blocks(cudaStream_t stream) {
+    const uint32_t blocks = P_.total_blocks;
+    cpv_batch_scan<<<(blocks + CPV_SCAN_BLOCK - 1) / CPV_SCAN_BLOCK, CPV_SCAN_THREADS, 0, stream>>>(block_pairs_, block_offsets_, blocks, chunk_sums_);
+    CPV_CUDA(cudaGetLastError());
+    count_launch();
+    return kOk;
 }
 
 // The vertex stage: every vertex id of a triangle draw's range, of every
@@ -942,27 +913,28 @@ int BatchPlan::enqueue(const Module& m, cudaStream_t stream) {
         count_launch();
     }
     profile_begin(stream, "cpv_batch_bin");
-    int r = scan_u32(stream, block_pairs_, block_offsets_, blocks, words_, scan_);
+    const int r = scan_blocks(stream);
     if (r != kOk) return r;
-    cpv_batch_emit<<<blocks, 256, 0, stream>>>(rects_, block_pairs_, block_offsets_, P_.tiles_x, keys_[0], vals_[0], cap_, words_);
+    cpv_batch_emit<<<(blocks + 7u) / 8u, 256, 0, stream>>>(rects_, block_pairs_, block_offsets_, chunk_sums_, blocks, P_.tiles_x, keys_[0], vals_[0], cap_,
+                                                           words_);
     count_launch();
+    const uint32_t digits = 1u << digit_bits_;
     for (uint32_t pass = 0; pass < passes_; pass++) {
-        const uint32_t src = pass & 1u, dst = src ^ 1u;
-        cpv_radix_hist<<<radix_ctas_, CPV_RADIX_THREADS, 0, stream>>>(keys_[src], words_, cap_, 8u * pass, hist_);
-        count_launch();
-        r = scan_u32(stream, hist_, hist_offsets_, static_cast<uint64_t>(CPV_RADIX_DIGITS) * radix_ctas_, nullptr, scan_);
-        if (r != kOk) return r;
-        cpv_radix_scatter<<<radix_ctas_, CPV_RADIX_THREADS, 0, stream>>>(keys_[src], vals_[src], keys_[dst], vals_[dst], words_, cap_, 8u * pass,
-                                                                       hist_offsets_);
-        count_launch();
+        const uint32_t src = pass & 1u, dst = src ^ 1u, shift = digit_bits_ * pass;
+        cpv_radix_hist<<<radix_ctas_, CPV_RADIX_THREADS, 0, stream>>>(keys_[src], words_, cap_, shift, digits, hist_,
+                                                                     passes_ > 1u && pass == 0u ? tile_range_ : nullptr, tiles_);
+        cpv_bin_scan<<<(digits + CPV_BIN_SCAN_BINS - 1u) / CPV_BIN_SCAN_BINS, CPV_BIN_SCAN_THREADS, 0, stream>>>(
+            hist_, radix_ctas_, digits, digit_range_, reinterpret_cast<unsigned long long*>(words_ + 4 + 2 * pass));
+        cpv_radix_scatter<<<radix_ctas_, CPV_RADIX_THREADS, 0, stream>>>(keys_[src], vals_[src], passes_ > 1u ? keys_[dst] : nullptr, vals_[dst], words_, cap_,
+                                                                        shift, digits, hist_);
+        count_launch(3);
     }
     const uint32_t fin = passes_ & 1u;
     P_.sorted_prims = vals_[fin];
-    CPV_CUDA(cudaMemsetAsync(tile_begin_, 0, tiles_ * sizeof(uint32_t), stream));
-    CPV_CUDA(cudaMemsetAsync(tile_end_, 0, tiles_ * sizeof(uint32_t), stream));
-    cpv_tile_ranges<<<radix_ctas_, 256, 0, stream>>>(keys_[fin], words_, cap_, tile_begin_, tile_end_);
-    count_launch();
-    CPV_CUDA(cudaMemsetAsync(words_ + 2, 0, sizeof(uint32_t), stream));
+    if (passes_ > 1u) {
+        cpv_tile_ranges<<<2 * radix_ctas_, 256, 0, stream>>>(keys_[fin], words_, cap_, tile_range_);
+        count_launch();
+    }
     profile_end(stream);
     {
         void* args[] = {&P_};
@@ -999,11 +971,9 @@ int BatchPlan::launch(const Module& m, cudaStream_t stream) {
     // correctly through the rectangle scan; grow the buffers for the next.
     if (exec_ && cudaEventQuery(done_) == cudaSuccess && *pinned_pairs_ > cap_) {
         const uint64_t pairs = *pinned_pairs_;
-        uint64_t cap = pairs + pairs / 4 + (1u << 20);
-        if (cap > 0xFFFFFFFFull) cap = 0xFFFFFFFFull;
         cudaGraphExecDestroy(exec_);
         exec_ = nullptr;
-        const int r = alloc_pairs(static_cast<uint32_t>(cap));
+        const int r = alloc_pairs(pairs, pairs + pairs / 4 + (1u << 20));
         if (r != kOk) return r;
     }
     cudaGetLastError();

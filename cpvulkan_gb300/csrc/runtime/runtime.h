@@ -72,7 +72,6 @@ public:
     int reserve_rects(uint64_t prims);
     int reserve_bins(uint64_t entries, uint64_t bins);  // the count matrix, and a list range per bin
     int reserve_list(uint64_t entries);                 // ids and rectangles
-    int reserve_scan(uint64_t n);
     int reserve_tables(uint64_t bytes);
     uint8_t* tables() const { return tables_; }
     uint2* rects() const { return rects_; }
@@ -82,7 +81,6 @@ public:
     uint32_t* list_rects() const { return list_rects_; }
     uint32_t list_capacity() const { return static_cast<uint32_t>(std::min(list_cap_, list_rects_cap_)); }
     uint32_t* words() const { return words_; }  // kWordsBytes
-    uint32_t* scan_level(int level) const { return scan_[level]; }
     int ensure_words();
     // Incremented whenever a buffer is (re)allocated: work captured in a CUDA
     // graph against older pointers must be captured again.
@@ -102,8 +100,6 @@ private:
     uint64_t list_cap_ = 0;
     uint32_t* list_rects_ = nullptr;
     uint64_t list_rects_cap_ = 0;
-    uint32_t* scan_[8] = {};
-    uint64_t scan_cap_[8] = {};
     uint32_t* words_ = nullptr;
     uint8_t* tables_ = nullptr;
     uint64_t tables_cap_ = 0;
@@ -170,12 +166,13 @@ public:
 
 private:
     int enqueue(const Module& m, cudaStream_t stream);
-    int alloc_pairs(uint32_t capacity);
+    // Buffers of `entries` pairs, for about `pairs` a frame.
+    int alloc_pairs(uint64_t pairs, uint64_t entries);
+    int scan_blocks(cudaStream_t stream);
     void free_pairs();
     int build_vertex_stage(const Module& m, const BatchDraws& in, cudaStream_t stream);
 
     CpvBatchParams P_{};
-    Scratch scan_;
     CpvDrawParams* draws_ = nullptr;
     uint32_t* pipeline_ = nullptr;
     uint32_t* draw_block_ = nullptr;
@@ -183,14 +180,14 @@ private:
     uint2* rects_ = nullptr;
     uint32_t* block_pairs_ = nullptr;
     uint32_t* block_offsets_ = nullptr;
-    uint32_t* keys_[2] = {};
+    uint32_t* chunk_sums_ = nullptr;
+    uint16_t* keys_[2] = {};
     uint32_t* vals_[2] = {};
     uint32_t cap_ = 0;
     uint32_t* hist_ = nullptr;
-    uint32_t* hist_offsets_ = nullptr;
-    uint32_t* tile_begin_ = nullptr;
-    uint32_t* tile_end_ = nullptr;
-    uint32_t* words_ = nullptr;         // [0] pair total, [1] status, [2] tile counter
+    uint2* digit_range_ = nullptr;      // of the sort's last scan; the tiles' with one digit
+    uint2* tile_range_ = nullptr;       // of cpv_tile_ranges
+    uint32_t* words_ = nullptr;         // [0] pair total, [1] status, [2] tile counter, [4..7] the digits' totals
     float* ndc_ = nullptr;              // pixel-centre NDC of the columns, then the rows
     float* vs_pos_ = nullptr;           // vertex stage: NDC position and clip w per slot
     float* vs_var_ = nullptr;           // vertex stage: outputs per slot
@@ -200,7 +197,7 @@ private:
     uint32_t* pinned_pairs_ = nullptr;  // pair total of the last launch (host)
     cudaEvent_t done_ = nullptr;
     uint64_t prims_ = 0;
-    uint32_t tiles_ = 0, radix_ctas_ = 0, raster_ctas_ = 0, passes_ = 1, kernels_ = 0;
+    uint32_t tiles_ = 0, radix_ctas_ = 0, radix_max_ctas_ = 0, raster_ctas_ = 0, passes_ = 1, digit_bits_ = 1, kernels_ = 0;
     cudaGraphExec_t exec_ = nullptr;
 };
 
@@ -243,9 +240,6 @@ int fill_rect(cudaStream_t stream, uint8_t* base, uint64_t pitch, uint32_t w, ui
 // aligned), the unaligned remainder by cudaMemcpyAsync. CPV_H2D_KERNEL=0
 // uses cudaMemcpyAsync for everything.
 int copy_host_to_device(cudaStream_t stream, uint8_t* dst, const uint8_t* host, uint64_t bytes);
-
-// Exclusive scan helper (exposed for tests through the C ABI).
-int scan_u32(cudaStream_t stream, const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* total, Scratch& scratch);
 
 const char* last_error();
 void set_last_error(const std::string& e);
