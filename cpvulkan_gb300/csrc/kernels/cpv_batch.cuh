@@ -50,9 +50,15 @@ extern "C" __global__ void __launch_bounds__(CPV_BATCH_BLOCK) cpv_batch_vs(const
 }
 
 /* register budget of the set-up: eight resident CTAs of 256 threads (32
- * registers a thread). Its dependent loads (draw table, indices, vertex
- * slots) leave it latency-bound: C4 set-up 11.8 ms at eight, 12.0 at six,
- * 13.4 at five */
+ * registers a thread). Issue-bound, with dependent loads (draw table,
+ * indices, vertex slots) to hide: 99 M triangles take 1100 us at eight, 1101
+ * at seven, 1212 at six. 1342 us with a pretest whose loops ran over each lane's own box,
+ * 64-bit box limits and a bounds check per index; the pretest of four by four pixels
+ * instead of four pixels in all leaves 26 M of 30 M pairs (512 draws' raster
+ * 3002 us, then 2659; 2 M triangles at 1920x1080: set-up 39 us, then 35,
+ * raster 216, then 175). Limits of 2, 3 and 4 pixels a side in one step each:
+ * 5060, 4840 and 4920 us a 512-draw frame, 317, 301 and 289 us a 1920x1080
+ * one; three first and the fourth where it is needed 4831 and 287. */
 #ifndef CPV_SETUP_MIN_BLOCKS
 #define CPV_SETUP_MIN_BLOCKS 8
 #endif

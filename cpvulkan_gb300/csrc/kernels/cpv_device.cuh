@@ -665,4 +665,21 @@ __device__ __forceinline__ uint32_t cpv_vertex_id(const CpvDrawParams& P, uint32
     return static_cast<uint32_t>(P.vertex_offset) + index;
 }
 
+/* The three of a triangle: one bounds check when the largest is inside. */
+__device__ __forceinline__ void cpv_vertex_ids(const CpvDrawParams& P, const uint32_t raw[3], uint32_t id[3]) {
+    const uint32_t size = P.index_size, last = max(raw[0], max(raw[1], raw[2]));
+    if (size != 0u && (static_cast<uint64_t>(P.first) + last + 1u) * size <= P.ib_bytes) {
+        const uint8_t* base = P.ib + static_cast<uint64_t>(P.first) * size;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const uint8_t* at = base + static_cast<uint64_t>(raw[k]) * size;
+            const uint32_t index = size == 2u ? __ldg(reinterpret_cast<const uint16_t*>(at)) : __ldg(reinterpret_cast<const uint32_t*>(at));
+            id[k] = static_cast<uint32_t>(P.vertex_offset) + index;
+        }
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) id[k] = cpv_vertex_id(P, raw[k]);
+}
+
 #endif /* CPV_DEVICE_CUH */

@@ -174,26 +174,70 @@ __device__ __forceinline__ bool cpv_covers(const CpvTri& t, float xf, float yf, 
     return !(w[0] < 0.0f || w[1] < 0.0f || w[2] < 0.0f);
 }
 
+/* Whether a primitive covers any pixel centre of a box of at most four by
+ * four pixels (cpv_covers): every column and row of the first three by
+ * three, a smaller box's repeated, so that no loop's trips differ between
+ * lanes; the rest where the box is larger and none is covered yet. A rounded
+ * difference is negative where its first operand is the smaller and nowhere
+ * else (equal or NaN operands give 0 or NaN, also for infinities), so a
+ * triangle's products are compared and not subtracted. Pixel centres come
+ * from the tables when given (the box lies inside the attachment). */
+__device__ __forceinline__ bool cpv_covers_any(const CpvTri& t, int4 b, float vw, float vh, const float* ndc_x, const float* ndc_y) {
+    auto column = [&](int32_t i) {
+        const int32_t x = min(b.x + i, b.z - 1);
+        return ndc_x ? __ldg(ndc_x + x) : cpv_pixel_ndc(x, vw);
+    };
+    auto row = [&](int32_t i) {
+        const int32_t y = min(b.y + i, b.w - 1);
+        return ndc_y ? __ldg(ndc_y + y) : cpv_pixel_ndc(y, vh);
+    };
+    bool any = false;
+#if CPV_ANY_LINES
+    if (((__float_as_uint(t.wf.w) >> 6) & 3u) == 3u) {
+        for (int32_t i = 0; i < 16; i++) {
+            float w[3];
+            any = cpv_covers(t, column(i & 3), row(i >> 2), w) || any;
+        }
+        return any;
+    }
+#endif
+    float tx[4][3];
+    auto set_column = [&](int32_t c) {
+        const float xf = column(c);
+#pragma unroll
+        for (int k = 0; k < 3; k++) tx[c][k] = __fmul_rn(__fsub_rn(xf, t.e[k].x), t.e[k].w);
+    };
+    auto test_row = [&](int32_t r, int32_t c0, int32_t c1) {
+        const float yf = row(r);
+        float ty[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) ty[k] = __fmul_rn(__fsub_rn(yf, t.e[k].y), t.e[k].z);
+#pragma unroll
+        for (int32_t c = 0; c < 4; c++)
+            if (c >= c0 && c < c1) any = any | !((tx[c][0] < ty[0]) | (tx[c][1] < ty[1]) | (tx[c][2] < ty[2]));
+    };
+#pragma unroll
+    for (int32_t c = 0; c < 3; c++) set_column(c);
+#pragma unroll
+    for (int32_t r = 0; r < 3; r++) test_row(r, 0, 3);
+    if (!any && (b.z - b.x > 3 || b.w - b.y > 3)) {
+        set_column(3);
+#pragma unroll
+        for (int32_t r = 0; r < 3; r++) test_row(r, 3, 4);
+        test_row(3, 0, 4);
+    }
+    return any;
+}
+
 /* Tile rectangle of a set-up primitive with pixel box b (empty when culled, off screen, or
- * when a bounding box of at most four pixels covers none of its pixel
- * centres — the raster would find no fragment there either). Packed as
+ * when none of the pixel centres of a box of at most four by four is covered
+ * — the raster would find no fragment there either). Packed as
  * x0 | y0 << 16, x1 | y1 << 16 in tile units, end exclusive. */
 __device__ __forceinline__ uint2 cpv_tile_rect(const CpvTri& t, int4 b, float vw, float vh, const float* ndc_x = nullptr, const float* ndc_y = nullptr) {
     uint32_t r[4] = {0, 0, 0, 0};
     if (cpv_tri_live(t)) {
         bool any = true;
-        if ((b.z - b.x) * (b.w - b.y) <= 4) {
-            /* pixel centres from the tables when given (the box lies inside
-             * the attachment), else computed */
-            any = false;
-            for (int32_t y = b.y; y < b.w; y++) {
-                const float yf = ndc_y ? __ldg(ndc_y + y) : cpv_pixel_ndc(y, vh);
-                for (int32_t x = b.x; x < b.z; x++) {
-                    float w[3];
-                    if (cpv_covers(t, ndc_x ? __ldg(ndc_x + x) : cpv_pixel_ndc(x, vw), yf, w)) any = true;
-                }
-            }
-        }
+        if (b.z - b.x <= 4 && b.w - b.y <= 4) any = cpv_covers_any(t, b, vw, vh, ndc_x, ndc_y);
         if (any) {
             r[0] = static_cast<uint32_t>(b.x >> CPV_TILE_SHIFT);
             r[1] = static_cast<uint32_t>(b.y >> CPV_TILE_SHIFT);

@@ -310,21 +310,14 @@ __device__ __forceinline__ void cpv_setup_tri(const CpvDrawParams& P, const floa
         sx[k] = cpv_f2i(__fmul_rn(__fmul_rn(__fadd_rn(Pn[k][0], 1.0f), 0.5f), vw));
         sy[k] = cpv_f2i(__fmul_rn(__fmul_rn(__fadd_rn(Pn[k][1], 1.0f), 0.5f), vh));
     }
-    const int64_t minx = min(sx[0], min(sx[1], sx[2]));
-    const int64_t miny = min(sy[0], min(sy[1], sy[2]));
-    const int64_t maxx = max(sx[0], max(sx[1], sx[2]));
-    const int64_t maxy = max(sy[0], max(sy[1], sy[2]));
-    int64_t x0 = minx > 0 ? minx : 0, y0 = miny > 0 ? miny : 0;
-    int64_t x1 = maxx + 1, y1 = maxy + 1;
-    const int64_t iw = cpv_f2i(vw), ih = cpv_f2i(vh);
-    x1 = x1 < iw ? x1 : iw;
-    y1 = y1 < ih ? y1 : ih;
-    x1 = x1 < static_cast<int64_t>(P.fb_width) ? x1 : static_cast<int64_t>(P.fb_width);
-    y1 = y1 < static_cast<int64_t>(P.fb_height) ? y1 : static_cast<int64_t>(P.fb_height);
-    box.x = static_cast<int32_t>(x0);
-    box.y = static_cast<int32_t>(y0);
-    box.z = static_cast<int32_t>(x1 > x0 ? x1 : x0);
-    box.w = static_cast<int32_t>(y1 > y0 ? y1 : y0);
+    /* the ends, one past the largest pixel, are limited before the addition
+     * (which could overflow past the limit) */
+    const int32_t maxx = max(sx[0], max(sx[1], sx[2])), maxy = max(sy[0], max(sy[1], sy[2]));
+    const int32_t lx = min(cpv_f2i(vw), static_cast<int32_t>(P.fb_width)), ly = min(cpv_f2i(vh), static_cast<int32_t>(P.fb_height));
+    box.x = max(min(sx[0], min(sx[1], sx[2])), 0);
+    box.y = max(min(sy[0], min(sy[1], sy[2])), 0);
+    box.z = max(maxx < lx ? maxx + 1 : lx, box.x);
+    box.w = max(maxy < ly ? maxy + 1 : ly, box.y);
 
     float area = cpv_edge(Pn[0][0], Pn[0][1], Pn[1][0], Pn[1][1], Pn[2][0], Pn[2][1]);
     /* Edges (a → b): front (area >= 0) w0 = E(p1,p2), w1 = E(p2,p0), w2 = E(p0,p1);
@@ -387,10 +380,12 @@ __device__ __forceinline__ void cpv_setup(const CpvDrawParams& P, uint64_t g, Cp
     uint32_t raw[3], instance, pslot, inst;
     cpv_tri_vertices(P, g32, raw, instance, pslot, inst);
     const uint32_t vs_count = P.vs_count;
+    uint32_t vids[3];
+    cpv_vertex_ids(P, raw, vids);
     float Pn[3][4];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const uint32_t vid = cpv_vertex_id(P, raw[k]);
+        const uint32_t vid = vids[k];
         const uint32_t rel = vid - P.vs_lo;
         if (rel < vs_count) {
             const uint64_t slot = static_cast<uint64_t>(inst) * vs_count + rel;
