@@ -618,12 +618,13 @@ ModuleConfig batch_config(const std::vector<Pipeline*>& pipelines) {
 // A pass of at least CPV_BATCH_MIN_DRAWS (16) draws, or of at least
 // CPV_BATCH_MIN_PRIMS (2^20) primitives when none of its pipelines uses
 // blend tables (CPV_BATCH=0: none). The second rule exists because the
-// per-draw path bins through a (tile x span) count matrix whose size grows
-// with the tiles times the primitives / 256, while the batched path sorts
-// the (tile, primitive) pairs: the 2.09 M-triangle heightfield renders in
-// 0.59 ms batched against 0.74 ms per draw. Blend-table pipelines stay per
-// draw, where their tables exist (the 400k-triangle blend scene: 2.84 ms per
-// draw, 3.28 ms batched).
+// batched path shades each vertex once and sorts the (tile, primitive) pairs:
+// the 2.09 M-triangle heightfield takes 0.27 ms batched and 0.46 per draw. Of
+// one draw below the limit, 500k triangles at 2048x2048 take 0.183 and 0.194
+// ms, 180k at 1366x767 0.128 and 0.120, and a serving mix with the limit at
+// 400k takes as long (16.9 ms, 16.8; 24 at 100k, where requests build plans).
+// Blend-table pipelines stay per draw, where their tables and the register
+// blend exist (the 400k-triangle blend scene: 2.14 ms per draw, 2.89 batched).
 // Indirect draws count as the draws their records hold (at recording, where
 // the records are not read yet, as their maximum draw count, with no
 // primitives).

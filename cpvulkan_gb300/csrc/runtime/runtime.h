@@ -207,9 +207,9 @@ void batch_stats(uint64_t out[3]);
 
 // Fixed binning scratch for submissions that may not allocate: one
 // 32 MiB file-scope device array per device. A draw needs 8 bytes per
-// primitive for its tile rectangles plus its bins; one that does not fit even
-// with one span per tile is rejected (kErrOutOfMemory, message in
-// last_error()). The array is shared by every queue of the process on that
+// primitive for its tile rectangles; its bins take what is left, and a draw
+// whose bins do not fit filters the rectangles instead. One whose rectangles
+// do not fit is rejected (kErrOutOfMemory, message in last_error()). The array is shared by every queue of the process on that
 // device, so draw_plain_static calls whose work overlaps on the GPU race.
 #define CPV_STATIC_SCRATCH_BYTES (32ull << 20)
 // Resolves the array's device address for the current device

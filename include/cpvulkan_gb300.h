@@ -118,8 +118,7 @@ CPV_EXPORT void cpv_profile_reset(void);
  *   rewrites is checked again when its draw runs, and one that no longer
  *   fits then ends the submission with VK_ERROR_OUT_OF_DEVICE_MEMORY after
  *   the commands before it were enqueued.
- * - The bin counters must start at zero for every draw; the call zeroes
- *   them on the queue's stream itself. Nothing else needs an initial value.
+ * - Nothing in the array needs an initial value.
  * - The array is shared by every queue of the process on a device: calls
  *   whose work overlaps on the GPU (two queues, or two devices' queues on
  *   one GPU) race on it. Serialise them, e.g. wait for the fence of one
