@@ -297,12 +297,12 @@ def run_reference(args, world, rank, dist):
               "the frame's draws in API order into its attachments, continuing across steps: %d draws (%d triangles) in %d timed steps "
               "of about %.0f s" % (draws, tris, len(per_step), args.ref_seconds))
     line = {
-        "impl": "reference", "metric": "Mtri/s", "value": round(value, 3), "unit": "Mtri/s", "n_gpus": world, "steps": args.steps,
+        "impl": "reference", "metric": "Mtri/s", "value": round(value, 6), "unit": "Mtri/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(1000 * dt / len(per_step), 3), "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded scene)",
         "config": {"workload": args.config, "description": cfg_desc, "triangles": scene.triangles},
-        "cpu_baseline": {"value": round(value, 3), "unit": "Mtri/s", "cores": threads, "kind": "port", "sample": sample},
-        "e2e": {"value": round(value, 3), "unit": "Mtri/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
+        "cpu_baseline": {"value": round(value, 6), "unit": "Mtri/s", "cores": threads, "kind": "port", "sample": sample},
+        "e2e": {"value": round(value, 6), "unit": "Mtri/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
     print(json.dumps(line), flush=True)
 
