@@ -156,6 +156,7 @@ std::string compose_module(const std::vector<std::string>& stages, const std::ve
         int depth = mc.depth ? static_cast<int>(mc.depth) : (mc.samples ? 16 : 24);
         if (const char* v = std::getenv("CPV_SLOT_DEPTH")) depth = std::atoi(v);
         if (depth >= 1 && depth <= 255) src << "#define CPV_SLOT_DEPTH " << depth << "\n";
+        if (batched) src << "#define CPV_DENSE 32\n";  // see cpv_raster.cuh
         if (const char* v = std::getenv("CPV_SMALL_PX")) {
             const int k = std::atoi(v);
             if (k >= 1 && k <= 1024) src << "#define CPV_SMALL_PX " << k << "\n";

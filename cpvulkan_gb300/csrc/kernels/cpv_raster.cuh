@@ -33,6 +33,19 @@
 #ifndef CPV_SMALL_PX
 #define CPV_SMALL_PX 64 /* sparse: largest in-tile bounding box listed by the warp-spread tests (C4 raster 21.37 ms at 64, 21.65 at 32, 21.86 at 128) */
 #endif
+#ifndef CPV_DENSE
+/* sparse: large primitives' pixels per tile pixel from which a batch runs the
+ * immediate schedule. A pixel whose list overflows walks the whole batch, a
+ * warp of the immediate schedule only what may cover its block: 6k smooth
+ * quads at 1280x720 take 420 us without this rule, 273 at 2 to 8, 275 at 16,
+ * 289 at 24, 355 at 32; 300 half-float triangles 416, 322, 328, 340 and 386. By
+ * the boxes instead of the triangles' areas, slivers count too much (180k
+ * triangles at 1366x767: 95 us, 150 at 8 by boxes). Batched modules mix their
+ * draws' small and large primitives in a batch, where the lists are better for
+ * longer (compose_module: 32): 512 draws at 2560x1440 take 2436 us without
+ * it, 2878 at 8, 2588 at 16, 2485 at 24, 2437 at 32. */
+#define CPV_DENSE 8
+#endif
 #ifndef CPV_RT_WARPS
 #define CPV_RT_WARPS 8
 #endif
@@ -704,7 +717,7 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
     uint32_t* list_count = boxes + CPV_BATCH;  /* per tile pixel: fragments listed this batch */
     uint8_t* list_j = reinterpret_cast<uint8_t*>(list_count + CPV_TILE_PX);  /* per tile pixel: CPV_SLOT_DEPTH batch indices */
     uint8_t* large = list_j + CPV_TILE_PX * CPV_SLOT_DEPTH;                  /* batch indices of large primitives */
-    __shared__ uint32_t large_count[2];  /* of this batch and the next, by turns */
+    __shared__ uint32_t large_count[2];  /* of this batch and the next, by turns: their number (at most 256), and from bit 9 their pixels */
     if (threadIdx.x == 0u) large_count[0] = 0u;
     uint32_t turn = 0u;
     for (uint32_t i = threadIdx.x; i < CPV_TILE_PX; i += CPV_RT_THREADS) list_count[i] = 0u;
@@ -755,8 +768,14 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
 #if CPV_SPARSE
             /* 1. large primitives (box covering more than CPV_SMALL_PX pixels
              *    of the tile) are collected, in any order (by a block scan and
-             *    three barriers after the set-up: rasters 2 to 4% longer) */
-            if (cpv_tile_class(boxes[i]) == 2u) large[atomicAdd(&large_count[turn], 1u)] = static_cast<uint8_t>(i);
+             *    three barriers after the set-up: rasters 2 to 4% longer), and
+             *    the pixels they may cover summed: the triangle's area, if
+             *    that is less than the box's (an estimate that only chooses
+             *    the schedule; NaN counts as none) */
+            if (cpv_tile_class(boxes[i]) == 2u) {
+                const float px = fminf(fmaxf(t.za.w * (src.vw * src.vh * 0.125f), 0.0f), static_cast<float>((rx1 - rx0) * (ry1 - ry0)));
+                large[atomicAdd(&large_count[turn], 1u + (static_cast<uint32_t>(px) << 9)) & 0x1FFu] = static_cast<uint8_t>(i);
+            }
 #endif
 #if CPV_WARP_BLOCKS
             live_flags[i] = live ? (0x100u | (centres_finite && cpv_edges_finite(t) ? 1u : 0u)) : 0u;
@@ -780,10 +799,11 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
         __syncthreads();
 #endif
 #if CPV_SPARSE
-        const uint32_t nlarge = large_count[turn];
+        const uint32_t nlarge = large_count[turn] & 0x1FFu, large_px = large_count[turn] >> 9;
         turn ^= 1u;
-        /* mostly large primitives: this batch runs the immediate schedule */
-        const bool immediate_batch = nlarge * 4u >= 3u * n;
+        /* mostly large primitives, or enough of them over each pixel that its
+         * list may overflow: this batch runs the immediate schedule */
+        const bool immediate_batch = nlarge * 4u >= 3u * n || large_px >= CPV_DENSE * static_cast<uint32_t>(CPV_TILE_PX);
         if (!immediate_batch) {
             /* 2. small primitives: each warp lists the pixels its 32 cover */
             for (uint32_t j0 = threadIdx.x & ~31u; j0 < n; j0 += CPV_RT_THREADS)
