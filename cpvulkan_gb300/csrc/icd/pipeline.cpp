@@ -150,8 +150,8 @@ std::string compose_module(const std::vector<std::string>& stages, const std::ve
     // fallback. Measured on GB300: 24 for flat or lit shading (C4 raster
     // 34.0 ms, against 39.4 at 16 and 36.5 at 32), 16 when a fragment shader
     // samples images (the heightfield raster 0.41 ms, against 0.44 at 32).
-    // CPV_SLOT_DEPTH overrides; CPV_SMALL_PX sets the largest in-tile box one
-    // thread rasterises (default 32).
+    // CPV_SLOT_DEPTH overrides; CPV_SMALL_PX sets the largest in-tile box
+    // listed by a warp's spread tests (default 64).
     {
         int depth = mc.depth ? static_cast<int>(mc.depth) : (mc.samples ? 16 : 24);
         if (const char* v = std::getenv("CPV_SLOT_DEPTH")) depth = std::atoi(v);

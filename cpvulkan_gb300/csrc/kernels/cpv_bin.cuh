@@ -1,6 +1,6 @@
 /*
  * cpv_bin.cuh — order-preserving sort-middle binning and the other generic
- * device kernels (scan, fills).
+ * device kernels (the batched sort, blits, fills, copies).
  *
  * The per-draw binning builds, for every bin (a square of screen tiles, at
  * most CPV_MAX_BINS on the target), the list of primitive ids that touch it,
