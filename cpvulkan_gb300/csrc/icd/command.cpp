@@ -489,10 +489,10 @@ VkResult read_buffer(Queue* q, const Buffer* b, uint64_t offset, uint64_t size, 
     if (!b || !b->memory || offset + size > b->size) return VK_ERROR_DEVICE_LOST;
     DeviceMemory* m = b->memory;
     const uint64_t at = b->offset + offset;
-    const bool device_newer = !m->host || !m->dirty.empty() ||
-                              std::find_if(written.begin(), written.end(), [m](const WrittenRange& w) { return w.memory == m; }) != written.end();
-    if (device_newer) reads(q->device, b, &written);
-    if (!device_newer) {
+    const bool newer = !m->host || device_newer(q->device, m) ||
+                       std::find_if(written.begin(), written.end(), [m](const WrittenRange& w) { return w.memory == m; }) != written.end();
+    if (newer) reads(q->device, b, &written);
+    if (!newer) {
         std::memcpy(out, m->host + at, size);
     } else if (cudaStreamSynchronize(q->stream) != cudaSuccess || cudaMemcpy(out, m->device + at, size, cudaMemcpyDeviceToHost) != cudaSuccess) {
         cudaGetLastError();

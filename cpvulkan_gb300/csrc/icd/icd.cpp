@@ -452,29 +452,42 @@ bool copy_dirty(DeviceMemory* m) {
     return true;
 }
 
-// Completion of a submission: what it wrote in host-visible memories and did
-// not copy back itself is dirty there, or copied now where the memory is
-// mapped (coherent memory semantics). Under dev->memory_mutex.
-void complete_readback(std::vector<WrittenRange>& ranges) {
-    for (const WrittenRange& w : ranges) {
-        if (w.copied) continue;
+// The host has seen submissions 1 .. `last` of a queue finish: what they wrote
+// in host-visible memories and did not copy back themselves is dirty there,
+// or copied now where the memory is mapped (coherent memory semantics). Under
+// dev->memory_mutex.
+void retire(Queue* q, uint64_t last) {
+    auto& pending = q->pending_readback;
+    size_t kept = 0;
+    for (const WrittenRange& w : pending) {
+        if (w.submission > last) {
+            pending[kept++] = w;
+            continue;
+        }
         add_dirty(w.memory, w.lo, w.hi);
         if (w.memory->mapped) copy_dirty(w.memory);
     }
-    ranges.clear();
+    pending.resize(kept);
 }
 
-// Waits for all queues and brings a memory's mirror up to date, whatever
-// fences have been looked at. Under dev->memory_mutex.
-bool settle(Device* dev, DeviceMemory* m, const std::vector<WrittenRange>* written = nullptr) {
-    sync_queues(dev);
-    if (written)
-        for (const WrittenRange& w : *written)
-            if (w.memory == m) add_dirty(m, w.lo, w.hi);
-    for (Queue* q : dev->queues)
+// Whether unfinished work may write `m` without copying it back.
+bool has_pending(const Device* dev, const DeviceMemory* m) {
+    for (const Queue* q : dev->queues)
         for (const WrittenRange& w : q->pending_readback)
-            if (w.memory == m && !w.copied) add_dirty(m, w.lo, w.hi);
-    return copy_dirty(m);
+            if (w.memory == m) return true;
+    return false;
+}
+
+// Waits for all queues and retires what they had been given, whatever fences
+// have been looked at. Under dev->memory_mutex; with `lock` (which holds it)
+// it is released during the wait.
+void settle(Device* dev, std::unique_lock<std::mutex>* lock = nullptr) {
+    std::vector<uint64_t> last;
+    for (const Queue* q : dev->queues) last.push_back(q->submissions);
+    if (lock) lock->unlock();
+    sync_queues(dev);
+    if (lock) lock->lock();
+    for (size_t i = 0; i < last.size(); i++) retire(dev->queues[i], last[i]);
 }
 
 // Copies a memory's mirror to HBM and waits for it: by the SMs over the
@@ -486,46 +499,55 @@ void upload(Device* dev, DeviceMemory* m) {
     cudaStreamSynchronize(s);
 }
 
-void require_upload_locked(Device* dev, DeviceMemory* m, const std::vector<WrittenRange>* written) {
+}  // namespace
+
+void require_upload(Device* dev, DeviceMemory* m, const std::vector<WrittenRange>* written) {
+    std::lock_guard<std::mutex> lock(dev->memory_mutex);
     if (m->device_reads) return;
     m->device_reads = true;
     if (dev->compile_only || !m->host) return;
     if (m->host_newer || m->mapped) {
-        settle(dev, m, written);  // the mirror holds every byte: host writes and device writes
+        settle(dev);
+        if (written)
+            for (const WrittenRange& w : *written)
+                if (w.memory == m) add_dirty(m, w.lo, w.hi);
+        copy_dirty(m);  // the mirror holds every byte: host writes and device writes
         upload(dev, m);
     }
     m->host_newer = false;
 }
 
-}  // namespace
-
-void require_upload(Device* dev, DeviceMemory* m, const std::vector<WrittenRange>* written) {
+bool device_newer(Device* dev, const DeviceMemory* m) {
     std::lock_guard<std::mutex> lock(dev->memory_mutex);
-    require_upload_locked(dev, m, written);
+    return !m->dirty.empty() || has_pending(dev, m);
 }
 
 namespace {
+
+// Waits for a queue, and for what its submissions up to now have written to
+// be readable.
+VkResult wait_queue(Queue* q) {
+    std::lock_guard<std::mutex> queue_lock(q->mutex);
+    std::unique_lock<std::mutex> lock(q->device->memory_mutex);
+    const uint64_t last = q->submissions;
+    lock.unlock();
+    if (cudaStreamSynchronize(q->stream) != cudaSuccess) return VK_ERROR_DEVICE_LOST;
+    lock.lock();
+    retire(q, last);
+    return VK_SUCCESS;
+}
 
 VKAPI_ATTR VkResult VKAPI_CALL DeviceWaitIdle(VkDevice device) {
     auto* dev = reinterpret_cast<Device*>(device);
     if (dev->compile_only) return VK_SUCCESS;
     for (Queue* q : dev->queues) {
-        std::lock_guard<std::mutex> lock(q->mutex);
-        if (cudaStreamSynchronize(q->stream) != cudaSuccess) return VK_ERROR_DEVICE_LOST;
-        std::lock_guard<std::mutex> memory_lock(dev->memory_mutex);
-        complete_readback(q->pending_readback);
+        const VkResult r = wait_queue(q);
+        if (r != VK_SUCCESS) return r;
     }
     return VK_SUCCESS;
 }
 
-VKAPI_ATTR VkResult VKAPI_CALL QueueWaitIdle(VkQueue queue) {
-    auto* q = reinterpret_cast<Queue*>(queue);
-    std::lock_guard<std::mutex> lock(q->mutex);
-    if (cudaStreamSynchronize(q->stream) != cudaSuccess) return VK_ERROR_DEVICE_LOST;
-    std::lock_guard<std::mutex> memory_lock(q->device->memory_mutex);
-    complete_readback(q->pending_readback);
-    return VK_SUCCESS;
-}
+VKAPI_ATTR VkResult VKAPI_CALL QueueWaitIdle(VkQueue queue) { return wait_queue(reinterpret_cast<Queue*>(queue)); }
 
 // ------------------------------------------------------------------ memory --
 
@@ -600,15 +622,24 @@ VKAPI_ATTR VkResult VKAPI_CALL MapMemory(VkDevice device, VkDeviceMemory memory,
         *data = m->host + offset;
         return VK_SUCCESS;
     }
-    std::vector<std::pair<uint64_t, uint64_t>> dirty;
-    {
-        std::lock_guard<std::mutex> lock(dev->memory_mutex);
+    // What the device has written, whatever fences have been looked at: a
+    // range still pending here belongs to a submission that no observed fence
+    // covers, or whose later writer of the same bytes none covers.
+    std::unique_lock<std::mutex> lock(dev->memory_mutex);
+    if (has_pending(dev, m)) settle(dev, &lock);
+    while (!m->dirty.empty()) {
+        std::vector<std::pair<uint64_t, uint64_t>> dirty;
         dirty.swap(m->dirty);
+        lock.unlock();
+        bool ok = true;
+        for (const auto& d : dirty)
+            ok = ok && cudaMemcpy(m->host + d.first, m->device + d.first, d.second - d.first, cudaMemcpyDeviceToHost) == cudaSuccess;
+        lock.lock();
+        if (!ok) {
+            for (const auto& d : dirty) add_dirty(m, d.first, d.second);
+            return VK_ERROR_MEMORY_MAP_FAILED;
+        }
     }
-    if (!dirty.empty()) sync_queues(dev);
-    for (const auto& d : dirty)
-        if (cudaMemcpy(m->host + d.first, m->device + d.first, d.second - d.first, cudaMemcpyDeviceToHost) != cudaSuccess) return VK_ERROR_MEMORY_MAP_FAILED;
-    std::lock_guard<std::mutex> lock(dev->memory_mutex);
     m->mapped = true;
     m->reads_back = true;
     *data = m->host + offset;
@@ -623,16 +654,16 @@ VKAPI_ATTR void VKAPI_CALL UnmapMemory(VkDevice device, VkDeviceMemory memory) {
         m->mapped = false;
         return;
     }
-    {
-        std::lock_guard<std::mutex> lock(dev->memory_mutex);
-        if (!m->device_reads) {
-            m->mapped = false;
-            m->host_newer = true;
-            return;
-        }
+    std::unique_lock<std::mutex> lock(dev->memory_mutex);
+    if (!m->device_reads) {
+        m->mapped = false;
+        m->host_newer = true;
+        return;
     }
-    // The host's writes reach HBM before the call returns.
-    sync_queues(dev);
+    // The host's writes reach HBM before the call returns, and the mirror has
+    // what the device wrote before it is copied there.
+    settle(dev, &lock);
+    lock.unlock();
     upload(dev, m);
     m->mapped = false;
 }
@@ -661,8 +692,10 @@ VKAPI_ATTR VkResult VKAPI_CALL InvalidateMappedMemoryRanges(VkDevice device, uin
         auto* m = reinterpret_cast<DeviceMemory*>(r[i].memory);
         if (!m->host) continue;
         // what the device has written; the mirror's other bytes are current
+        if (dev->compile_only) continue;
         std::lock_guard<std::mutex> lock(dev->memory_mutex);
-        if (!dev->compile_only && !settle(dev, m)) return VK_ERROR_OUT_OF_DEVICE_MEMORY;
+        settle(dev);
+        if (!copy_dirty(m)) return VK_ERROR_OUT_OF_DEVICE_MEMORY;
     }
     return VK_SUCCESS;
 }
@@ -1304,8 +1337,8 @@ VKAPI_ATTR VkResult VKAPI_CALL ResetFences(VkDevice, uint32_t n, const VkFence* 
     return VK_SUCCESS;
 }
 
-// Queries a fence without blocking; on completion runs the coherence
-// readback of its submission.
+// Queries a fence without blocking; on completion what its submission and
+// those before it on the queue wrote becomes readable.
 VkResult poll_fence(Device* dev, Fence* f) {
     if (f->signalled) return VK_SUCCESS;
     if (!f->pending) return VK_NOT_READY;
@@ -1317,13 +1350,7 @@ VkResult poll_fence(Device* dev, Fence* f) {
     }
     {
         std::lock_guard<std::mutex> lock(dev->memory_mutex);
-        for (const WrittenRange& w : f->readback) {
-            if (w.copied || !f->queue) continue;
-            auto& pr = f->queue->pending_readback;
-            const auto it = std::find(pr.begin(), pr.end(), w);
-            if (it != pr.end() && --it->submissions == 0) pr.erase(it);
-        }
-        complete_readback(f->readback);
+        retire(f->queue, f->submission);
     }
     f->pending = false;
     f->signalled = true;
@@ -1413,17 +1440,25 @@ VkResult submit(VkQueue queue, uint32_t n, const VkSubmitInfo* si, VkFence fence
             s->signalled = true;
         }
     }
-    std::vector<WrittenRange> host_visible;
-    for (const WrittenRange& w : written)
-        if (w.memory->host && std::find(host_visible.begin(), host_visible.end(), w) == host_visible.end()) host_visible.push_back(w);
-    if (!host_visible.empty()) {
+    uint64_t number;
+    {
+        std::vector<WrittenRange> host_visible;
+        for (const WrittenRange& w : written)
+            if (w.memory->host && std::find(host_visible.begin(), host_visible.end(), w) == host_visible.end()) host_visible.push_back(w);
         // A memory whose host reads what the device writes is copied back in
         // the submission, before its fence; others when they are mapped.
         std::lock_guard<std::mutex> lock(dev->memory_mutex);
-        for (WrittenRange& w : host_visible)
-            w.copied = (w.memory->mapped || w.memory->reads_back) &&
-                       cudaMemcpyAsync(w.memory->host + w.lo, w.memory->device + w.lo, w.hi - w.lo, cudaMemcpyDeviceToHost, q->stream) == cudaSuccess;
-        for (WrittenRange& w : host_visible) w.memory->reads_back = false;
+        number = ++q->submissions;
+        for (WrittenRange& w : host_visible) {
+            w.submission = number;
+            if ((w.memory->mapped || w.memory->reads_back) &&
+                cudaMemcpyAsync(w.memory->host + w.lo, w.memory->device + w.lo, w.hi - w.lo, cudaMemcpyDeviceToHost, q->stream) == cudaSuccess)
+                continue;
+            const auto it = std::find(q->pending_readback.begin(), q->pending_readback.end(), w);
+            if (it != q->pending_readback.end()) it->submission = number;
+            else q->pending_readback.push_back(w);
+        }
+        for (const WrittenRange& w : host_visible) w.memory->reads_back = false;
     }
     if (fence) {
         auto* f = reinterpret_cast<Fence*>(fence);
@@ -1431,16 +1466,7 @@ VkResult submit(VkQueue queue, uint32_t n, const VkSubmitInfo* si, VkFence fence
         f->pending = true;
         f->signalled = false;
         f->queue = q;
-        f->readback = host_visible;
-    }
-    if (!host_visible.empty()) {
-        std::lock_guard<std::mutex> lock(dev->memory_mutex);
-        for (const WrittenRange& w : host_visible) {
-            if (w.copied) continue;
-            const auto it = std::find(q->pending_readback.begin(), q->pending_readback.end(), w);
-            if (it != q->pending_readback.end()) it->submissions++;
-            else q->pending_readback.push_back(w);
-        }
+        f->submission = number;
     }
     if (cudaGetLastError() != cudaSuccess) return VK_ERROR_DEVICE_LOST;
     return VK_SUCCESS;

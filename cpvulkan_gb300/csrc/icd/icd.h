@@ -50,8 +50,8 @@ struct DeviceMemory {
     VkDeviceSize size = 0;
     uint32_t type = 0;
     bool mapped = false;
-    // Byte ranges in which HBM is newer than the mirror: what finished
-    // submissions wrote and the mirror has not received.
+    // Byte ranges in which HBM is newer than the mirror: what submissions
+    // that the host has seen finish wrote and the mirror has not received.
     std::vector<std::pair<uint64_t, uint64_t>> dirty;
     // Mapped since its last copy back within a submission: its host reads
     // what the device writes, so the next submission copies it back itself.
@@ -64,13 +64,11 @@ struct DeviceMemory {
     bool host_newer = false;
 };
 
-// Bytes [lo, hi) of a memory that a submission writes; copied: the
-// submission also copies them to the mirror.
+// Bytes [lo, hi) of a memory that a submission writes.
 struct WrittenRange {
     DeviceMemory* memory = nullptr;
     uint64_t lo = 0, hi = 0;
-    bool copied = false;
-    uint32_t submissions = 1;  // in a queue's list: how many unfinished submissions write it
+    uint64_t submission = 0;  // in a queue's list: the last of the queue's submissions that writes it
     bool operator==(const WrittenRange& o) const { return memory == o.memory && lo == o.lo && hi == o.hi; }
 };
 
@@ -297,8 +295,8 @@ struct Fence {
     cudaEvent_t event = nullptr;
     bool signalled = false;   // created signalled or completed and observed
     bool pending = false;     // a submission will record the event
-    Queue* queue = nullptr;  // of the pending submission
-    std::vector<WrittenRange> readback;  // what the submission wrote in host-visible memories
+    Queue* queue = nullptr;   // of the pending submission
+    uint64_t submission = 0;  // its number there: the fence covers it and all before it
 };
 
 struct Semaphore {
@@ -311,7 +309,11 @@ struct Queue : Dispatchable {
     cudaStream_t stream = nullptr;
     cudaEvent_t timing[16] = {};
     rt::Scratch scratch;
-    std::vector<WrittenRange> pending_readback;  // under the device's memory_mutex
+    // Under the device's memory_mutex: the number of submissions, and what
+    // they write in host-visible memories without copying it back, until the
+    // host sees them finish (the only list that a range is in until then).
+    uint64_t submissions = 0;
+    std::vector<WrittenRange> pending_readback;
     std::mutex mutex;
 };
 
@@ -356,6 +358,8 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<WrittenRange>& written
 // at unmap and submission, and what is newer there is copied now.
 // `written`: what the submission being enqueued writes before that.
 void require_upload(Device* dev, DeviceMemory* m, const std::vector<WrittenRange>* written = nullptr);
+// Whether earlier submissions wrote bytes of `m` that its mirror has not received.
+bool device_newer(Device* dev, const DeviceMemory* m);
 // At vkEndCommandBuffer: compiles (NVRTC) and caches the batched module of
 // every render pass that will run batched, so its first submission does not.
 void precompile_batches(CommandBuffer* cb);
