@@ -387,6 +387,7 @@ VKAPI_ATTR VkResult VKAPI_CALL CreateDevice(VkPhysicalDevice pd, const VkDeviceC
     for (uint32_t i = 0; i < queues; i++) {
         auto* q = new Queue();
         q->device = dev;
+        q->index = i;
         dev->queues.push_back(q);
         if (!dev->compile_only && cudaStreamCreateWithFlags(&q->stream, cudaStreamNonBlocking) != cudaSuccess) {
             cudaGetLastError();
@@ -452,22 +453,24 @@ bool copy_dirty(DeviceMemory* m) {
     return true;
 }
 
-// The host has seen submissions 1 .. `last` of a queue finish: what they wrote
-// in host-visible memories and did not copy back themselves is dirty there,
-// or copied now where the memory is mapped (coherent memory semantics). Under
+// The host has seen `done` finish: what those submissions wrote in host-visible
+// memories and did not copy back themselves is dirty there, or copied now
+// where the memory is mapped (coherent memory semantics). Under
 // dev->memory_mutex.
-void retire(Queue* q, uint64_t last) {
-    auto& pending = q->pending_readback;
-    size_t kept = 0;
-    for (const WrittenRange& w : pending) {
-        if (w.submission > last) {
-            pending[kept++] = w;
-            continue;
+void retire(Device* dev, const Progress& done) {
+    for (Queue* q : dev->queues) {
+        auto& pending = q->pending_readback;
+        size_t kept = 0;
+        for (const WrittenRange& w : pending) {
+            if (w.submission > done[q->index]) {
+                pending[kept++] = w;
+                continue;
+            }
+            add_dirty(w.memory, w.lo, w.hi);
+            if (w.memory->mapped) copy_dirty(w.memory);
         }
-        add_dirty(w.memory, w.lo, w.hi);
-        if (w.memory->mapped) copy_dirty(w.memory);
+        pending.resize(kept);
     }
-    pending.resize(kept);
 }
 
 // Whether unfinished work may write `m` without copying it back.
@@ -482,12 +485,12 @@ bool has_pending(const Device* dev, const DeviceMemory* m) {
 // have been looked at. Under dev->memory_mutex; with `lock` (which holds it)
 // it is released during the wait.
 void settle(Device* dev, std::unique_lock<std::mutex>* lock = nullptr) {
-    std::vector<uint64_t> last;
-    for (const Queue* q : dev->queues) last.push_back(q->submissions);
+    Progress given{};
+    for (const Queue* q : dev->queues) given[q->index] = q->covers[q->index];
     if (lock) lock->unlock();
     sync_queues(dev);
     if (lock) lock->lock();
-    for (size_t i = 0; i < last.size(); i++) retire(dev->queues[i], last[i]);
+    retire(dev, given);
 }
 
 // Copies a memory's mirror to HBM and waits for it: by the SMs over the
@@ -529,11 +532,11 @@ namespace {
 VkResult wait_queue(Queue* q) {
     std::lock_guard<std::mutex> queue_lock(q->mutex);
     std::unique_lock<std::mutex> lock(q->device->memory_mutex);
-    const uint64_t last = q->submissions;
+    const Progress covers = q->covers;
     lock.unlock();
     if (cudaStreamSynchronize(q->stream) != cudaSuccess) return VK_ERROR_DEVICE_LOST;
     lock.lock();
-    retire(q, last);
+    retire(q->device, covers);
     return VK_SUCCESS;
 }
 
@@ -1337,8 +1340,8 @@ VKAPI_ATTR VkResult VKAPI_CALL ResetFences(VkDevice, uint32_t n, const VkFence* 
     return VK_SUCCESS;
 }
 
-// Queries a fence without blocking; on completion what its submission and
-// those before it on the queue wrote becomes readable.
+// Queries a fence without blocking; on completion what its submission, those
+// before it on the queue and those they waited for wrote becomes readable.
 VkResult poll_fence(Device* dev, Fence* f) {
     if (f->signalled) return VK_SUCCESS;
     if (!f->pending) return VK_NOT_READY;
@@ -1350,7 +1353,7 @@ VkResult poll_fence(Device* dev, Fence* f) {
     }
     {
         std::lock_guard<std::mutex> lock(dev->memory_mutex);
-        retire(f->queue, f->submission);
+        retire(dev, f->covers);
     }
     f->pending = false;
     f->signalled = true;
@@ -1406,6 +1409,28 @@ VKAPI_ATTR void VKAPI_CALL DestroySemaphore(VkDevice, VkSemaphore sem, const VkA
     host_delete(s, alloc);
 }
 
+// Ends a batch of a submission that writes `written[from ..]`: numbers it and
+// sees to its host-visible ranges. Those of a memory whose host reads what the
+// device writes are copied back here, before the batch's semaphores and the
+// fence; others when they are mapped.
+void finish_batch(Queue* q, const std::vector<WrittenRange>& written, size_t from) {
+    std::lock_guard<std::mutex> lock(q->device->memory_mutex);
+    const uint64_t number = ++q->covers[q->index];
+    for (size_t i = from; i < written.size(); i++) {
+        WrittenRange w = written[i];
+        if (!w.memory->host || std::find(written.begin() + static_cast<std::ptrdiff_t>(from), written.begin() + static_cast<std::ptrdiff_t>(i), w) !=
+                                   written.begin() + static_cast<std::ptrdiff_t>(i))
+            continue;
+        if ((w.memory->mapped || w.memory->reads_back) &&
+            cudaMemcpyAsync(w.memory->host + w.lo, w.memory->device + w.lo, w.hi - w.lo, cudaMemcpyDeviceToHost, q->stream) == cudaSuccess)
+            continue;
+        w.submission = number;
+        const auto it = std::find(q->pending_readback.begin(), q->pending_readback.end(), w);
+        if (it != q->pending_readback.end()) it->submission = number;
+        else q->pending_readback.push_back(w);
+    }
+}
+
 // vkQueueSubmit (CPVulkan/Queue.cpp:11-77): waits, replays each command
 // buffer onto the queue's stream, signals semaphores and the fence. Returns
 // once the work is enqueued. no_alloc selects the fixed binning scratch.
@@ -1427,46 +1452,37 @@ VkResult submit(VkQueue queue, uint32_t n, const VkSubmitInfo* si, VkFence fence
     for (uint32_t i = 0; i < n; i++) {
         for (uint32_t k = 0; k < si[i].waitSemaphoreCount; k++) {
             auto* s = reinterpret_cast<Semaphore*>(si[i].pWaitSemaphores[k]);
-            if (s->signalled) cudaStreamWaitEvent(q->stream, s->event, 0);
+            std::lock_guard<std::mutex> lock(dev->memory_mutex);
+            if (s->signalled && cudaStreamWaitEvent(q->stream, s->event, 0) == cudaSuccess)
+                for (size_t j = 0; j < kMaxQueues; j++) q->covers[j] = std::max(q->covers[j], s->covers[j]);
             s->signalled = false;
         }
+        const size_t from = written.size();
         for (uint32_t k = 0; k < si[i].commandBufferCount; k++) {
             const VkResult r = run_command_buffer(q, reinterpret_cast<CommandBuffer*>(si[i].pCommandBuffers[k]), written, no_alloc);
             if (r != VK_SUCCESS) return r;
         }
+        finish_batch(q, written, from);
         for (uint32_t k = 0; k < si[i].signalSemaphoreCount; k++) {
             auto* s = reinterpret_cast<Semaphore*>(si[i].pSignalSemaphores[k]);
             cudaEventRecord(s->event, q->stream);
+            std::lock_guard<std::mutex> lock(dev->memory_mutex);
+            s->covers = q->covers;
             s->signalled = true;
         }
     }
-    uint64_t number;
+    Progress covers;
     {
-        std::vector<WrittenRange> host_visible;
-        for (const WrittenRange& w : written)
-            if (w.memory->host && std::find(host_visible.begin(), host_visible.end(), w) == host_visible.end()) host_visible.push_back(w);
-        // A memory whose host reads what the device writes is copied back in
-        // the submission, before its fence; others when they are mapped.
         std::lock_guard<std::mutex> lock(dev->memory_mutex);
-        number = ++q->submissions;
-        for (WrittenRange& w : host_visible) {
-            w.submission = number;
-            if ((w.memory->mapped || w.memory->reads_back) &&
-                cudaMemcpyAsync(w.memory->host + w.lo, w.memory->device + w.lo, w.hi - w.lo, cudaMemcpyDeviceToHost, q->stream) == cudaSuccess)
-                continue;
-            const auto it = std::find(q->pending_readback.begin(), q->pending_readback.end(), w);
-            if (it != q->pending_readback.end()) it->submission = number;
-            else q->pending_readback.push_back(w);
-        }
-        for (const WrittenRange& w : host_visible) w.memory->reads_back = false;
+        for (const WrittenRange& w : written) w.memory->reads_back = false;
+        covers = q->covers;
     }
     if (fence) {
         auto* f = reinterpret_cast<Fence*>(fence);
         if (cudaEventRecord(f->event, q->stream) != cudaSuccess) return VK_ERROR_DEVICE_LOST;
         f->pending = true;
         f->signalled = false;
-        f->queue = q;
-        f->submission = number;
+        f->covers = covers;
     }
     if (cudaGetLastError() != cudaSuccess) return VK_ERROR_DEVICE_LOST;
     return VK_SUCCESS;

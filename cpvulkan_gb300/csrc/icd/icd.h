@@ -291,17 +291,24 @@ struct CommandPool {
     std::set<CommandBuffer*> buffers;
 };
 
+// Queues a device may create in its one queue family.
+constexpr uint32_t kMaxQueues = 16;
+
+// What has finished when something has: per queue, the number of its last
+// submission (each batch of a vkQueueSubmit counts as one).
+using Progress = std::array<uint64_t, kMaxQueues>;
+
 struct Fence {
     cudaEvent_t event = nullptr;
     bool signalled = false;   // created signalled or completed and observed
     bool pending = false;     // a submission will record the event
-    Queue* queue = nullptr;   // of the pending submission
-    uint64_t submission = 0;  // its number there: the fence covers it and all before it
+    Progress covers{};        // the pending submission, all before it and all they waited for
 };
 
 struct Semaphore {
     cudaEvent_t event = nullptr;
     bool signalled = false;
+    Progress covers{};  // of its last signal
 };
 
 struct Queue : Dispatchable {
@@ -309,16 +316,16 @@ struct Queue : Dispatchable {
     cudaStream_t stream = nullptr;
     cudaEvent_t timing[16] = {};
     rt::Scratch scratch;
-    // Under the device's memory_mutex: the number of submissions, and what
-    // they write in host-visible memories without copying it back, until the
-    // host sees them finish (the only list that a range is in until then).
-    uint64_t submissions = 0;
+    uint32_t index = 0;  // among the device's queues
+    // Under the device's memory_mutex: what has finished when the queue's
+    // work has (its own submissions and, through semaphores, other queues'),
+    // and what its submissions write in host-visible memories without copying
+    // it back, until the host sees them finish (the only list that a range is
+    // in until then).
+    Progress covers{};
     std::vector<WrittenRange> pending_readback;
     std::mutex mutex;
 };
-
-// Queues a device may create in its one queue family.
-constexpr uint32_t kMaxQueues = 16;
 
 struct Device : Dispatchable {
     PhysicalDevice* physical = nullptr;

@@ -1,6 +1,6 @@
-"""A fence covers its submission and every earlier one on the queue: what they
-wrote in host-visible memory is there for the host once the fence has been
-waited for, whatever fences the earlier ones had and whether those were ever
+"""A fence covers its submission, every earlier one on the queue and those that
+these waited for through semaphores: what they wrote in host-visible memory is
+there for the host once the fence has been waited for, whatever fences the earlier ones had and whether those were ever
 looked at, and a fence that is looked at late takes nothing back from the
 host. Bytes against one array per memory."""
 import ctypes
@@ -8,7 +8,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from tests.test_gpu_host_memory import DST, SIZE, SRC, BeginInfo, CommandInfo, FenceInfo, SubmitInfo, Vulkan, struct, u32, u64, vp
+from tests.test_gpu_host_memory import DST, SIZE, SRC, BeginInfo, BufferInfo, CommandInfo, FenceInfo, MemoryInfo, SubmitInfo, Vulkan, struct, u32, u64, vp
 
 pytestmark = pytest.mark.gpu
 
@@ -154,3 +154,41 @@ def test_random_submissions(native, seed, usage):
         for k in range(last):
             vk.reset(k)
         assert vk.check(memory, model), (step, "late")
+
+
+@pytest.mark.parametrize("mapped", ["never", "before", "all along"])
+@pytest.mark.parametrize("queues", [1, 2])
+def test_a_fence_covers_what_its_submission_waited_for(native, mapped, queues):
+    """Queue 0 writes without a fence and signals a semaphore; a submission of
+    queue 0 or 1 waits for it and has the fence. The range is large enough that
+    a copy back after the semaphore would still run when the fence is
+    signalled."""
+    vk = Submissions()
+    size = 64 << 20
+    b = vk.make("vkCreateBuffer", vp(vk.device), BufferInfo(12, None, 0, size, DST, 0, 0, None))
+    memory = vk.make("vkAllocateMemory", vp(vk.device), MemoryInfo(5, None, size, 0))
+    vk.call("vkBindBufferMemory", vp(vk.device), vp(b), vp(memory), u64(0))
+    semaphore = vk.make("vkCreateSemaphore", vp(vk.device), SemaphoreInfo(9))
+
+    def pointer():
+        p = vp()
+        vk.call("vkMapMemory", vp(vk.device), vp(memory), u64(0), u64(2 ** 64 - 1), u32(0), ctypes.byref(p))
+        return np.ctypeslib.as_array(ctypes.cast(p, ctypes.POINTER(ctypes.c_uint32)), (size // 4,))
+
+    if mapped != "never":
+        host = pointer()
+        host[:] = 5
+        if mapped == "before":
+            vk.unmap(memory)
+    first, second = vk.queues[0], vk.queues[queues - 1]
+    for value in (0x0A0A0A0A, 0x0B0B0B0B):
+        vk.send(0, first, lambda: vk.fill(b, 0, size, value), signals=[semaphore])
+        vk.send(1, second, lambda: None, fence=True, waits=[semaphore])
+        vk.wait(1)
+        if mapped != "all along":
+            host = pointer()
+        assert host[-1] == value  # the last to arrive
+        assert np.all(host == value)
+        if mapped != "all along":
+            vk.unmap(memory)
+        vk.reset(1)
