@@ -419,6 +419,9 @@ struct BinShape {
     uint32_t row_prims = 256, rows = 0;
 };
 
+// Primitives x tiles up to which a draw may be walked whole by every tile.
+uint64_t direct_limit() { return env_u32("CPV_DIRECT_LIMIT", 1u << 20); }
+
 // A draw of at most CPV_DIRECT_PRIMS primitives (and CPV_DIRECT_LIMIT
 // primitives x tiles) is walked whole by every tile: no launch but the
 // raster. One of at most CPV_FILTER_PRIMS is filtered by every tile from the
@@ -428,11 +431,11 @@ struct BinShape {
 // launches); 12000 triangles on 3600 tiles take 677 us filtered, 598 us
 // binned; the serving mix (1000 to 100000 triangles) 26.2 ms with the line
 // at 512 or 2048, 32.8 ms at 8192.
-BinShape bin_shape(uint64_t prims, uint32_t tiles_x, uint32_t tiles_y, uint64_t direct_limit) {
+BinShape bin_shape(uint64_t prims, uint32_t tiles_x, uint32_t tiles_y) {
     const uint32_t direct_prims = env_u32("CPV_DIRECT_PRIMS", 64u), filter_prims = env_u32("CPV_FILTER_PRIMS", 2048u);
     BinShape b;
     const uint64_t tiles = static_cast<uint64_t>(tiles_x) * tiles_y;
-    if (prims <= direct_prims && prims * tiles <= direct_limit) return b;
+    if (prims <= direct_prims && prims * tiles <= direct_limit()) return b;
     b.mode = BinShape::kFilter;
     b.rows = static_cast<uint32_t>((prims + 255u) / 256u);
     if (prims <= filter_prims) return b;
@@ -508,7 +511,7 @@ int draw_plain(cudaStream_t stream, const Module& m, CpvDrawParams P, Scratch& s
     if (r != kOk) return r;
     P.status = sc.words() + 2;
     if (G > 0xFFFFFFFFull) return kErrInvalid;
-    const BinShape b = bin_shape(G, P.tiles_x, P.tiles_y, env_u32("CPV_DIRECT_LIMIT", 1u << 20));
+    const BinShape b = bin_shape(G, P.tiles_x, P.tiles_y);
     if (b.mode != BinShape::kDirect) {
         if ((r = sc.reserve_rects(G)) != kOk) return r;
         if (b.mode == BinShape::kLists) {
@@ -1043,19 +1046,24 @@ uint8_t* g_static_addr[kMaxStaticDevices] = {};
 
 uint64_t align256(uint64_t b) { return (b + 255u) & ~255ull; }
 
-// Whether a draw of the fixed array is walked whole by every tile.
-// CPV_DIRECT_LIMIT is read once per process, so the pre-check and the draw
-// always take the same path.
-uint64_t static_direct_limit() {
-    static const uint32_t limit = env_u32("CPV_DIRECT_LIMIT", 1u << 18);
-    return limit;
-}
-
 // Bytes a draw may ask of the fixed array: 8 per primitive and 8 per tile
 // beside 8256 fixed ones. (The draw itself needs the rectangles only and
 // uses the rest as far as it goes; the limit is part of the entry point's
 // contract and stays with it.)
 uint64_t static_need(uint64_t prims, uint64_t tiles) { return 8256u + align256(prims * 8) + 2u * align256(tiles * 4); }
+
+// How a draw of the fixed array finds a tile's primitives; false when it is
+// refused. A draw whose rectangles do not fit is walked whole by every tile
+// where CPV_DIRECT_LIMIT allows that (it then needs nothing of the array).
+bool static_shape(uint64_t prims, uint32_t tiles_x, uint32_t tiles_y, BinShape& b) {
+    const uint64_t tiles = static_cast<uint64_t>(tiles_x) * tiles_y;
+    if (static_need(prims, tiles) <= CPV_STATIC_SCRATCH_BYTES) {
+        b = bin_shape(prims, tiles_x, tiles_y);
+        return true;
+    }
+    b = BinShape();
+    return prims * tiles <= direct_limit();
+}
 
 }  // namespace
 
@@ -1083,15 +1091,15 @@ int static_scratch_setup(std::string& error) {
 int static_scratch_check(uint64_t prims, uint32_t tile_shift, uint32_t width, uint32_t height, std::string& error) {
     if (prims == 0 || width == 0 || height == 0) return kOk;
     const uint64_t tile = 1ull << tile_shift;
-    const uint64_t tiles = ((width + tile - 1) / tile) * ((height + tile - 1) / tile);
+    const uint64_t tiles_x = (width + tile - 1) / tile, tiles_y = (height + tile - 1) / tile, tiles = tiles_x * tiles_y;
     if (prims > 0xFFFFFFFFull) {
         error = "draw of " + std::to_string(prims) + " primitives exceeds 2^32 - 1";
         return kErrInvalid;
     }
-    if (prims * tiles <= static_direct_limit()) return kOk;
-    const uint64_t need = static_need(prims, tiles);
-    if (need > CPV_STATIC_SCRATCH_BYTES) {
-        error = "draw of " + std::to_string(prims) + " primitives over " + std::to_string(tiles) + " tiles needs " + std::to_string(need) +
+    BinShape b;
+    if (!static_shape(prims, static_cast<uint32_t>(tiles_x), static_cast<uint32_t>(tiles_y), b)) {
+        error = "draw of " + std::to_string(prims) + " primitives over " + std::to_string(tiles) + " tiles needs " +
+                std::to_string(static_need(prims, tiles)) +
                 " bytes of binning scratch; the fixed scratch holds " + std::to_string(static_cast<uint64_t>(CPV_STATIC_SCRATCH_BYTES));
         return kErrOutOfMemory;
     }
@@ -1122,9 +1130,10 @@ int draw_plain_static(cudaStream_t stream, const Module& m, CpvDrawParams P) {
     }
     uint32_t* words = reinterpret_cast<uint32_t*>(base);
     P.status = words + 2;
-    BinShape b = bin_shape(G, P.tiles_x, P.tiles_y, static_direct_limit());
+    BinShape b;
+    if (!static_shape(G, P.tiles_x, P.tiles_y, b)) return kErrOutOfMemory;  // (as the check has)
     if (b.mode != BinShape::kDirect) {
-        // static_scratch_check has made sure that the rectangles fit
+        // the rectangles fit: any shape but the direct one is of a draw within static_need
         const uint64_t rects_at = align256(kWordsBytes), ranges_at = rects_at + align256(G * 8);
         const uint64_t counts_at = ranges_at + align256(static_cast<uint64_t>(b.bins) * 8);
         uint64_t lists_at = 0, entries = 0;

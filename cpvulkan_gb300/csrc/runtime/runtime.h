@@ -209,8 +209,10 @@ void batch_stats(uint64_t out[3]);
 // 32 MiB file-scope device array per device. A draw needs 8 bytes per
 // primitive for its tile rectangles; its bins take what is left, and a draw
 // whose bins do not fit filters the rectangles instead. One whose rectangles
-// do not fit is rejected (kErrOutOfMemory, message in last_error()). The array is shared by every queue of the process on that
-// device, so draw_plain_static calls whose work overlaps on the GPU race.
+// do not fit is rejected (kErrOutOfMemory, message in last_error()) unless
+// CPV_DIRECT_LIMIT lets every tile walk it whole. The array is shared by every
+// queue of the process on that device, so draw_plain_static calls whose work
+// overlaps on the GPU race.
 #define CPV_STATIC_SCRATCH_BYTES (32ull << 20)
 // Resolves the array's device address for the current device
 // (cudaGetSymbolAddress, once per device). Call outside any stream capture.
