@@ -103,6 +103,8 @@ def harness():
     h.cpvh_render.argtypes = [vp, u32, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_double)]
     h.cpvh_render_e2e.restype = ctypes.c_int
     h.cpvh_render_e2e.argtypes = [vp, u32, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(u64), ctypes.POINTER(u64)]
+    h.cpvh_renderer_upload.restype = ctypes.c_int
+    h.cpvh_renderer_upload.argtypes = [vp]
     h.cpvh_renderer_update.restype = ctypes.c_int
     h.cpvh_renderer_update.argtypes = [vp]
     h.cpvh_renderer_set_indirect.restype = ctypes.c_int
@@ -324,6 +326,12 @@ class Renderer:
         if r != VK_SUCCESS:
             raise RuntimeError("end-to-end render failed (%d)" % r)
         return total.value, h2d.value, d2h.value
+
+    def upload(self):
+        """Uploads the scene's vertex, index and uniform bytes again; the recorded frame stays."""
+        r = harness().cpvh_renderer_upload(self.ptr)
+        if r != VK_SUCCESS:
+            raise RuntimeError("upload failed (%d)" % r)
 
     def update(self):
         r = harness().cpvh_renderer_update(self.ptr)

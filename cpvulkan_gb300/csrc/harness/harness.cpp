@@ -1234,7 +1234,7 @@ extern "C" {
 
 void cpvh_renderer_destroy(cpvh_renderer* r) { renderer_destroy(r, true); }
 
-int cpvh_renderer_update(cpvh_renderer* r) {
+int cpvh_renderer_upload(cpvh_renderer* r) {
     cpvh_context* c = r->ctx;
     void* map = nullptr;
     if (c->f.vkMapMemory(c->device, r->staging.memory, 0, VK_WHOLE_SIZE, 0, &map) != VK_SUCCESS) return VK_ERROR_MEMORY_MAP_FAILED;
@@ -1245,7 +1245,11 @@ int cpvh_renderer_update(cpvh_renderer* r) {
     c->f.vkBeginCommandBuffer(r->copy_cmd, &bi);
     record_upload(r, r->copy_cmd);
     c->f.vkEndCommandBuffer(r->copy_cmd);
-    const VkResult res = submit_and_wait(r, r->copy_cmd);
+    return submit_and_wait(r, r->copy_cmd);
+}
+
+int cpvh_renderer_update(cpvh_renderer* r) {
+    const int res = cpvh_renderer_upload(r);
     record_all(r);
     return res;
 }

@@ -37,22 +37,33 @@
 
 #include "cpv_device.cuh"
 
+/* The words of a batch: its pairs, the raster's tile counter, the sort's
+ * chunks a CTA and its CTAs that have any, the two digits' totals. */
+#define CPV_WORD_PAIRS 0
+#define CPV_WORD_TILE 2
+#define CPV_WORD_CHUNKS 3
+#define CPV_WORD_DIGITS 4
+#define CPV_WORD_ROWS 8
+
 /* 2. counts[row][bin] → the list position of the row's first entry in the
  * bin; range[bin] = the bin's list. One CTA of 1024 threads per 8 bins: 128
  * groups of rows are summed, scanned over the groups and walked again. A
  * bin's list starts where an atomic on *total puts it (the lists' order in
  * memory does not matter); *total (zeroed by cpv_setup_rects) ends as the
- * draw's pair count. */
+ * draw's pair count. With `words` the columns are a sort digit's counts and
+ * the rows are those of CPV_WORD_ROWS. */
 #define CPV_BIN_SCAN_THREADS 1024
 #define CPV_BIN_SCAN_BINS 8
 extern "C" __global__ void __launch_bounds__(CPV_BIN_SCAN_THREADS) cpv_bin_scan(uint32_t* __restrict__ counts, uint32_t rows, uint32_t bins,
-                                                                               uint2* __restrict__ range, unsigned long long* __restrict__ total) {
+                                                                               uint2* __restrict__ range, unsigned long long* __restrict__ total,
+                                                                               const uint32_t* __restrict__ words) {
     __shared__ uint32_t warp_sums[CPV_BIN_SCAN_THREADS / 32][CPV_BIN_SCAN_BINS];
     __shared__ uint32_t list_base[CPV_BIN_SCAN_BINS];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t b = threadIdx.x % CPV_BIN_SCAN_BINS, group = threadIdx.x / CPV_BIN_SCAN_BINS;
     const uint32_t bin = blockIdx.x * CPV_BIN_SCAN_BINS + b;
     const uint32_t groups = CPV_BIN_SCAN_THREADS / CPV_BIN_SCAN_BINS;
+    if (words) rows = words[CPV_WORD_ROWS];
     const uint32_t per = (rows + groups - 1u) / groups;
     const uint32_t r0 = per * group < rows ? per * group : rows;
     const uint32_t r1 = bin < bins ? (r0 + per < rows ? r0 + per : rows) : r0;
@@ -221,8 +232,8 @@ extern "C" __global__ void __launch_bounds__(256) cpv_bin_write(const uint2* __r
 #define CPV_RADIX_ITEMS 8
 #define CPV_RADIX_CHUNK (CPV_RADIX_THREADS * CPV_RADIX_ITEMS)
 
-__device__ __forceinline__ uint32_t cpv_pairs_in_bounds(const uint32_t* pair_total, uint32_t capacity) {
-    const uint32_t p = *pair_total;
+__device__ __forceinline__ uint32_t cpv_pairs_in_bounds(const uint32_t* words, uint32_t capacity) {
+    const uint32_t p = words[CPV_WORD_PAIRS];
     return p <= capacity ? p : 0u;
 }
 
@@ -287,14 +298,20 @@ extern "C" __global__ void __launch_bounds__(CPV_SCAN_THREADS) cpv_batch_scan(co
  * the warp. Two dependent loads, then stores of 6 bytes a pair: latency-bound
  * (99 M primitives, 30 M pairs: 260 us; a CTA per block, a block-wide scan
  * and a division a pair took 500, every register of one fewer CTA an SM 272).
- * CTA 0 stores the pair total and clears the words of the kernels
- * that follow: words[2], the raster's tile counter, and words[4..7], the two
- * digits' totals. */
+ * CTA 0 stores the pair total, clears the words of the kernels that follow
+ * and shares the pairs out among the sort's CTAs: whole chunks, as few each as
+ * cover them, for the `sort_ctas` that are launched (four an SM); those
+ * without any leave at once. One digit's scatter with the pairs split evenly
+ * over all 608 CTAs, then in whole chunks: 14.6 us then 8.5 for 316k pairs and
+ * 1024 digits (155 CTAs; 12.2 at 78 of two chunks), 15.9 then 12.4 for 1.7 M
+ * pairs and 128 digits. By the pairs of each frame, since those of the plan's
+ * build may be none: geometry moves under a recorded command buffer. */
 #define CPV_EMIT_LANE_PAIRS 16u
 extern "C" __global__ void __launch_bounds__(256, 6) cpv_batch_emit(const uint2* __restrict__ rects, const uint32_t* __restrict__ block_pairs,
                                                                  const uint32_t* __restrict__ block_offsets, const uint32_t* __restrict__ chunk_sums,
                                                                  uint32_t blocks, uint32_t tiles_x, uint16_t* __restrict__ keys,
-                                                                 uint32_t* __restrict__ vals, uint32_t capacity, uint32_t* __restrict__ words) {
+                                                                 uint32_t* __restrict__ vals, uint32_t capacity, uint32_t* __restrict__ words,
+                                                                 uint32_t sort_ctas) {
     __shared__ uint32_t sums[2][8];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t block = blockIdx.x * 8u + warp;
@@ -320,7 +337,15 @@ extern "C" __global__ void __launch_bounds__(256, 6) cpv_batch_emit(const uint2*
         before += sums[0][w];
         total += sums[1][w];
     }
-    if (blockIdx.x == 0u && threadIdx.x < 8u && (threadIdx.x == 0u || threadIdx.x == 2u || threadIdx.x >= 4u)) words[threadIdx.x] = threadIdx.x ? 0u : total;
+    if (blockIdx.x == 0u && threadIdx.x == 0u) {
+        const uint32_t chunks_of_pairs = total <= capacity ? total / CPV_RADIX_CHUNK + (total % CPV_RADIX_CHUNK ? 1u : 0u) : 0u;
+        const uint32_t per = (chunks_of_pairs + sort_ctas - 1u) / sort_ctas;
+        words[CPV_WORD_PAIRS] = total;
+        words[CPV_WORD_TILE] = 0u;
+        words[CPV_WORD_CHUNKS] = per;
+        words[CPV_WORD_ROWS] = per ? (chunks_of_pairs + per - 1u) / per : 0u;
+        for (uint32_t i = 0; i < 4u; i++) words[CPV_WORD_DIGITS + i] = 0u;
+    }
     if (total > capacity || block_n == 0u) return;
     uint2 r[8];
     const uint32_t g0 = block * 256u + lane;
@@ -421,11 +446,11 @@ extern "C" __global__ void __launch_bounds__(256) cpv_index_range(const CpvDrawP
     }
 }
 
-/* Contiguous item range of CTA c of `ctas` over n items, starting at a
- * multiple of 8 (16 bytes of keys). */
-__device__ __forceinline__ void cpv_cta_range(uint32_t n, uint32_t c, uint32_t ctas, uint32_t& begin, uint32_t& end) {
-    const uint64_t per = ((n + ctas - 1u) / ctas + 7u) & ~7u;
-    const uint64_t b = per * c, e = b + per;
+/* The CTA's range of the pairs. */
+__device__ __forceinline__ void cpv_cta_range(const uint32_t* words, uint32_t capacity, uint32_t& begin, uint32_t& end) {
+    const uint32_t n = cpv_pairs_in_bounds(words, capacity);
+    const uint64_t per = static_cast<uint64_t>(words[CPV_WORD_CHUNKS]) * CPV_RADIX_CHUNK;
+    const uint64_t b = per * blockIdx.x, e = b + per;
     begin = static_cast<uint32_t>(b < n ? b : n);
     end = static_cast<uint32_t>(e < n ? e : n);
 }
@@ -433,16 +458,17 @@ __device__ __forceinline__ void cpv_cta_range(uint32_t n, uint32_t c, uint32_t c
 /* counts[cta * digits + digit] = items of the CTA's range with that digit.
  * With tile_range (the first of two digits) it is also cleared here, for
  * cpv_tile_ranges to fill. */
-extern "C" __global__ void __launch_bounds__(CPV_RADIX_THREADS) cpv_radix_hist(const uint16_t* __restrict__ keys, const uint32_t* __restrict__ pair_total,
+extern "C" __global__ void __launch_bounds__(CPV_RADIX_THREADS) cpv_radix_hist(const uint16_t* __restrict__ keys, const uint32_t* __restrict__ words,
                                                                                uint32_t capacity, uint32_t shift, uint32_t digits,
                                                                                uint32_t* __restrict__ counts, uint2* __restrict__ tile_range, uint32_t tiles) {
     __shared__ uint32_t count[CPV_RADIX_DIGITS];
-    for (uint32_t d = threadIdx.x; d < digits; d += CPV_RADIX_THREADS) count[d] = 0u;
     if (tile_range)
         for (uint32_t i = blockIdx.x * CPV_RADIX_THREADS + threadIdx.x; i < tiles; i += gridDim.x * CPV_RADIX_THREADS) tile_range[i] = make_uint2(0u, 0u);
-    __syncthreads();
     uint32_t begin, end;
-    cpv_cta_range(cpv_pairs_in_bounds(pair_total, capacity), blockIdx.x, gridDim.x, begin, end);
+    cpv_cta_range(words, capacity, begin, end);
+    if (begin >= end) return;  /* not one of the rows */
+    for (uint32_t d = threadIdx.x; d < digits; d += CPV_RADIX_THREADS) count[d] = 0u;
+    __syncthreads();
     for (uint32_t i = begin + 8u * threadIdx.x; i < end; i += 8u * CPV_RADIX_THREADS) {
         /* the buffer is a multiple of 8 keys long */
         const uint4 v = *reinterpret_cast<const uint4*>(keys + i);
@@ -467,7 +493,7 @@ extern "C" __global__ void __launch_bounds__(CPV_RADIX_THREADS) cpv_radix_hist(c
  * 32-bit keys; ballots per bit instead of the match 328). */
 extern "C" __global__ void __launch_bounds__(CPV_RADIX_THREADS) cpv_radix_scatter(const uint16_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                                                                                   uint16_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-                                                                                  const uint32_t* __restrict__ pair_total, uint32_t capacity, uint32_t shift,
+                                                                                  const uint32_t* __restrict__ words, uint32_t capacity, uint32_t shift,
                                                                                   uint32_t digits, const uint32_t* __restrict__ offsets) {
     __shared__ uint32_t next[CPV_RADIX_DIGITS];   /* the digit's next position */
     __shared__ uint32_t place[CPV_RADIX_DIGITS];  /* that, less the digit's first position in the chunk */
@@ -479,7 +505,7 @@ extern "C" __global__ void __launch_bounds__(CPV_RADIX_THREADS) cpv_radix_scatte
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t per_thread = (digits + CPV_RADIX_THREADS - 1u) / CPV_RADIX_THREADS, d0 = threadIdx.x * per_thread;
     uint32_t begin, end;
-    cpv_cta_range(cpv_pairs_in_bounds(pair_total, capacity), blockIdx.x, gridDim.x, begin, end);
+    cpv_cta_range(words, capacity, begin, end);
     if (begin >= end) return;
     for (uint32_t d = threadIdx.x; d < digits; d += CPV_RADIX_THREADS) {
         next[d] = offsets[blockIdx.x * digits + d];
@@ -563,9 +589,9 @@ extern "C" __global__ void __launch_bounds__(CPV_RADIX_THREADS) cpv_radix_scatte
 }
 
 /* tile_range (zeroed beforehand) from the sorted keys, eight a thread. */
-extern "C" __global__ void __launch_bounds__(256) cpv_tile_ranges(const uint16_t* __restrict__ keys, const uint32_t* __restrict__ pair_total,
+extern "C" __global__ void __launch_bounds__(256) cpv_tile_ranges(const uint16_t* __restrict__ keys, const uint32_t* __restrict__ words,
                                                                   uint32_t capacity, uint2* __restrict__ tile_range) {
-    const uint32_t n = cpv_pairs_in_bounds(pair_total, capacity);
+    const uint32_t n = cpv_pairs_in_bounds(words, capacity);
     for (uint64_t at = 8ull * (blockIdx.x * 256u + threadIdx.x); at < n; at += 8ull * 256u * gridDim.x) {
         const uint32_t i = static_cast<uint32_t>(at);
         const uint4 v = *reinterpret_cast<const uint4*>(keys + i);

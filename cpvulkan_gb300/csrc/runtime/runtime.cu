@@ -467,7 +467,7 @@ int bin_draw(cudaStream_t stream, const Module& m, const BinShape& b, CpvDrawPar
     if (b.mode != BinShape::kLists) return kOk;
     profile_begin(stream, "cpv_bin_scan");
     cpv_bin_scan<<<(b.bins + CPV_BIN_SCAN_BINS - 1u) / CPV_BIN_SCAN_BINS, CPV_BIN_SCAN_THREADS, 0, stream>>>(
-        P.bin_counts, b.rows, b.bins, const_cast<uint2*>(P.bin_range), P.pair_total);
+        P.bin_counts, b.rows, b.bins, const_cast<uint2*>(P.bin_range), P.pair_total, nullptr);
     profile_end(stream);
     count_launch();
     profile_begin(stream, "cpv_bin_write");
@@ -606,16 +606,10 @@ void BatchPlan::free_pairs() {
     cap_ = 0;
 }
 
-int BatchPlan::alloc_pairs(uint64_t pairs, uint64_t entries) {
+int BatchPlan::alloc_pairs(uint64_t entries) {
     free_pairs();
     // the sort's 32-bit positions may step past the last pair
     const uint32_t capacity = static_cast<uint32_t>(entries < 0xFFFF0000ull ? entries : 0xFFFF0000ull);
-    // Whole chunks for at most four sorting CTAs an SM. One digit's scatter on
-    // GB300, 608 CTAs then this: 14.6 us then 8.5 for 316k pairs and 1024
-    // digits (155 CTAs; 12.2 at 78 of two chunks), 15.9 then 12.4 for 1.7 M
-    // pairs and 128 digits (413 CTAs, two chunks each instead of 1.4).
-    const uint64_t per = ((pairs + radix_max_ctas_ - 1) / radix_max_ctas_ + CPV_RADIX_CHUNK - 1) / CPV_RADIX_CHUNK * CPV_RADIX_CHUNK;
-    radix_ctas_ = per ? static_cast<uint32_t>((pairs + per - 1) / per) : 1u;
     for (int i = 0; i < 2; i++) {
         int r;
         if ((r = dev_alloc(keys_[i], capacity + 8ull)) != kOk || (r = dev_alloc(vals_[i], capacity)) != kOk) {
@@ -708,8 +702,8 @@ int BatchPlan::build(const Module& m, const BatchDraws& in, cudaStream_t stream)
     if (per_sm < 1) per_sm = 1;
     raster_ctas_ = static_cast<uint32_t>(sms * per_sm);
     if (raster_ctas_ > tiles_) raster_ctas_ = tiles_;
-    radix_max_ctas_ = static_cast<uint32_t>(sms * 4);
-    if ((r = dev_alloc(hist_, static_cast<uint64_t>(radix_max_ctas_) << digit_bits_)) != kOk) return r;
+    radix_ctas_ = static_cast<uint32_t>(sms * 4);
+    if ((r = dev_alloc(hist_, static_cast<uint64_t>(radix_ctas_) << digit_bits_)) != kOk) return r;
 
     P_ = CpvBatchParams{};
     P_.draws = draws_;
@@ -732,7 +726,7 @@ int BatchPlan::build(const Module& m, const BatchDraws& in, cudaStream_t stream)
     P_.block_pairs = block_pairs_;
     P_.pair_total = words_;
     P_.tile_range = passes_ > 1u ? tile_range_ : digit_range_;
-    P_.tile_counter = words_ + 2;
+    P_.tile_counter = words_ + CPV_WORD_TILE;
     P_.status = words_ + 1;
     P_.ndc_x = ndc_;
     P_.ndc_y = ndc_ + in.fb_width;
@@ -756,8 +750,8 @@ int BatchPlan::build(const Module& m, const BatchDraws& in, cudaStream_t stream)
     }
     const uint64_t pairs = *pinned_pairs_;
     // CPV_BATCH_PAIR_CAPACITY forces a capacity (tests of the overflow path).
-    if (const uint32_t forced = env_u32("CPV_BATCH_PAIR_CAPACITY", 0u)) return alloc_pairs(pairs, forced);
-    return alloc_pairs(pairs, pairs + pairs / 4 + (1u << 20));
+    if (const uint32_t forced = env_u32("CPV_BATCH_PAIR_CAPACITY", 0u)) return alloc_pairs(forced);
+    return alloc_pairs(pairs + pairs / 4 + (1u << 20));
 }
 
 // Positions of the set-up blocks' pairs within chunks, and the chunks' totals.
@@ -919,7 +913,7 @@ int BatchPlan::enqueue(const Module& m, cudaStream_t stream) {
     const int r = scan_blocks(stream);
     if (r != kOk) return r;
     cpv_batch_emit<<<(blocks + 7u) / 8u, 256, 0, stream>>>(rects_, block_pairs_, block_offsets_, chunk_sums_, blocks, P_.tiles_x, keys_[0], vals_[0], cap_,
-                                                           words_);
+                                                           words_, radix_ctas_);
     count_launch();
     const uint32_t digits = 1u << digit_bits_;
     for (uint32_t pass = 0; pass < passes_; pass++) {
@@ -927,7 +921,7 @@ int BatchPlan::enqueue(const Module& m, cudaStream_t stream) {
         cpv_radix_hist<<<radix_ctas_, CPV_RADIX_THREADS, 0, stream>>>(keys_[src], words_, cap_, shift, digits, hist_,
                                                                      passes_ > 1u && pass == 0u ? tile_range_ : nullptr, tiles_);
         cpv_bin_scan<<<(digits + CPV_BIN_SCAN_BINS - 1u) / CPV_BIN_SCAN_BINS, CPV_BIN_SCAN_THREADS, 0, stream>>>(
-            hist_, radix_ctas_, digits, digit_range_, reinterpret_cast<unsigned long long*>(words_ + 4 + 2 * pass));
+            hist_, radix_ctas_, digits, digit_range_, reinterpret_cast<unsigned long long*>(words_ + CPV_WORD_DIGITS + 2 * pass), words_);
         cpv_radix_scatter<<<radix_ctas_, CPV_RADIX_THREADS, 0, stream>>>(keys_[src], vals_[src], passes_ > 1u ? keys_[dst] : nullptr, vals_[dst], words_, cap_,
                                                                         shift, digits, hist_);
         count_launch(3);
@@ -976,7 +970,7 @@ int BatchPlan::launch(const Module& m, cudaStream_t stream) {
         const uint64_t pairs = *pinned_pairs_;
         cudaGraphExecDestroy(exec_);
         exec_ = nullptr;
-        const int r = alloc_pairs(pairs, pairs + pairs / 4 + (1u << 20));
+        const int r = alloc_pairs(pairs + pairs / 4 + (1u << 20));
         if (r != kOk) return r;
     }
     cudaGetLastError();

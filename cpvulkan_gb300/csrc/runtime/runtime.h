@@ -166,8 +166,7 @@ public:
 
 private:
     int enqueue(const Module& m, cudaStream_t stream);
-    // Buffers of `entries` pairs, for about `pairs` a frame.
-    int alloc_pairs(uint64_t pairs, uint64_t entries);
+    int alloc_pairs(uint64_t entries);
     int scan_blocks(cudaStream_t stream);
     void free_pairs();
     int build_vertex_stage(const Module& m, const BatchDraws& in, cudaStream_t stream);
@@ -187,7 +186,7 @@ private:
     uint32_t* hist_ = nullptr;
     uint2* digit_range_ = nullptr;      // of the sort's last scan; the tiles' with one digit
     uint2* tile_range_ = nullptr;       // of cpv_tile_ranges
-    uint32_t* words_ = nullptr;         // [0] pair total, [1] status, [2] tile counter, [4..7] the digits' totals
+    uint32_t* words_ = nullptr;         // CPV_WORD_* and [1] status
     float* ndc_ = nullptr;              // pixel-centre NDC of the columns, then the rows
     float* vs_pos_ = nullptr;           // vertex stage: NDC position and clip w per slot
     float* vs_var_ = nullptr;           // vertex stage: outputs per slot
@@ -197,7 +196,7 @@ private:
     uint32_t* pinned_pairs_ = nullptr;  // pair total of the last launch (host)
     cudaEvent_t done_ = nullptr;
     uint64_t prims_ = 0;
-    uint32_t tiles_ = 0, radix_ctas_ = 0, radix_max_ctas_ = 0, raster_ctas_ = 0, passes_ = 1, digit_bits_ = 1, kernels_ = 0;
+    uint32_t tiles_ = 0, radix_ctas_ = 0, raster_ctas_ = 0, passes_ = 1, digit_bits_ = 1, kernels_ = 0;
     cudaGraphExec_t exec_ = nullptr;
 };
 

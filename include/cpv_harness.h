@@ -72,6 +72,9 @@ int cpvh_render_e2e(cpvh_renderer* r, uint32_t frames, double* total_ms, uint64_
  * translation and NVRTC compilation, without rendering. Returns a VkResult. */
 int cpvh_compile_pipelines(cpvh_context* ctx, const cpv_scene* scene, char* err, uint32_t err_len);
 
+/* Uploads the scene's vertex, index and uniform bytes again, as they stand; the recorded frame stays as it is. Returns a VkResult. */
+int cpvh_renderer_upload(cpvh_renderer* r);
+
 /* Re-uploads the scene's uniform buffer and push constants (e.g. after
  * cpvh_scene_set_frame) and re-records the frame. */
 int cpvh_renderer_update(cpvh_renderer* r);
