@@ -196,6 +196,7 @@ struct ModuleConfig {
     uint32_t batch = 256;     // primitives set up per shared-memory batch (set per schedule by module_config)
     uint32_t depth = 0;       // sparse schedule: fragments a pixel lists per batch (0: 24, or 16 when sampling)
     bool samples = false;     // a fragment shader samples images (register budget of the batched raster)
+    bool depth_ops = false;   // the pipeline tests or writes depth or stencil (per-draw modules)
     bool linear = false;      // the pipeline's fragments are a linear blend of a constant colour (per-draw modules)
 };
 

@@ -163,19 +163,26 @@ std::string compose_module(const std::vector<std::string>& stages, const std::ve
         }
     }
     // Register budget of the per-draw raster in resident CTAs of 256
-    // threads: seven for the immediate schedule; four for the others where a thread keeps one pixel of one
-    // attachment (a textured 500k-triangle request's raster 0.25 ms, 0.32 at
-    // the compiler's choice of 112 registers, 0.27 at five; half-float
-    // overdraw 0.51 ms, 0.58 at three, 0.55 at five). Several pixels or
-    // attachments a thread, and the quad-derivative mode, keep the
-    // compiler's choice. CPV_PLAIN_MIN_BLOCKS overrides.
+    // threads. The immediate schedule: five with depth or stencil
+    // operations, where more spill the fragment loop: 12000 large flat
+    // triangles at 1280x720, raster at five, six and seven, blended 2.83, 2.86
+    // and 3.25 ms, opaque 3.23, 3.68 and 3.98, with stencil 4.22, 4.54 and
+    // 4.78. Seven without, as tests/test_pipeline_compile.py expects of a
+    // blended flat pipeline, though six is faster in this loop as well (MAX
+    // blend 2.25 and 2.56 ms, logic op 2.07 and 2.19). A linear blend's raster
+    // has CPV_LINEAR_MIN_BLOCKS instead. Four for the other schedules where a
+    // thread keeps one pixel of one attachment (a textured 500k-triangle
+    // request's raster 0.25 ms, 0.32 at the compiler's choice of 112 registers,
+    // 0.27 at five; half-float overdraw 0.51 ms, 0.58 at three, 0.55 at five).
+    // Several pixels or attachments a thread, and the quad-derivative mode,
+    // keep the compiler's choice. CPV_PLAIN_MIN_BLOCKS overrides.
     const uint32_t pixels = 1u << (2 * mc.tile_shift), cta = std::min(pixels, 32u * mc.warps);
     bool lod_sites = false;
     for (const std::string& st : stages) {
         const size_t at = st.find("#define CPV_LOD_SITES ");
         lod_sites = lod_sites || (at != std::string::npos && std::atoi(st.c_str() + at + 22) > 0);
     }
-    int min_blocks = mc.schedule == 0 ? 7 : (pixels == cta && num_ca == 1 && !lod_sites ? static_cast<int>(1024u / cta) : 0);
+    int min_blocks = mc.schedule == 0 ? (mc.depth_ops ? 5 : 7) : (pixels == cta && num_ca == 1 && !lod_sites ? static_cast<int>(1024u / cta) : 0);
     if (const char* v = std::getenv("CPV_PLAIN_MIN_BLOCKS")) min_blocks = std::atoi(v);
     if (min_blocks >= 1 && min_blocks <= 32) src << "#define CPV_PLAIN_MIN_BLOCKS " << min_blocks << "\n";
     // Register budget of the persistent batched raster, in resident CTAs of
@@ -647,6 +654,7 @@ VkResult create_graphics_pipeline(Device* dev, PipelineCache* cache, const VkGra
     auto additive = [](VkBlendOp op) { return op == VK_BLEND_OP_ADD || op == VK_BLEND_OP_SUBTRACT || op == VK_BLEND_OP_REVERSE_SUBTRACT; };
     const bool depth_ops = dfmt != VK_FORMAT_UNDEFINED && (ds.depthTestEnable || stencil || ds.depthBoundsTestEnable);
     ModuleConfig mc = module_config(tile_shift, prefers_deferred, fs_constant, fr.samples > 0);
+    mc.depth_ops = depth_ops;
     mc.linear = fs_constant && nca == 1 && !logic && !depth_ops && (cfmt == VK_FORMAT_R8G8B8A8_UNORM || cfmt == VK_FORMAT_B8G8R8A8_UNORM) &&
                 (!blend.blendEnable || (!dst_factor(blend.srcColorBlendFactor) && !dst_factor(blend.dstColorBlendFactor) &&
                                         !dst_factor(blend.srcAlphaBlendFactor) && !dst_factor(blend.dstAlphaBlendFactor) && additive(blend.colorBlendOp) &&
