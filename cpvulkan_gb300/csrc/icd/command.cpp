@@ -1186,6 +1186,7 @@ void CommandBuffer::reset() {
 }
 
 VkResult run_command_buffer(Queue* q, CommandBuffer* cb, std::vector<WrittenRange>& written, bool no_alloc) {
+    if (!no_alloc) q->scratch.grow_lists();
     if (no_alloc || rt::profile_enabled() || env_u32("CPV_CB_GRAPH", 1u) == 0u || cb->graphable == 0) return execute(q, cb, written, no_alloc);
     if (cb->graphable < 0) {
         // First execution: eager. It decides whether the buffer can be a graph

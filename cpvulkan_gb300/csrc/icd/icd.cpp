@@ -1595,6 +1595,12 @@ CPV_EXPORT uint64_t cpv_queue_scratch_generation(VkQueue queue) {
     return q ? q->scratch.generation() : 0;
 }
 
+CPV_EXPORT void cpv_queue_list_stats(VkQueue queue, uint64_t out[2]) {
+    auto* q = reinterpret_cast<cpv::icd::Queue*>(queue);
+    out[0] = q ? q->scratch.list_capacity() : 0;
+    out[1] = q ? q->scratch.list_need() : 0;
+}
+
 CPV_EXPORT void cpv_profile_enable(int on) { cpv::rt::profile_enable(on != 0); }
 
 CPV_EXPORT int cpv_profile_get(const char* kernel, uint64_t* launches, double* total_ms) { return cpv::rt::profile_get(kernel, launches, total_ms); }

@@ -18,7 +18,7 @@
  *
  * Every launch has a shape the host knows and no value is carried from one
  * draw to the next, so the sequence needs no memset and can be captured in a
- * CUDA graph. The list has a fixed capacity; a draw that would exceed it
+ * CUDA graph. The list has a capacity; a draw that would exceed it
  * writes none and the raster filters the rectangles of all primitives
  * (slower, same result).
  *
@@ -111,13 +111,18 @@ extern "C" __global__ void __launch_bounds__(CPV_BIN_SCAN_THREADS) cpv_bin_scan(
  * row's running positions, and each warp then places its (primitive, bin)
  * pairs 32 at a time in primitive order (a match-any rank within the step,
  * the warp's own position per bin between steps, all in shared memory).
- * Dynamic shared memory: 9 words per bin. */
+ * A draw over the capacity leaves its pairs in *need (host memory; may be
+ * null), for the host to grow the lists. Dynamic shared memory: 9 words per
+ * bin. */
 extern "C" __global__ void __launch_bounds__(256) cpv_bin_write(const uint2* __restrict__ rects, uint64_t prims, uint32_t row_prims, uint32_t shift,
                                                                 uint32_t bins_x, uint32_t bins, const uint32_t* __restrict__ offsets,
                                                                 uint32_t* __restrict__ list, uint32_t* __restrict__ list_rects, uint32_t capacity,
-                                                                const unsigned long long* __restrict__ total) {
+                                                                const unsigned long long* __restrict__ total, unsigned long long* need) {
     extern __shared__ uint32_t cpv_bin_smem[];
-    if (*total > capacity) return;
+    if (*total > capacity) {
+        if (need && blockIdx.x == 0u && threadIdx.x == 0u && *need < *total) *need = *total;
+        return;
+    }
     uint32_t* next = cpv_bin_smem;  /* [bin]: the row's next position */
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint32_t* mine = cpv_bin_smem + (1u + warp) * bins;  /* [bin]: this warp's count, then its next position */

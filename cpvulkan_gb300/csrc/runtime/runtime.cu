@@ -287,6 +287,7 @@ Scratch::~Scratch() {
     cudaFree(list_);
     cudaFree(list_rects_);
     cudaFree(words_);
+    if (need_) cudaFreeHost(need_);
     cudaFree(tables_);
 }
 
@@ -312,12 +313,28 @@ int Scratch::reserve_list(uint64_t entries) {
     return grow_tracked(list_rects_, list_rects_cap_, entries);
 }
 
+void Scratch::grow_lists() {
+    const uint64_t want = std::min<uint64_t>(list_need(), list_limit());
+    if (list_full_ || want <= list_capacity()) return;
+    list_full_ = reserve_list(want) != kOk;  // no more than there is memory for
+}
+
+uint64_t Scratch::list_limit() { return env_u32("CPV_LIST_CAPACITY", 1u << 26); }
+
 int Scratch::reserve_tables(uint64_t bytes) { return grow_tracked(tables_, tables_cap_, bytes); }
 
 int Scratch::ensure_words() {
     if (words_) return kOk;
+    if (cudaMallocHost(reinterpret_cast<void**>(&need_), sizeof(*need_)) != cudaSuccess) {
+        cudaGetLastError();
+        need_ = nullptr;
+        return kErrOutOfMemory;
+    }
+    *need_ = 0;
     if (cudaMalloc(reinterpret_cast<void**>(&words_), kWordsBytes) != cudaSuccess) {
         cudaGetLastError();
+        cudaFreeHost(need_);
+        need_ = nullptr;
         return kErrOutOfMemory;
     }
     cudaMemset(words_, 0, kWordsBytes);
@@ -458,7 +475,8 @@ BinShape bin_shape(uint64_t prims, uint32_t tiles_x, uint32_t tiles_y) {
 }
 
 // The per-draw kernels after P's buffers are set: set-up and binning.
-int bin_draw(cudaStream_t stream, const Module& m, const BinShape& b, CpvDrawParams& P) {
+// `need`: receives the pairs of a draw over the lists' capacity (may be null).
+int bin_draw(cudaStream_t stream, const Module& m, const BinShape& b, CpvDrawParams& P, unsigned long long* need) {
     void* args[] = {&P};
     profile_begin(stream, "cpv_setup_rects");
     CPV_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(m.setup_rects), dim3(b.rows), dim3(256), args, 0, stream));
@@ -473,7 +491,7 @@ int bin_draw(cudaStream_t stream, const Module& m, const BinShape& b, CpvDrawPar
     profile_begin(stream, "cpv_bin_write");
     cpv_bin_write<<<b.rows, 256, 9u * b.bins * sizeof(uint32_t), stream>>>(P.rects, P.total_prims, b.row_prims, b.shift, b.bins_x, b.bins, P.bin_counts,
                                                                           const_cast<uint32_t*>(P.bin_list), const_cast<uint32_t*>(P.bin_rects),
-                                                                          P.list_capacity, P.pair_total);
+                                                                          P.list_capacity, P.pair_total, need);
     profile_end(stream);
     count_launch();
     CPV_CUDA(cudaGetLastError());
@@ -515,12 +533,19 @@ int draw_plain(cudaStream_t stream, const Module& m, CpvDrawParams P, Scratch& s
     if (b.mode != BinShape::kDirect) {
         if ((r = sc.reserve_rects(G)) != kOk) return r;
         if (b.mode == BinShape::kLists) {
-            // the list holds what the draw can need at most, up to CPV_LIST_CAPACITY entries
-            const uint64_t cap = std::min<uint64_t>(env_u32("CPV_LIST_CAPACITY", 1u << 26), G * b.bins);
+            // The lists hold 2^20 pairs, or what the draw can need at most up to
+            // 2^23 (64 MiB of ids and rectangles) or four a primitive; a draw
+            // that needs more filters (it covers so many bins a primitive that
+            // its lists would spare little) and has them grown for the next
+            // submission (Scratch::grow_lists). CPV_LIST_START sets the first
+            // capacity, CPV_LIST_CAPACITY the largest (tests).
+            const uint64_t usual = std::max<uint64_t>(1u << 20, std::min<uint64_t>(G * b.bins, std::max<uint64_t>(1u << 23, 4u * G)));
+            const uint64_t cap = std::min<uint64_t>(Scratch::list_limit(), env_u32("CPV_LIST_START", static_cast<uint32_t>(std::min<uint64_t>(usual, 1u << 31))));
             if ((r = sc.reserve_bins(static_cast<uint64_t>(b.rows) * b.bins, b.bins)) != kOk || (r = sc.reserve_list(cap)) != kOk) return r;
         }
-        set_bin_params(P, b, sc.rects(), sc.counts(), sc.ranges(), sc.list(), sc.list_rects(), sc.list_capacity(), sc.words());
-        if ((r = bin_draw(stream, m, b, P)) != kOk) return r;
+        set_bin_params(P, b, sc.rects(), sc.counts(), sc.ranges(), sc.list(), sc.list_rects(),
+                       static_cast<uint32_t>(std::min<uint64_t>(sc.list_capacity(), Scratch::list_limit())), sc.words());
+        if ((r = bin_draw(stream, m, b, P, sc.need())) != kOk) return r;
     }
     // Blend tables: 1 KiB per primitive, built once per draw, when the
     // pipeline blends a per-primitive constant colour (up to 4 GiB of them;
@@ -1149,7 +1174,7 @@ int draw_plain_static(cudaStream_t stream, const Module& m, CpvDrawParams P) {
         uint32_t* list = reinterpret_cast<uint32_t*>(base + lists_at);
         set_bin_params(P, b, reinterpret_cast<uint2*>(base + rects_at), reinterpret_cast<uint32_t*>(base + counts_at),
                        reinterpret_cast<uint2*>(base + ranges_at), list, list + entries, static_cast<uint32_t>(entries), words);
-        if ((r = bin_draw(stream, m, b, P)) != kOk) return r;
+        if ((r = bin_draw(stream, m, b, P, nullptr)) != kOk) return r;
     }
     {
         void* args[] = {&P};

@@ -80,6 +80,13 @@ public:
     uint32_t* list() const { return list_; }
     uint32_t* list_rects() const { return list_rects_; }
     uint32_t list_capacity() const { return static_cast<uint32_t>(std::min(list_cap_, list_rects_cap_)); }
+    // Pairs of the largest draw that the lists did not hold (0: none), and the
+    // word in pinned host memory in which the kernels leave them.
+    uint64_t list_need() const { return need_ ? *static_cast<volatile unsigned long long*>(need_) : 0; }
+    unsigned long long* need() const { return need_; }
+    // Grows the lists to that. Called between submissions.
+    void grow_lists();
+    static uint64_t list_limit();
     uint32_t* words() const { return words_; }  // kWordsBytes
     int ensure_words();
     // Incremented whenever a buffer is (re)allocated: work captured in a CUDA
@@ -100,6 +107,8 @@ private:
     uint64_t list_cap_ = 0;
     uint32_t* list_rects_ = nullptr;
     uint64_t list_rects_cap_ = 0;
+    unsigned long long* need_ = nullptr;
+    bool list_full_ = false;  // growing the lists has failed
     uint32_t* words_ = nullptr;
     uint8_t* tables_ = nullptr;
     uint64_t tables_cap_ = 0;

@@ -84,6 +84,11 @@ CPV_EXPORT double cpv_queue_elapsed_ms(VkQueue queue, uint32_t slot_begin, uint3
  * only ever ran cpv_queue_submit_no_alloc. */
 CPV_EXPORT uint64_t cpv_queue_scratch_generation(VkQueue queue);
 
+/* The queue's bin lists: out[0] (primitive, bin) pairs they hold (8 bytes
+ * each), out[1] the pairs of the largest draw that did not fit when it ran (0:
+ * none; such a draw filters all its primitives in every tile). */
+CPV_EXPORT void cpv_queue_list_stats(VkQueue queue, uint64_t out[2]);
+
 /* Per-kernel device timing: while enabled, every kernel of the draw paths is
  * bracketed by CUDA events on its stream (batched render passes then run
  * without their CUDA graph). cpv_profile_get returns the launches and the
