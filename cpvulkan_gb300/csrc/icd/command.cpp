@@ -986,6 +986,7 @@ VkResult execute(Queue* q, CommandBuffer* cb, std::vector<WrittenRange>& written
             const bool to_image = c.type == CmdType::CopyBufferToImage;
             Buffer* buf = static_cast<Buffer*>(c.p[0]);
             Image* img = static_cast<Image*>(c.p[1]);
+            if (!buf->memory || !img->memory) return VK_ERROR_DEVICE_LOST;
             if (to_image) reads(q->device, buf, &written);
             for (const auto& reg : c.image_regions) {
                 const uint32_t level = reg.imageSubresource.mipLevel;
