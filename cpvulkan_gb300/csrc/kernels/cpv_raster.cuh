@@ -35,15 +35,17 @@
 #endif
 #ifndef CPV_DENSE
 /* sparse: large primitives' pixels per tile pixel from which a batch runs the
- * immediate schedule. A pixel whose list overflows walks the whole batch, a
- * warp of the immediate schedule only what may cover its block: 6k smooth
- * quads at 1280x720 take 420 us without this rule, 273 at 2 to 8, 275 at 16,
- * 289 at 24, 355 at 32; 300 half-float triangles 416, 322, 328, 340 and 386. By
- * the boxes instead of the triangles' areas, slivers count too much (180k
- * triangles at 1366x767: 95 us, 150 at 8 by boxes). Batched modules mix their
- * draws' small and large primitives in a batch, where the lists are better for
- * longer (compose_module: 32): 512 draws at 2560x1440 take 2436 us without
- * it, 2878 at 8, 2588 at 16, 2485 at 24, 2437 at 32. */
+ * immediate schedule: every pixel's thread walks the whole batch in order,
+ * testing boxes (sparse modules have no per-warp lists), and shades what
+ * covers it. A pixel whose list overflows walks the batch as well, but after
+ * the listing, and its warp waits for it. 6k smooth quads at 1280x720 take 420
+ * us without this rule, 273 at 2 to 8, 275 at 16, 289 at 24, 355 at 32; 300
+ * half-float triangles 416, 322, 328, 340 and 386. By the boxes instead of the
+ * triangles' areas, slivers count too much (180k triangles at 1366x767: 95 us,
+ * 150 at 8 by boxes). Batched modules mix their draws' small and large
+ * primitives in a batch, where the lists are better for longer
+ * (compose_module: 32): 512 draws at 2560x1440 take 2436 us without it, 2878
+ * at 8, 2588 at 16, 2485 at 24, 2437 at 32. */
 #define CPV_DENSE 8
 #endif
 #ifndef CPV_RT_WARPS
@@ -651,15 +653,17 @@ __device__ __forceinline__ void cpv_clear_tile(const Source& src, uint32_t tx, u
  *               coverage pattern), and finally every pixel's thread applies
  *               its own fragments' per-fragment operations in primitive
  *               order (expensive shaders);
- *   2 sparse  — coverage is found per primitive instead of per pixel: a
- *               primitive whose bounding box covers at most CPV_SMALL_PX
- *               pixels of the tile is rasterised by one thread, which tests
- *               only those pixels; larger ones are tested by the pixels'
- *               threads. Either appends the primitive's batch index to each
- *               covered pixel's list (up to CPV_SLOT_DEPTH per batch); each
- *               pixel's thread then shades and applies its list in
- *               primitive order (tiny primitives, heavy overdraw). A pixel
- *               whose list overflowed walks the whole batch instead.
+ *   2 sparse  — coverage is found per primitive instead of per pixel: the
+ *               primitives whose bounding boxes cover at most CPV_SMALL_PX
+ *               pixels of the tile are rasterised by warps, 32 primitives'
+ *               pixels spread over the lanes; larger ones are tested by the
+ *               pixels' threads. Either appends the primitive's batch index
+ *               to each covered pixel's list (up to CPV_SLOT_DEPTH per
+ *               batch); each pixel's thread then shades and applies its list
+ *               in primitive order (tiny primitives, heavy overdraw). A pixel
+ *               whose list overflowed walks the whole batch instead, and a
+ *               batch dense in large primitives (CPV_DENSE) runs the
+ *               immediate schedule.
  * All apply each pixel's fragments in API primitive order, as the
  * reference's serial loop does. */
 template <class Source>
@@ -866,9 +870,10 @@ __device__ __forceinline__ void cpv_raster_tile(Source& src, uint32_t first, uin
 #endif
 #if !CPV_DEFERRED
         /* immediate: every pixel's thread tests each primitive in order,
-         * shading and applying what it covers. Each warp first lists, in
-         * order, the batch's live primitives whose box reaches its rows, and
-         * walks only those. */
+         * shading and applying what it covers. In modules of the immediate
+         * schedule each warp first lists, in order, the batch's live
+         * primitives that may reach its pixels, and walks only those; a dense
+         * batch of a sparse module walks all. */
         if (immediate_batch) {
 #if CPV_WARP_LISTS
             const uint32_t lane = threadIdx.x & 31u;
